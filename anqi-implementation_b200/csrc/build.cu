@@ -28,6 +28,7 @@
 #include <cstdlib>
 
 #include "beam.cuh"
+#include "component.h"
 #include "internal.h"
 #include "util.cuh"
 
@@ -99,6 +100,10 @@ struct GatherParams {
     // row number -> original id.  Lists, rows and norms are given in the new
     // numbering; (dist, id) ties and the output use the original ids.
     const uint32_t* perm;
+    // and rows already gathered on their component's tables (run_component_gather):
+    // those with a component number whose bad flag is clear; null: none
+    const uint32_t* row_comp;
+    const uint32_t* comp_bad;
     // edge-policy prunes: the rows [row_base, row_base + row_count) of the work
     // list (row_count 0: all), each writing its pool (pool_cap entries apart)
     // and its size to the dump buffers instead of pruning it
@@ -315,6 +320,9 @@ __global__ void __launch_bounds__(128, kVam ? 5 : 7) gather_kernel(GatherParams 
         if (i >= p.n) {
             if (lane == 0) set_error(p.err, kDevBadId);
             continue;
+        }
+        if constexpr (kRen) {
+            if (p.row_comp && p.row_comp[i] != kEmpty && !p.comp_bad[p.row_comp[i]]) continue;
         }
 
         if (p.mode == kModeCommit) {
@@ -1213,8 +1221,11 @@ static int build_reverse(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K, 
 // The locality numbering of the gather (label propagation on the device, a
 // counting sort by label in tree-0 order on the host): perm (new -> original)
 // and inv (original -> new).  order: tree 0's permutation.
+// ranges receives the components of at most kCompMaxRows rows (none when the
+// propagation was cut off, whose labels are not whole components), in_ranges
+// how many rows they hold.
 static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K, const uint32_t* d_order, DevBuf& perm,
-                          DevBuf& inv) {
+                          DevBuf& inv, std::vector<CompRange>& ranges, uint64_t& in_ranges) {
     TmpBuf lab(c), flag(c);
     int rc;
     if ((rc = ensure(c, lab, n * 4)) || (rc = ensure(c, flag, 4)) || (rc = ensure(c, perm, n * 4)) ||
@@ -1225,14 +1236,15 @@ static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K,
     ANQI_CUDA(c, cudaGetLastError());
     // rounds until no label falls (bounded; a cut-off round count only
     // weakens the locality, never a result)
-    for (int round = 0; round < 64; round++) {
+    bool whole = false;
+    for (int round = 0; round < 64 && !whole; round++) {
         ANQI_CUDA(c, cudaMemsetAsync(flag.p, 0, 4, c->stream));
         label_prop_kernel<<<blocks, 256, 0, c->stream>>>(d_ids, n, K, lab.as<uint32_t>(), flag.as<uint32_t>());
         label_jump_kernel<<<blocks, 256, 0, c->stream>>>(lab.as<uint32_t>(), n);
         ANQI_CUDA(c, cudaGetLastError());
         uint32_t changed = 0;
         if ((rc = d2h(c, &changed, flag, 4)) || (rc = sync(c))) return rc;
-        if (!changed) break;
+        whole = !changed;
     }
     std::vector<uint32_t> hl(n), ho(n), start(n + 1, 0), out(n);
     ANQI_CUDA(c, cudaMemcpyAsync(ho.data(), d_order, n * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1242,6 +1254,14 @@ static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K,
         start[hl[i] + 1]++;
     }
     for (uint64_t l = 0; l < n; l++) start[l + 1] += start[l];
+    ranges.clear();
+    in_ranges = 0;
+    for (uint64_t l = 0; l < n && whole; l++) {
+        const uint32_t size = start[l + 1] - start[l];
+        if (size == 0 || size > kCompMaxRows) continue;
+        ranges.push_back({start[l], size});
+        in_ranges += size;
+    }
     for (uint64_t k = 0; k < n; k++) {
         const uint32_t o = ho[k];
         if (o >= n) return fail(c, ANQI_ERR_DEVICE, "locality numbering: bad tree order");
@@ -2462,8 +2482,10 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
     const char* ren_env = std::getenv("ANQI_B200_GATHER_RENUMBER");
     const bool ren = !ip && !(ren_env && ren_env[0] == '0');
     TmpBuf dxc(c), rperm(c), rinv(c), rids(c), rvals(c), rnorm(c);
+    std::vector<CompRange> ranges;
+    uint64_t in_ranges = 0;
     if (ren) {
-        if ((rc = locality_order(c, gid.as<uint32_t>(), n, K, order.as<uint32_t>(), rperm, rinv)) ||
+        if ((rc = locality_order(c, gid.as<uint32_t>(), n, K, order.as<uint32_t>(), rperm, rinv, ranges, in_ranges)) ||
             (rc = ensure(c, rids, n * K * 4)) || (rc = ensure(c, rvals, n * K * 4)) || (rc = ensure(c, rnorm, n * 4)) ||
             (rc = ensure(c, dxc, n * xs * 4ull)))
             return rc;
@@ -2515,7 +2537,51 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                       : order.as<uint32_t>();
     uint64_t pool_total = 0;
     double gather_kernel_ms = 0;
-    if ((rc = run_gather(c, p, max_reverse(c, roff, n), &pool_total, &gather_kernel_ms))) return rc;
+    // rows of small components search on their component's distance matrix and
+    // adjacency bitmaps; ANQI_B200_GATHER_COMPONENTS=0 leaves them to the general gather
+    TmpBuf row_comp(c), comp_bad(c), comp_pool(c);
+    bool rest = true;  // rows left for the general gather
+    const char* comp_env = std::getenv("ANQI_B200_GATHER_COMPONENTS");
+    if (!ranges.empty() && !(comp_env && comp_env[0] == '0')) {
+        if ((rc = ensure(c, comp_pool, 8))) return rc;
+        ANQI_CUDA(c, cudaMemsetAsync(comp_pool.p, 0, 8, c->stream));
+        CompGather g{};
+        g.x = p.x;
+        g.norms = p.norms;
+        g.n = n;
+        g.stride = p.stride;
+        g.dim = p.dim;
+        g.cols = p.cols;
+        g.g_ids = p.g_ids;
+        g.g_vals = p.g_vals;
+        g.K = K;
+        g.rev_off = p.rev_off;
+        g.rev_ids = p.rev_ids;
+        g.ef = p.ef;
+        g.cap = p.cap;
+        g.out_k = K;
+        g.perm = p.perm;
+        g.out_ids = p.out_ids;
+        g.out_d = p.out_d;
+        g.pool_total = comp_pool.as<unsigned long long>();
+        bool any_bad = false;
+        ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+        if ((rc = run_component_gather(c, g, ranges, row_comp, comp_bad, &any_bad))) return rc;
+        ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+        ANQI_CUDA(c, cudaMemcpyAsync(&pool_total, comp_pool.p, 8, cudaMemcpyDeviceToHost, c->stream));
+        if ((rc = sync(c))) return rc;
+        float ms = 0;
+        ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+        gather_kernel_ms += ms;
+        p.row_comp = row_comp.as<uint32_t>();
+        p.comp_bad = comp_bad.as<uint32_t>();
+        rest = in_ranges < n || any_bad;
+    }
+    if (rest) {
+        uint64_t pooled = 0;
+        if ((rc = run_gather(c, p, max_reverse(c, roff, n), &pooled, &gather_kernel_ms))) return rc;
+        pool_total += pooled;
+    }
     const double gather_ms = ms_since(t);
     if ((rc = d2h(c, ids, oi, n * K * 4)) || (rc = d2h(c, dists, od, n * K * 4)) || (rc = sync(c))) return rc;
     if (st) {
