@@ -266,18 +266,59 @@ __global__ void __launch_bounds__(1024) fit_bitonic_shared_kernel(double* __rest
     for (uint32_t t = threadIdx.x; t < kSortChunk; t += blockDim.x) a[base + t] = s[t];
 }
 
-// prefix[k][0] = 0, prefix[k][i+1] = prefix[k][i] + s[k][i], in index order (np.cumsum)
-__global__ void fit_prefix_kernel(const double* __restrict__ a, uint64_t m, uint32_t nk, uint64_t n2,
-                                  double* __restrict__ prefix) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    const double* s = a + (uint64_t)k * n2;
-    double* pf = prefix + (uint64_t)k * (m + 1);
+// prefix[k][0] = 0, prefix[k][i+1] = prefix[k][i] + s[k][i], in index order
+// (np.cumsum): one serial chain of FP64 additions a column, which bounds it.  A
+// block per column keeps that chain fed: thread 0 adds a tile out of shared
+// memory into shared memory while the other warps bring the next tile in and
+// write the last one out.
+constexpr uint32_t kPrefixTile = 1024;
+__global__ void __launch_bounds__(128) fit_prefix_kernel(const double* __restrict__ a, uint64_t m, uint64_t n2,
+                                                         double* __restrict__ prefix) {
+    __shared__ __align__(16) double in[2][kPrefixTile], out[2][kPrefixTile];
+    const double* s = a + (uint64_t)blockIdx.x * n2;
+    double* pf = prefix + (uint64_t)blockIdx.x * (m + 1);
+    const uint64_t tiles = (m + kPrefixTile - 1) / kPrefixTile;
+    const uint32_t helper = threadIdx.x - 32, helpers = blockDim.x - 32;  // warps 1..
+    auto bring = [&](uint64_t t) {
+        for (uint32_t i = helper; i < kPrefixTile; i += helpers) {
+            const uint64_t at = t * kPrefixTile + i;
+            in[t & 1][i] = at < m ? s[at] : 0.0;
+        }
+    };
+    if (threadIdx.x >= 32) bring(0);
+    if (threadIdx.x == 0) pf[0] = 0.0;
+    __syncthreads();
     double run = 0.0;
-    pf[0] = 0.0;
-    for (uint64_t i = 0; i < m; i++) {
-        run = __dadd_rn(run, s[i]);
-        pf[i + 1] = run;
+    for (uint64_t t = 0; t <= tiles; t++) {
+        if (threadIdx.x == 0 && t < tiles) {
+            const double2* src = reinterpret_cast<const double2*>(in[t & 1]);
+            double2* dst = reinterpret_cast<double2*>(out[t & 1]);
+            double2 v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) v[q] = src[q];
+#pragma unroll 2
+            for (uint32_t i = 0; i < kPrefixTile / 2; i += 4) {
+                double2 nx[4];
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) nx[q] = src[(i + 4 + q) % (kPrefixTile / 2)];
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) {
+                    double2 r;
+                    r.x = __dadd_rn(run, v[q].x);
+                    run = r.y = __dadd_rn(r.x, v[q].y);
+                    dst[i + q] = r;
+                    v[q] = nx[q];
+                }
+            }
+        } else if (threadIdx.x >= 32) {
+            if (t + 1 < tiles) bring(t + 1);
+            if (t > 0)
+                for (uint32_t i = helper; i < kPrefixTile; i += helpers) {
+                    const uint64_t at = (t - 1) * kPrefixTile + i;
+                    if (at < m) pf[at + 1] = out[(t - 1) & 1][i];
+                }
+        }
+        __syncthreads();
     }
 }
 
@@ -462,7 +503,7 @@ int anqi_lrq_fit_codebooks(const double* res, uint64_t m, uint32_t nk, uint32_t 
             fit_bitonic_global_kernel<<<grid_for(total / 2, 256), 256, 0, st>>>(a, total, n2, kk, j);
         fit_bitonic_shared_kernel<<<chunks, 1024, 0, st>>>(a, n2, kk, kk);
     }
-    fit_prefix_kernel<<<(nk + 31) / 32, 32, 0, st>>>(a, m, nk, n2, prefix);
+    fit_prefix_kernel<<<nk, 128, 0, st>>>(a, m, n2, prefix);
     fit_lloyd_kernel<<<nk, 256, 0, st>>>(a, m, n2, prefix, cs, iters, codebooks);
     return cudaGetLastError() == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
 }
