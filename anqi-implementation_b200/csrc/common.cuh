@@ -63,11 +63,13 @@ __device__ __forceinline__ float group_reduce16(float a0, float a1, float a2, fl
 
 // Squared L2 (distance.h:58-86).  a, b: 16-byte aligned rows whose allocation
 // extends to a multiple of 4 floats past dim.  gt = thread index in the group.
+// kUnroll chunks are loaded together (8 for rows read straight from L2).
+template <int kUnroll = 4>
 __device__ __forceinline__ float group_l2sqr(const float* __restrict__ a, const float* __restrict__ b,
                                              uint32_t dim, uint32_t gt, unsigned mask) {
     const uint32_t q16 = dim >> 4, rem = dim & 15u;
     float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-#pragma unroll 4
+#pragma unroll kUnroll
     for (uint32_t c = 0; c < q16; c++) {
         float4 x = *reinterpret_cast<const float4*>(a + 16 * c + 4 * gt);
         float4 y = *reinterpret_cast<const float4*>(b + 16 * c + 4 * gt);

@@ -144,6 +144,7 @@ struct Ctx {
     uint32_t last_cfg_hash = 0, last_cfg_gcap = 0, last_cfg_blocks = 0;
     size_t last_cfg_smem = 0;
     uint32_t last_cfg_wpb = 4, last_cfg_post = 8;  // block shape and candidate tile
+    bool last_cfg_block = false;                   // one block per query
     cudaGraphExec_t qgraph = nullptr;
     DevBuf init_cnt, init_cid, init_key;  // tensor-core init_knn candidate buffers
     GraphBuild gb;                        // staged G48 build

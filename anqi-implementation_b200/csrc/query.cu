@@ -562,6 +562,298 @@ __global__ void __launch_bounds__(32 * kWpb, 32 / kWpb) rknn_search_kernel(Searc
     }
 }
 
+// ------------------------------------------------- one block per query
+// The search of a batch too small to fill the machine with a warp per query,
+// where a query's latency is the batch's: 64 groups of 4 threads take every
+// fresh neighbour of an expansion at once (rows straight from L2 into
+// registers, one round trip instead of one per 8 staged rows), the visited set
+// is one bitmap over all objects in shared memory, and the beam is merged in
+// one step between two buffers, a thread per entry.  Same expansions, same
+// arithmetic, same (dist, original id) order as rknn_search_kernel, so the
+// results are its.  Bound by the latency of its chain per expansion: links,
+// visited test, rows, rank and merge, four block barriers.  One query, 50,000 x
+// 128, L = 128: 827 us a warp per query, 518 us this way; 333 queries, 60,000 x
+// 100 (ip), L = 85: 1,540 us and 472 us.
+constexpr uint32_t kBlockThreads = 256;
+constexpr uint32_t kBlockCand = 1024;  // candidates kept in shared memory; the rest in the slot's scratch
+
+__device__ __host__ __forceinline__ size_t block_search_words(uint32_t L_max, uint32_t lstride, uint64_t n) {
+    return (size_t)lstride + 4 * (size_t)L_max + 4 * 64 + kBlockCand + 32 + ((n + 127) / 128) * 4;
+}
+
+template <uint32_t kDim>
+__global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(SearchParams p) {
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, gt = t & 3u, grp = t >> 2;
+    const uint32_t ls = search_lstride<kDim>(p);
+    float* qhat = reinterpret_cast<float*>(g_smem);
+    auto beam = [&](uint32_t b) { return qhat + ls + b * 2 * p.L_max; };  // two beam buffers: distances, then ids
+    float* nd = qhat + ls + 4 * p.L_max;  // fresh neighbours in link order ...
+    uint32_t* ni = reinterpret_cast<uint32_t*>(nd + 64);
+    float* sd = reinterpret_cast<float*>(ni + 64);  // ... and sorted
+    uint32_t* si = reinterpret_cast<uint32_t*>(sd + 64);
+    uint32_t* clist = si + 64;
+    uint32_t* s_u = clist + kBlockCand;  // block scalars, 32 words
+    uint32_t* bits = s_u + 32;
+    const uint32_t words4 = (uint32_t)((p.n + 127) / 128);
+    uint32_t* cspill = p.cand_scratch + (size_t)blockIdx.x * p.cand_cap;
+    auto cand_at = [&](uint32_t i) -> uint32_t& { return i < kBlockCand ? clist[i] : cspill[i]; };
+    enum { kWork = 0, kM, kNcand, kOver, kCn, kDep, kAt, kWarpCnt = 16 };
+    const PermOrder ord{p.perm};
+    auto row_dist = [&](uint32_t id) {
+        const float* row = p.lifted + (size_t)id * ls;
+        if constexpr (kDim == kColsDim) return group_l2sqr_cols<kColsDim>(row, qhat, gt, kFull);
+        else return group_l2sqr<8>(row, qhat, p.dim, gt, kFull);
+    };
+
+    for (;;) {
+        __syncthreads();  // the last query's reads of the shared state
+        if (t == 0) s_u[kWork] = atomicAdd(p.work, 1u);
+        for (uint32_t w = t; w < words4; w += kBlockThreads)
+            reinterpret_cast<uint4*>(bits)[w] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        const uint32_t wi = s_u[kWork];
+        if (wi >= p.nq) break;
+        const uint32_t qi = p.order ? p.order[wi] : wi;
+        const uint32_t L = min(p.qL ? p.qL[qi] : p.L_all, p.L_max);
+        const uint32_t tslot = p.qslot ? p.qslot[qi] : p.slot_all;
+        const float* q = p.queries + (size_t)qi * p.bstride;
+        const float r2f = p.ip ? p.qR2f[qi] : p.R2f;
+        for (uint32_t j = t; j < ls; j += kBlockThreads) {
+            float v = 0.0f;
+            if (j < p.d) v = __double2float_rn(__dmul_rn((double)q[j], p.scale));
+            else if (j == p.d) v = 1.0f;
+            qhat[kDim == kColsDim ? chunk_col_pos(j, kColsDim / 16 * 16) : j] = v;
+        }
+        uint32_t ep = p.entry[qi];
+        if (ep >= p.n) ep = 0;
+        __syncthreads();
+        if (warp == 0) {
+            const float dep = row_dist(ep);
+            if (lane == 0) {
+                bits[ep >> 5] |= 1u << (ep & 31u);
+                beam(0)[0] = dep;
+                reinterpret_cast<uint32_t*>(beam(0) + p.L_max)[0] = ep;
+                const bool in = dep <= r2f;
+                if (in) clist[0] = ep;
+                s_u[kNcand] = in ? 1u : 0u;
+                s_u[kOver] = 0u;
+            }
+        }
+        __syncthreads();
+        uint32_t buf = 0, size = 1, cur = 0, nvis = 1, nexp = 0, nfl = 0, head = 0;
+        uint32_t ncand = s_u[kNcand];
+        bool over = false, flood = false;
+        // warp 0: links of the next node to expand, requested an expansion ahead
+        uint32_t pre_node = kEmpty, pl0 = kEmpty, pl1 = kEmpty, pdg = 0;
+        for (;;) {
+            const float* bd = beam(buf);
+            uint32_t* bi = reinterpret_cast<uint32_t*>(beam(buf) + p.L_max);
+            uint32_t node, nxt = 0;
+            if (!flood) {
+                if (cur >= size || over) {
+                    flood = true;
+                    continue;
+                }
+                node = bi[cur] & kIdMask;
+                nexp++;
+                nxt = size;
+                for (uint32_t s0 = cur + 1; s0 < size; s0 += 32) {
+                    const uint32_t idx = s0 + lane;
+                    const unsigned b = __ballot_sync(kFull, idx < size && !(bi[idx] & kExpanded));
+                    if (b) {
+                        nxt = s0 + __ffs(b) - 1;
+                        break;
+                    }
+                }
+            } else {
+                if (head >= ncand || over) break;
+                node = cand_at(head++);
+                nfl++;
+            }
+            if (warp == 0) {
+                uint32_t l0 = pl0, l1 = pl1, dg = pdg;
+                if (node != pre_node) load_links(p, node, lane, l0, l1, dg);
+                if (!flood && nxt < size) {
+                    pre_node = bi[nxt] & kIdMask;
+                    load_links(p, pre_node, lane, pl0, pl1, pdg);
+                } else if (flood && head < ncand) {
+                    pre_node = cand_at(head);
+                    load_links(p, pre_node, lane, pl0, pl1, pdg);
+                }
+                bool f0 = false, f1 = false, bad = false;
+                if (lane < dg) {
+                    if (l0 < p.n) f0 = visit_first(bits, l0);
+                    else bad = true;
+                }
+                if (lane + 32 < dg) {
+                    if (l1 < p.n) f1 = visit_first(bits, l1);
+                    else bad = true;
+                }
+                if (bad) set_error(p.err, kDevBadId);
+                const unsigned b0 = __ballot_sync(kFull, f0), b1 = __ballot_sync(kFull, f1);
+                const uint32_t lt = lanemask_lt();
+                if (f0) ni[__popc(b0 & lt)] = l0;
+                if (f1) ni[__popc(b0) + __popc(b1 & lt)] = l1;
+                if (lane == 0) {
+                    s_u[kM] = __popc(b0) + __popc(b1);
+                    if (!flood) bi[cur] = node | kExpanded;
+                }
+            }
+            __syncthreads();
+            const uint32_t m = s_u[kM];
+            nvis += m;
+            if (m == 0) {
+                // nothing new; the barrier keeps the next expansion's kM apart from this one's
+                __syncthreads();
+                if (!flood) cur = nxt;
+                continue;
+            }
+            if (warp * 8 < m) {
+                const float d = row_dist(ni[min(grp, m - 1)]);
+                if (gt == 0 && grp < m) nd[grp] = d;
+            }
+            __syncthreads();
+            if (warp == 7) {
+                // in-range neighbours join the candidate / flood list in link order
+                const bool in0 = lane < m && nd[lane] <= r2f, in1 = lane + 32 < m && nd[lane + 32] <= r2f;
+                const unsigned b0 = __ballot_sync(kFull, in0), b1 = __ballot_sync(kFull, in1);
+                const uint32_t lt = lanemask_lt();
+                const uint32_t p0 = ncand + __popc(b0 & lt), p1 = ncand + __popc(b0) + __popc(b1 & lt);
+                if (in0 && p0 < p.cand_cap) cand_at(p0) = ni[lane];
+                if (in1 && p1 < p.cand_cap) cand_at(p1) = ni[lane + 32];
+                const uint32_t tot = ncand + __popc(b0) + __popc(b1);
+                if (lane == 0) {
+                    s_u[kNcand] = min(tot, p.cand_cap);
+                    if (tot > p.cand_cap) s_u[kOver] = 1u;
+                }
+            }
+            uint32_t mk = 0;
+            if (!flood) {
+                // rank of fresh entry grp: each thread of its group counts a quarter
+                const bool full = size >= L;
+                const bool mine = grp < m;
+                const float dv = mine ? nd[grp] : 0.f;
+                const uint32_t iv = mine ? ni[grp] : kEmpty;
+                uint32_t rank = 0;
+                if (mine)
+                    for (uint32_t x = gt; x < m; x += 4) rank += ord(nd[x], ni[x], dv, iv) ? 1u : 0u;
+                rank += __shfl_xor_sync(kFull, rank, 1);
+                rank += __shfl_xor_sync(kFull, rank, 2);
+                if (mine && gt == 0) {
+                    sd[rank] = dv;
+                    si[rank] = iv;
+                }
+                const bool keep = mine && gt == 0 && (!full || ord(dv, iv, bd[L - 1], bi[L - 1]));
+                mk = __syncthreads_count(keep);
+            } else {
+                __syncthreads();
+            }
+            ncand = s_u[kNcand];
+            over = s_u[kOver] != 0u;
+            if (flood) continue;
+            if (mk == 0) {
+                cur = nxt;
+                continue;
+            }
+            // merge into the other buffer: fresh entry r (of the mk kept, a
+            // prefix of the sorted) lands at r + (beam entries before it), beam
+            // entry j at j + (fresh entries before it)
+            const uint32_t ns = min(L, size + mk);
+            float* od = beam(buf ^ 1);
+            uint32_t* oi = reinterpret_cast<uint32_t*>(od + p.L_max);
+            if (warp < 2) {
+                uint32_t r0 = 0;
+                if (t < mk) {
+                    r0 = lower_rank(bd, bi, size, sd[t], si[t], ord);
+                    if (t + r0 < ns) {
+                        od[t + r0] = sd[t];
+                        oi[t + r0] = si[t];
+                    }
+                }
+                if (warp == 0) {
+                    const uint32_t cn = __shfl_sync(kFull, r0, 0);
+                    if (!(nxt < cn)) {
+                        pre_node = si[0];
+                        load_links(p, pre_node, lane, pl0, pl1, pdg);
+                    }
+                    if (lane == 0) s_u[kCn] = cn;
+                }
+            }
+            // the warps without fresh entries take the beam entries first
+            for (uint32_t j = (t + kBlockThreads - 64) % kBlockThreads; j < size; j += kBlockThreads) {
+                const float dv = bd[j];
+                const uint32_t iv = bi[j];
+                const uint32_t pos = j + lower_rank(sd, si, mk, dv, iv, ord);
+                if (pos < ns) {
+                    od[pos] = dv;
+                    oi[pos] = iv;
+                }
+            }
+            __syncthreads();
+            const uint32_t cn = s_u[kCn];
+            cur = nxt < cn ? nxt : cn;
+            size = ns;
+            buf ^= 1u;
+        }
+        if (over && t == 0) set_error(p.err, kDevCandOverflow);
+
+        // ---- candidates out (optional), then the postfilter (see rknn_search_kernel)
+        if (p.keep_cand) {
+            if (t == 0) {
+                const unsigned long long at = atomicAdd(&p.fill[1], (unsigned long long)ncand);
+                if (at + ncand > p.cand_out_cap) set_error(p.err, kDevOutOverflow);
+                p.cand_at[qi] = at;
+                reinterpret_cast<unsigned long long*>(s_u + kAt + 2)[0] = at;
+            }
+            __syncthreads();
+            const unsigned long long at = reinterpret_cast<unsigned long long*>(s_u + kAt + 2)[0];
+            if (at + ncand <= p.cand_out_cap)
+                for (uint32_t i = t; i < ncand; i += kBlockThreads) p.cand_buf[at + i] = p.perm[cand_at(i)];
+            __syncthreads();
+        } else if (t == 0) {
+            p.cand_at[qi] = 0;
+        }
+        const float qn = group_ip(q, q, p.d, gt, kFull);
+        const float* thr = p.thr + (size_t)tslot * p.n;
+        uint32_t npred = 0;
+        for (uint32_t r0 = 0; r0 < ncand; r0 += kBlockThreads / 4) {
+            const uint32_t idx = r0 + grp;
+            const bool ok = idx < ncand;
+            const uint32_t o = cand_at(ok ? idx : r0);
+            const float ip = group_ip(p.base + (size_t)o * p.bstride, q, p.d, gt, kFull);
+            const float key = p.ip ? -ip : __fsub_rn(__fadd_rn(p.onorm[o], qn), __fmul_rn(2.0f, ip));
+            const bool pass = ok && gt == 0 && key <= thr[o];
+            const unsigned b = __ballot_sync(kFull, pass);
+            if (lane == 0) s_u[kWarpCnt + warp] = __popc(b);
+            __syncthreads();
+            uint32_t before = npred, all = 0;
+            for (uint32_t w = 0; w < kBlockThreads / 32; w++) {
+                const uint32_t c = s_u[kWarpCnt + w];
+                if (w < warp) before += c;
+                all += c;
+            }
+            if (pass) cand_at(before + __popc(b & lanemask_lt())) = o;
+            npred += all;
+            __syncthreads();
+        }
+        if (t == 0) {
+            const unsigned long long at = atomicAdd(&p.fill[0], (unsigned long long)npred);
+            if (at + npred > p.pred_cap) set_error(p.err, kDevOutOverflow);
+            p.npred[qi] = npred;
+            p.ncand[qi] = ncand;
+            p.ndist[qi] = nvis;
+            p.nexp[qi] = nexp;
+            p.nflood[qi] = nfl;
+            p.pred_at[qi] = at;
+            reinterpret_cast<unsigned long long*>(s_u + kAt + 2)[0] = at;
+        }
+        __syncthreads();
+        const unsigned long long at = reinterpret_cast<unsigned long long*>(s_u + kAt + 2)[0];
+        if (at + npred <= p.pred_cap)
+            for (uint32_t i = t; i < npred; i += kBlockThreads) p.pred_buf[at + i] = p.perm[cand_at(i)];
+    }
+}
+
 // Query lift and RP-tree entry (rknn_query.cpp:2724-2729, rptrees.h:108-124;
 // |margin| <= EPS goes left): every 4-lane group of a warp descends for its
 // own query (qpw queries per warp, 8 unless the rows are long), staging each
@@ -851,6 +1143,7 @@ struct SearchCfg {
     uint32_t post_rows = 8; // candidate tile
     uint32_t blocks = 0;
     size_t smem = 0;
+    bool block = false;     // one block per query (rknn_search_block_kernel)
     uint64_t code() const { return hash_cap | (uint64_t)gcap << 24 | (uint64_t)wpb << 48 | (uint64_t)post_rows << 56; }
 };
 
@@ -868,6 +1161,33 @@ static int search_cfg(Ctx* c, uint32_t hash_cap, uint32_t gcap, uint32_t wpb, ui
     ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, cfg.smem));
     if (per_sm < 1) return ANQI_ERR_ARGS;
     cfg.blocks = std::min<uint32_t>((uint32_t)per_sm * c->sm_count, (b.nq + wpb - 1) / wpb);
+    return ANQI_OK;
+}
+
+// The block-per-query form, when every query of the batch gets a block at once
+// (below that a query's latency is the batch's; above it queries would wait for
+// a free block while the warp-per-query form holds many more at once) and the
+// rows are short enough for a 4-thread group each.  ANQI_B200_BLOCK=0 turns it off.
+static SearchKernel block_kernel_for(uint32_t dim) {
+    return dim == kColsDim ? rknn_search_block_kernel<kColsDim> : rknn_search_block_kernel<0>;
+}
+static int block_cfg(Ctx* c, SearchCfg& cfg, bool* fits) {
+    const Batch& b = c->batch;
+    *fits = false;
+    const char* env = std::getenv("ANQI_B200_BLOCK");
+    const size_t smem = block_search_words(b.L_max, c->ix.lstride, c->ix.n) * 4;
+    if ((env && env[0] == '0') || c->inject || smem > 227 * 1024 || stage_rows_for(c->ix.lstride, c->ix.bstride) != 8)
+        return ANQI_OK;
+    auto kern = block_kernel_for(c->ix.dim);
+    ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlockThreads, smem));
+    if ((uint64_t)per_sm * c->sm_count < b.nq) return ANQI_OK;
+    cfg.block = true;
+    cfg.wpb = kBlockThreads / 32;
+    cfg.blocks = b.nq;
+    cfg.smem = smem;
+    *fits = true;
     return ANQI_OK;
 }
 
@@ -1096,9 +1416,9 @@ extern "C" int anqi_query_upload(anqi_ctx* h, const float* queries, uint32_t nq,
 
 extern "C" {
 
-// Entry objects of the batch (lift + RP-tree descent) and, unless
-// ANQI_B200_ORDER=0, the work list ordered by entry leaf.
-static int prepare_entries(Ctx* c, bool* ordered) {
+// Entry objects of the batch (lift + RP-tree descent) and, when `order` is set
+// and unless ANQI_B200_ORDER=0, the work list ordered by entry leaf.
+static int prepare_entries(Ctx* c, bool order, bool* ordered) {
     Batch& b = c->batch;
     const QueryIndex& ix = c->ix;
     int rc;
@@ -1133,7 +1453,7 @@ static int prepare_entries(Ctx* c, bool* ordered) {
     const uint32_t blocks = std::min<uint32_t>(c->sm_count * 8, (nq + 4 * qpw - 1) / (4 * qpw));
     rknn_entry_kernel<<<blocks, 128, smem, c->stream>>>(p, b.enode.as<uint32_t>(), b.entry.as<uint32_t>(), qpw);
     const char* env = std::getenv("ANQI_B200_ORDER");
-    *ordered = !(env && env[0] == '0');
+    *ordered = order && !(env && env[0] == '0');
     if (*ordered) {
         uint32_t* cnt = b.leaf_cnt.as<uint32_t>();
         uint32_t* cursor = cnt + ix.tree_nodes + 1;
@@ -1222,7 +1542,7 @@ static int enqueue_search(Ctx* c, const SearchCfg& cfg, int keep_candidates, boo
     p.gtab = cfg.gcap ? c->vis_gtab.as<uint32_t>() : nullptr;
     p.drop_row_copies = (c->inject & ANQI_FAULT_DROP_ROW_COPIES) ? 1u : 0u;
     p.post_rows = cfg.post_rows;
-    auto kern = search_kernel_for(ix.dim, cfg.wpb);
+    auto kern = cfg.block ? block_kernel_for(ix.dim) : search_kernel_for(ix.dim, cfg.wpb);
     ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem));
     // in a captured graph the events become event-record nodes (so the replay
     // is timed like a plain launch)
@@ -1311,7 +1631,14 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
     static const uint32_t kShapes[][2] = {{4, 8}, {2, 8}, {8, 8}, {4, 4}, {2, 4}, {8, 4}};
     // cfgs: every (visited set, shape) candidate; the first shape is the default
     std::vector<SearchCfg> cfgs;
+    SearchCfg blk;
+    bool use_block = false;
+    if (!forced && !fshape) {
+        if ((rc = block_cfg(c, blk, &use_block))) return rc;
+        if (use_block) cfgs.push_back(blk);
+    }
     for (const auto& shape : kShapes) {
+        if (use_block) break;
         if (fshape && (shape[0] != f_w || (f_t && shape[1] != f_t))) continue;
         for (const auto& cand : kCandidates) {
             if (forced && (cand[0] != f_hc || cand[1] != f_gc)) continue;
@@ -1357,14 +1684,16 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
         c->log_cap = log_cap;
         c->cand_cap = cand_cap;
     }
-    if ((rc = prepare_entries(c, &b.ordered))) return rc;
+    if ((rc = prepare_entries(c, !use_block, &b.ordered))) return rc;
     if (b.pred_cap == 0) b.pred_cap = std::max<uint64_t>(1024, (uint64_t)b.nq * 128);
     if (keep_candidates && b.cand_cap == 0) b.cand_cap = std::max<uint64_t>(1024, (uint64_t)b.nq * 256);
     // autotune once per (n, L_max, nq): time every configuration, keep the fastest
     const uint64_t key = ix.n * 1000003ull ^ ((uint64_t)b.L_max << 40) ^ ((uint64_t)b.nq << 20);
     SearchCfg best = cfgs[0];
     auto it = c->tuned.find(key);
-    if (it != c->tuned.end()) {
+    if (use_block) {
+        // one configuration, chosen by the batch's size
+    } else if (it != c->tuned.end()) {
         for (const SearchCfg& g : cfgs)
             if (g.code() == it->second) best = g;
     } else if (cfgs.size() > 1) {
@@ -1416,6 +1745,7 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
         c->last_cfg_smem = best.smem;
         c->last_cfg_wpb = best.wpb;
         c->last_cfg_post = best.post_rows;
+        c->last_cfg_block = best.block;
         b.have_results = true;
         b.have_cands = keep_candidates != 0;
         if (st) {
@@ -1444,7 +1774,7 @@ static std::vector<uint64_t> query_graph_key(Ctx* c, int keep_candidates) {
     auto u = [](const void* q) { return (uint64_t)(uintptr_t)q; };
     return {b.nq, b.L_max, (uint64_t)b.has_k, (uint64_t)b.has_L, b.k_all, b.L_all, (uint64_t)keep_candidates,
             (uint64_t)b.ordered, c->last_cfg_hash, c->last_cfg_gcap, c->last_cfg_blocks, c->last_cfg_smem,
-            c->last_cfg_wpb, c->last_cfg_post,
+            c->last_cfg_wpb, c->last_cfg_post, (uint64_t)c->last_cfg_block,
             b.pred_cap, b.cand_cap, u(b.q.p), u(b.qslot.p), u(b.qL.p), u(b.pred_buf.p), u(b.cand_buf.p),
             u(b.pred_csr.p), u(b.cand_csr.p), u(b.pred_off.p), u(b.cand_off.p), u(b.entry.p), u(b.enode.p),
             u(b.order.p), u(b.leaf_cnt.p), u(b.npred.p), u(b.ncand.p), u(b.ndist.p), u(b.nexp.p), u(b.nflood.p),
@@ -1519,10 +1849,11 @@ int anqi_query_run_graph(anqi_ctx* h, int keep_candidates, anqi_query_stats* st)
     cfg.smem = c->last_cfg_smem;
     cfg.wpb = c->last_cfg_wpb;
     cfg.post_rows = c->last_cfg_post;
+    cfg.block = c->last_cfg_block;
     bool ordered = false;
     cudaGraph_t g = nullptr;
     ANQI_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = prepare_entries(c, &ordered);
+    rc = prepare_entries(c, !cfg.block, &ordered);
     if (!rc) rc = enqueue_search(c, cfg, keep_candidates, true);
     if (!rc) rc = enqueue_compaction(c, keep_candidates);
     const cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
