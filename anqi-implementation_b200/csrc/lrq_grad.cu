@@ -16,8 +16,12 @@
 //   dL/dmu[k]  = 2/(n nk) sum_o (r[o,k] - sum_m G[m,k] s[o,m]),  s = r G^T
 //   dL/dG[m,k] = 2/(n nk) sum_o (r[o,k] c[o,m] + (T[o,k] - mu[k]) s[o,m])
 //
-// One warp per row, lanes over the nk columns.  Entry points take device
-// pointers and a stream and allocate nothing.
+// Forward and the basis half of the backward: one warp per row, lanes over the
+// nk columns, one resident block per SM; the codebook half of the backward: a
+// histogram per column.  Entry points take device pointers and a stream and
+// allocate nothing.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -32,17 +36,34 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// decode_nearest on one ascending codebook row.
-__device__ __forceinline__ uint32_t nearest_code(const double* __restrict__ row, uint32_t cs, double v) {
-    uint32_t lo = 0, hi = cs;  // first index with row[i] >= v
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (row[mid] < v) lo = mid + 1;
-        else hi = mid;
+// Warp sums of M values at once (M = 8 or 16): every step halves the values a
+// lane still carries, so M = 8 takes 9 exchanges instead of 40.  Each value is
+// summed in warp_sum's tree (partners 16, 8, 4, 2, 1 apart), so the bits are
+// the same.  Returns the sum of value sum_index<M>(lane).
+template <uint32_t M>
+__device__ __forceinline__ double warp_sum_many(double (&v)[M], uint32_t lane) {
+    uint32_t o = 16;
+#pragma unroll
+    for (uint32_t h = M / 2; h > 0; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (uint32_t i = 0; i < h; i++) {
+            const double mine = up ? v[i + h] : v[i];
+            const double other = up ? v[i] : v[i + h];
+            v[i] = mine + __shfl_xor_sync(kWarp, other, o);
+        }
     }
-    const uint32_t high = lo < cs ? lo : cs - 1;
-    const uint32_t low = lo > 0 ? lo - 1 : 0;
-    return fabs(row[high] - v) < fabs(v - row[low]) ? high : low;
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(kWarp, v[0], o);
+    return v[0];
+}
+// The value a lane receives, and the first lane that receives value i.
+template <uint32_t M>
+__device__ __forceinline__ uint32_t sum_index(uint32_t lane) {
+    return lane / (32 / M);
+}
+template <uint32_t M>
+__device__ __forceinline__ uint32_t sum_lane(uint32_t i) {
+    return i * (32 / M);
 }
 
 struct ObjParams {
@@ -57,57 +78,167 @@ struct ObjParams {
     double* c;
     uint8_t* a;
     double* loss;             // one accumulator, zeroed by the host
+    uint32_t bcols, bpitch;   // codebook rows kept in shared memory (whole groups of 32 columns, or all), and their
+                              // pitch: the next power of two plus one (odd: lanes on different banks)
 };
 
-// M: compile-time bound on the rank (m <= M), so per-rank values stay in registers.
-template <uint32_t M>
-__global__ void lrq_objective_forward_kernel(ObjParams p) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    double part = 0.0;
-    for (uint64_t o = w; o < p.n; o += nw) {
-        const double* t = p.T + o * p.nk;
-        double tv[kMaxCols], cen[kMaxCols];
+extern __shared__ __align__(16) double s_lrq[];
+
+// decode_nearest on the lane's column of each group of 32: first index with
+// row[i] >= v, then the closer of it and its predecessor, the lower on ties.
+// The kMaxCols searches run side by side.
+template <class Row>
+__device__ __forceinline__ void nearest_codes(const Row& row, uint32_t nk, uint32_t cs, uint32_t lane, uint32_t j0,
+                                              uint32_t j1, const double (&v)[kMaxCols], uint32_t (&code)[kMaxCols]) {
+    uint32_t lo[kMaxCols];
+#pragma unroll
+    for (uint32_t j = 0; j < kMaxCols; j++) lo[j] = 0;
+#pragma unroll 1
+    for (uint32_t step = 256; step > 0; step >>= 1) {
 #pragma unroll
         for (uint32_t j = 0; j < kMaxCols; j++) {
-            const uint32_t k = lane + 32 * j;
-            tv[j] = k < p.nk ? t[k] : 0.0;
-            cen[j] = k < p.nk ? tv[j] - p.mu[k] : 0.0;
+            if (j < j0 || j >= j1 || lane + 32 * j >= nk) continue;
+            if (lo[j] + step <= cs && row(j)[lo[j] + step - 1] < v[j]) lo[j] += step;
         }
-        double cm[M];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kMaxCols; j++) {
+        if (j < j0 || j >= j1 || lane + 32 * j >= nk) continue;
+        const uint32_t high = lo[j] < cs ? lo[j] : cs - 1;
+        const uint32_t low = lo[j] > 0 ? lo[j] - 1 : 0;
+        code[j] = fabs(row(j)[high] - v[j]) < fabs(v[j] - row(j)[low]) ? high : low;
+    }
+}
+
+// The same on codebook rows in shared memory, padded with +inf to a power of
+// two: a halving step is one load at a constant offset from the running
+// position, a compare and a predicated add, without bounds.
+// Lanes past the last of the `rows` rows search that one (their codes are not
+// used).
+__device__ __forceinline__ void nearest_codes_padded(const double* sB, uint32_t pitch, uint32_t cs, uint32_t rows,
+                                                     uint32_t lane, const double (&v)[kMaxCols],
+                                                     uint32_t (&code)[kMaxCols]) {
+    const uint32_t top = pitch - 1;  // the padded row length
+    uint32_t at[kMaxCols];
+#pragma unroll
+    for (uint32_t j = 0; j < kMaxCols; j++) at[j] = min(lane + 32 * j, rows - 1) * pitch;
+#pragma unroll
+    for (uint32_t step = 128; step > 0; step >>= 1) {
+        if (step >= top) continue;
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++)
+            if (sB[at[j] + step - 1] < v[j]) at[j] += step;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kMaxCols; j++) {
+        const uint32_t r0 = min(lane + 32 * j, rows - 1) * pitch;
+        const uint32_t lo = at[j] - r0 + (sB[at[j]] < v[j] ? 1u : 0u);
+        const uint32_t high = lo < cs ? lo : cs - 1;
+        const uint32_t low = lo > 0 ? lo - 1 : 0;
+        code[j] = fabs(sB[r0 + high] - v[j]) < fabs(v[j] - sB[r0 + low]) ? high : low;
+    }
+}
+
+// M: compile-time bound on the rank (m <= M).  One block per SM holds the
+// codebook in shared memory (as many columns as fit; the rest is read through
+// L1) and the basis, and walks the rows with the next row's cutoffs on their
+// way.  Bound by latency and issue of the nine dependent shared-memory gathers
+// of the code search (lanes in different codebook rows, about four bank
+// conflicts each).  120,000 x 100, rank 8, 256 codes: 526 us with the codebook
+// read from global memory by 8 blocks of 8 warps an SM, 174 us now.
+template <uint32_t M, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads, 1) lrq_objective_forward_kernel(ObjParams p) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t w = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * kThreads) >> 5;
+    double* sG = s_lrq;                              // M x 128 (columns past nk and ranks past m zero)
+    double* sB = s_lrq + M * 32 * kMaxCols;          // bcols x bpitch
+    for (uint32_t t = threadIdx.x; t < M * 32 * kMaxCols; t += kThreads) {
+        const uint32_t mm = t / (32 * kMaxCols), k = t % (32 * kMaxCols);
+        sG[t] = mm < p.m && k < p.nk ? p.G[(size_t)mm * p.nk + k] : 0.0;
+    }
+    if (!p.codes_in)
+        for (uint32_t k = threadIdx.x >> 5; k < p.bcols; k += kThreads / 32)
+            for (uint32_t i = lane; i < p.bpitch; i += 32)
+                sB[k * p.bpitch + i] = i < p.cs ? p.B[(size_t)k * p.cs + i] : __longlong_as_double(0x7ff0000000000000ll);
+    __syncthreads();
+    double mu[kMaxCols];
+#pragma unroll
+    for (uint32_t j = 0; j < kMaxCols; j++) mu[j] = lane + 32 * j < p.nk ? p.mu[lane + 32 * j] : 0.0;
+    // the lane's columns of the basis stay in registers up to rank 8
+    double gr[M == 8 ? M : 1][kMaxCols];
+    if constexpr (M == 8) {
+#pragma unroll
+        for (uint32_t mm = 0; mm < M; mm++)
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++) gr[mm][j] = sG[mm * 32 * kMaxCols + 32 * j + lane];
+    }
+    auto g = [&](uint32_t mm, uint32_t j) {
+        if constexpr (M == 8) return gr[mm][j];
+        else return sG[mm * 32 * kMaxCols + 32 * j + lane];
+    };
+    const uint32_t jb = (p.bcols + 31) / 32;  // column groups in shared memory
+    double part = 0.0;
+    double nxt[kMaxCols];
+    auto load = [&](uint64_t o) {
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++)
+            nxt[j] = o < p.n && lane + 32 * j < p.nk ? p.T[o * p.nk + lane + 32 * j] : 0.0;
+    };
+    load(w);
+    for (uint64_t o = w; o < p.n; o += nw) {
+        double tv[kMaxCols], v[kMaxCols], base[kMaxCols];
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++) {
+            tv[j] = nxt[j];
+            v[j] = lane + 32 * j < p.nk ? tv[j] - mu[j] : 0.0;
+            base[j] = mu[j];
+        }
+        load(o + nw);
+        double s[M];
 #pragma unroll
         for (uint32_t mm = 0; mm < M; mm++) {
-            cm[mm] = 0.0;
-            if (mm >= p.m) continue;
-            double s = 0.0;
+            s[mm] = 0.0;
 #pragma unroll
-            for (uint32_t j = 0; j < kMaxCols; j++) {
-                const uint32_t k = lane + 32 * j;
-                if (k < p.nk) s = fma(cen[j], p.G[(size_t)mm * p.nk + k], s);
-            }
-            cm[mm] = warp_sum(s);
-            if (lane == 0) p.c[o * p.m + mm] = cm[mm];
+            for (uint32_t j = 0; j < kMaxCols; j++)
+                if (32 * j < p.nk) s[mm] = fma(v[j], g(mm, j), s[mm]);
+        }
+        const double cm = warp_sum_many<M>(s, lane);
+        const uint32_t ci = sum_index<M>(lane);
+        if (lane == sum_lane<M>(ci) && ci < p.m) p.c[o * p.m + ci] = cm;
+#pragma unroll
+        for (uint32_t mm = 0; mm < M; mm++) {
+            if (mm >= p.m) break;
+            const double cv = __shfl_sync(kWarp, cm, sum_lane<M>(mm));
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++)
+                if (32 * j < p.nk) base[j] = fma(cv, g(mm, j), base[j]);
+        }
+        uint32_t code[kMaxCols] = {0, 0, 0, 0};
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++) v[j] = tv[j] - base[j];
+        if (p.codes_in) {
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++)
+                if (lane + 32 * j < p.nk) code[j] = min((uint32_t)p.codes_in[o * p.nk + lane + 32 * j], p.cs - 1);
+        } else {
+            auto in_global = [&](uint32_t j) { return p.B + (size_t)(lane + 32 * j) * p.cs; };
+            if (p.bcols) nearest_codes_padded(sB, p.bpitch, p.cs, p.bcols, lane, v, code);
+            if (32 * jb < p.nk) nearest_codes(in_global, p.nk, p.cs, lane, jb, kMaxCols, v, code);
         }
 #pragma unroll
         for (uint32_t j = 0; j < kMaxCols; j++) {
             const uint32_t k = lane + 32 * j;
             if (k >= p.nk) continue;
-            double base = p.mu[k];
-#pragma unroll
-            for (uint32_t mm = 0; mm < M; mm++)
-                if (mm < p.m) base = fma(cm[mm], p.G[(size_t)mm * p.nk + k], base);
-            const double* row = p.B + (size_t)k * p.cs;
-            const uint32_t code =
-                p.codes_in ? min((uint32_t)p.codes_in[o * p.nk + k], p.cs - 1) : nearest_code(row, p.cs, tv[j] - base);
-            const double rv = base + row[code] - tv[j];
+            const double b = !p.codes_in && j < jb ? sB[(size_t)k * p.bpitch + code[j]] : p.B[(size_t)k * p.cs + code[j]];
+            const double rv = base[j] + b - tv[j];
             p.r[o * p.nk + k] = rv;
-            p.a[o * p.nk + k] = (uint8_t)code;
+            p.a[o * p.nk + k] = (uint8_t)code[j];
             part = fma(rv, rv, part);
         }
     }
     part = warp_sum(part);
-    if (lane == 0) atomicAdd(p.loss, part);
+    if (lane == 0 && part != 0.0) atomicAdd(p.loss, part);
 }
 
 struct GradParams {
@@ -125,65 +256,181 @@ struct GradParams {
     double* g_B;
 };
 
-template <uint32_t M>
-__global__ void lrq_objective_backward_kernel(GradParams p) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    double gmu[kMaxCols] = {0, 0, 0, 0};
-    double gG[M][kMaxCols];
-#pragma unroll
-    for (uint32_t mm = 0; mm < M; mm++)
-#pragma unroll
-        for (uint32_t j = 0; j < kMaxCols; j++) gG[mm][j] = 0.0;
-    for (uint64_t o = w; o < p.n; o += nw) {
-        double rv[kMaxCols], cen[kMaxCols];
-#pragma unroll
-        for (uint32_t j = 0; j < kMaxCols; j++) {
-            const uint32_t k = lane + 32 * j;
-            rv[j] = k < p.nk ? p.r[o * p.nk + k] : 0.0;
-            cen[j] = k < p.nk ? p.T[o * p.nk + k] - p.mu[k] : 0.0;
-            if (k < p.nk) atomicAdd(p.g_B + (size_t)k * p.cs + p.a[o * p.nk + k], p.scale * rv[j]);
-        }
-#pragma unroll
-        for (uint32_t mm = 0; mm < M; mm++) {
-            if (mm >= p.m) continue;
-            double s = 0.0;
-#pragma unroll
-            for (uint32_t j = 0; j < kMaxCols; j++) {
-                const uint32_t k = lane + 32 * j;
-                if (k < p.nk) s = fma(p.G[(size_t)mm * p.nk + k], rv[j], s);
-            }
-            s = warp_sum(s);
-            const double cm = p.c[o * p.m + mm];
-#pragma unroll
-            for (uint32_t j = 0; j < kMaxCols; j++) {
-                const uint32_t k = lane + 32 * j;
-                if (k >= p.nk) continue;
-                gmu[j] = fma(-p.G[(size_t)mm * p.nk + k], s, gmu[j]);
-                gG[mm][j] = fma(rv[j], cm, fma(cen[j], s, gG[mm][j]));
-            }
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < kMaxCols; j++) gmu[j] += rv[j];
+// Gradients of mu and G.  A warp keeps its lanes' columns of both in registers
+// over all its rows; mu's needs only the sums of s over the rows,
+// sum_o r - G^T (sum_o s).  The block's warps add up in shared memory first:
+// per-warp atomics to the same m nk + nk addresses, with the codebook's, were
+// most of the backward's 529 us at 120,000 x 100; now 95 us, bound by the FP64
+// and shuffle work of a row.
+template <uint32_t M, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads, 1) lrq_objective_backward_kernel(GradParams p) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t w = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * kThreads) >> 5;
+    constexpr uint32_t kRow = 32 * kMaxCols;
+    double* sG = s_lrq;               // M x 128
+    double* acc = s_lrq + M * kRow;   // (M + 1) x 128: block sums of g_G, then g_mu
+    for (uint32_t t = threadIdx.x; t < M * kRow; t += kThreads) {
+        const uint32_t mm = t / kRow, k = t % kRow;
+        sG[t] = mm < p.m && k < p.nk ? p.G[(size_t)mm * p.nk + k] : 0.0;
     }
+    for (uint32_t t = threadIdx.x; t < (M + 1) * kRow; t += kThreads) acc[t] = 0.0;
+    __syncthreads();
+    double mu[kMaxCols], gmu[kMaxCols], gG[M][kMaxCols], ssum = 0.0;
 #pragma unroll
     for (uint32_t j = 0; j < kMaxCols; j++) {
-        const uint32_t k = lane + 32 * j;
-        if (k >= p.nk) continue;
-        atomicAdd(p.g_mu + k, p.scale * gmu[j]);
+        mu[j] = lane + 32 * j < p.nk ? p.mu[lane + 32 * j] : 0.0;
+        gmu[j] = 0.0;
 #pragma unroll
-        for (uint32_t mm = 0; mm < M; mm++)
-            if (mm < p.m) atomicAdd(p.g_G + (size_t)mm * p.nk + k, p.scale * gG[mm][j]);
+        for (uint32_t mm = 0; mm < M; mm++) gG[mm][j] = 0.0;
+    }
+    // the next row's residuals, cutoffs and coefficients are on their way while
+    // this one is added
+    double nr[kMaxCols], nt[kMaxCols], nc = 0.0;
+    auto load = [&](uint64_t o) {
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++) {
+            const bool in = o < p.n && lane + 32 * j < p.nk;
+            nr[j] = in ? p.r[o * p.nk + lane + 32 * j] : 0.0;
+            nt[j] = in ? p.T[o * p.nk + lane + 32 * j] : 0.0;
+        }
+        nc = o < p.n && lane < p.m ? p.c[o * p.m + lane] : 0.0;
+    };
+    load(w);
+    for (uint64_t o = w; o < p.n; o += nw) {
+        double rv[kMaxCols], cen[kMaxCols], s[M];
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++) {
+            rv[j] = nr[j];
+            cen[j] = lane + 32 * j < p.nk ? nt[j] - mu[j] : 0.0;
+            gmu[j] += rv[j];
+        }
+        const double cl = nc;
+        load(o + nw);
+#pragma unroll
+        for (uint32_t mm = 0; mm < M; mm++) {
+            s[mm] = 0.0;
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++)
+                if (32 * j < p.nk) s[mm] = fma(sG[mm * kRow + 32 * j + lane], rv[j], s[mm]);
+        }
+        const double sm = warp_sum_many<M>(s, lane);
+        ssum += sm;
+#pragma unroll
+        for (uint32_t mm = 0; mm < M; mm++) {
+            if (mm >= p.m) break;
+            const double sv = __shfl_sync(kWarp, sm, sum_lane<M>(mm));
+            const double cv = __shfl_sync(kWarp, cl, mm);
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++)
+                if (32 * j < p.nk) gG[mm][j] = fma(rv[j], cv, fma(cen[j], sv, gG[mm][j]));
+        }
+    }
+#pragma unroll
+    for (uint32_t mm = 0; mm < M; mm++) {
+        const double sv = __shfl_sync(kWarp, ssum, sum_lane<M>(mm));
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxCols; j++) gmu[j] = fma(-sG[mm * kRow + 32 * j + lane], sv, gmu[j]);
+    }
+    for (uint32_t turn = 0; turn < kThreads / 32; turn++) {
+        if (turn == warp) {
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxCols; j++) {
+#pragma unroll
+                for (uint32_t mm = 0; mm < M; mm++) acc[mm * kRow + 32 * j + lane] += gG[mm][j];
+                acc[M * kRow + 32 * j + lane] += gmu[j];
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t t = threadIdx.x; t < (M + 1) * kRow; t += kThreads) {
+        const uint32_t mm = t / kRow, k = t % kRow;
+        if (k >= p.nk) continue;
+        if (mm == M) atomicAdd(p.g_mu + k, p.scale * acc[t]);
+        else if (mm < p.m) atomicAdd(p.g_G + (size_t)mm * p.nk + k, p.scale * acc[t]);
     }
 }
 
-// One warp per row, 8 warps per block, at most 8 blocks per SM (grid-stride).
-int launch_grid(uint64_t rows) {
+// Gradient of B: the sums of r by code.  A block has the histograms of 32
+// columns in shared memory, lane l of every warp adding to column l's (bank
+// pair l: no conflicts inside a warp, hardly any collisions between warps), and
+// adds them to g_B once (43 us at 120,000 x 100 x 256).  Adding every r to g_B in
+// global memory took an atomic per matrix entry.
+constexpr uint32_t kHistThreads = 1024;
+__global__ void __launch_bounds__(kHistThreads, 1) lrq_codebook_grad_kernel(GradParams p) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, k0 = blockIdx.x * 32, k = k0 + lane;
+    for (uint32_t t = threadIdx.x; t < p.cs * 32; t += kHistThreads) s_lrq[t] = 0.0;
+    __syncthreads();
+    constexpr uint32_t kAhead = 4, kWarps = kHistThreads / 32;
+    if (k < p.nk) {
+        for (uint64_t o = (uint64_t)blockIdx.y * kWarps + warp; o < p.n; o += (uint64_t)gridDim.y * kWarps * kAhead) {
+            double rv[kAhead];
+            uint32_t a[kAhead];
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; q++) {
+                const uint64_t row = o + (uint64_t)q * gridDim.y * kWarps;
+                const bool ok = row < p.n;
+                rv[q] = ok ? p.r[row * p.nk + k] : 0.0;
+                a[q] = ok ? min((uint32_t)p.a[row * p.nk + k], p.cs - 1) : 0u;
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kAhead; q++) atomicAdd(s_lrq + a[q] * 32 + lane, rv[q]);
+        }
+    }
+    __syncthreads();
+    // diagonally, so that a warp's reads fall on all banks
+    for (uint32_t t = threadIdx.x; t < p.cs * 32; t += kHistThreads) {
+        const uint32_t a = t >> 5, kk = ((t & 31u) + a) & 31u;
+        const double v = s_lrq[a * 32 + kk];
+        if (v != 0.0) atomicAdd(p.g_B + (size_t)(k0 + kk) * p.cs + a, p.scale * v);
+    }
+}
+
+int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return (int)std::min<uint64_t>((rows + 7) / 8, (uint64_t)sms * 8);
+    return sms;
+}
+
+constexpr size_t kSmemMax = 227 * 1024;
+
+// At least four rows a warp, so small inputs do not pay for filling every SM's
+// shared memory.
+template <uint32_t M, uint32_t kThreads>
+cudaError_t launch_forward(ObjParams p, cudaStream_t st) {
+    const size_t fixed = (size_t)M * 32 * kMaxCols * 8;
+    uint32_t top = 1;
+    while (top < p.cs) top <<= 1;
+    p.bpitch = top + 1;
+    const uint64_t fit = (kSmemMax - fixed) / (p.bpitch * 8ull);
+    p.bcols = fit >= p.nk ? p.nk : (uint32_t)fit / 32 * 32;
+    const size_t smem = fixed + (p.codes_in ? 0 : (size_t)p.bcols * p.bpitch * 8);
+    auto kern = lrq_objective_forward_kernel<M, kThreads>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    constexpr uint64_t rows = kThreads / 32 * 4;
+    kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
+    return cudaGetLastError();
+}
+
+template <uint32_t M, uint32_t kThreads>
+cudaError_t launch_backward(const GradParams& p, cudaStream_t st) {
+    const size_t smem = (size_t)(2 * M + 1) * 32 * kMaxCols * 8;
+    auto kern = lrq_objective_backward_kernel<M, kThreads>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    constexpr uint64_t rows = kThreads / 32 * 4;
+    kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // one block an SM, at least 64 rows a block
+    const size_t hist = (size_t)p.cs * 32 * 8;
+    e = cudaFuncSetAttribute(lrq_codebook_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist);
+    if (e != cudaSuccess) return e;
+    const uint32_t groups = (p.nk + 31) / 32;
+    const uint64_t rowgroups = std::min<uint64_t>((p.n + 63) / 64, std::max(1u, sm_count() / groups));
+    lrq_codebook_grad_kernel<<<dim3(groups, (unsigned)rowgroups), kHistThreads, hist, st>>>(p);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -200,10 +447,9 @@ int anqi_lrq_objective_forward(const double* T, uint64_t n, uint32_t nk, uint32_
     if (nk == 0 || nk > 32 * kMaxCols || m == 0 || m > 16 || cs == 0 || cs > 256) return ANQI_ERR_ARGS;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(loss, 0, sizeof(double), st) != cudaSuccess) return ANQI_ERR_DEVICE;
-    ObjParams p{T, n, nk, m, cs, mu, G, B, codes_in, r, c, a, loss};
-    if (m <= 8) lrq_objective_forward_kernel<8><<<launch_grid(n), 256, 0, st>>>(p);
-    else lrq_objective_forward_kernel<16><<<launch_grid(n), 256, 0, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
+    ObjParams p{T, n, nk, m, cs, mu, G, B, codes_in, r, c, a, loss, 0, 0};
+    const cudaError_t e = m <= 8 ? launch_forward<8, 384>(p, st) : launch_forward<16, 384>(p, st);
+    return e == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
 }
 
 int anqi_lrq_objective_backward(const double* T, uint64_t n, uint32_t nk, uint32_t m, const double* mu,
@@ -217,9 +463,8 @@ int anqi_lrq_objective_backward(const double* T, uint64_t n, uint32_t nk, uint32
         cudaMemsetAsync(g_B, 0, (size_t)nk * cs * sizeof(double), st) != cudaSuccess)
         return ANQI_ERR_DEVICE;
     GradParams p{T, n, nk, m, cs, mu, G, r, c, a, scale, g_mu, g_G, g_B};
-    if (m <= 8) lrq_objective_backward_kernel<8><<<launch_grid(n), 256, 0, st>>>(p);
-    else lrq_objective_backward_kernel<16><<<launch_grid(n), 256, 0, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
+    const cudaError_t e = m <= 8 ? launch_backward<8, 384>(p, st) : launch_backward<16, 256>(p, st);
+    return e == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
 }
 
 }  // extern "C"
