@@ -1,12 +1,13 @@
 // BF16 tensor-core (tcgen05) tiles for the brute-force distance work: the
 // exact ground truth (tools/dataset_gt.cpp:206-313) in the precision form.
 //
-// Rows are converted once to bf16 (padded to a multiple of 16).  A CTA of 4
-// warps owns a 128-row query tile resident in shared memory and streams
-// 128-row base tiles through a two-stage shared-memory ring; one thread
-// issues the K = 16 tcgen05.mma steps into one of two 128-column TMEM
-// accumulators while the four warps run the epilogue of the previous tile
-// (tcgen05.ld: thread = query row, 32 columns per load).
+// Rows are converted once to bf16 (padded to a multiple of 16).  Whole-matrix
+// work runs in tc_scan_kernel; init_knn's leaves in tc_filter_kernel, where a CTA
+// of 8 warps owns 128 rows of a leaf resident in shared memory and streams the
+// leaf's rows through a two-stage ring, one thread issuing the K = 16
+// tcgen05.mma steps into one of two 128-column TMEM accumulators while all run
+// the epilogue of the previous tile (tcgen05.ld: thread = row, 32 columns per
+// load).
 //
 // Epilogue: key~ = |q|^2 + |x|^2 - 2 <q~, x~> with the reference's FP32
 // norms.  A pair is a candidate when key~ - eps <= threshold, where eps bounds
@@ -151,8 +152,9 @@ __global__ void __launch_bounds__(128) gram_kernel(const __nv_bfloat16* __restri
 }
 
 // --------------------------------------------------------- filter
-// One CTA = 8 warps over a 128-row query tile; warp w reads TMEM lanes
-// 32 (w % 4) .. + 31 (its rows) and columns 64 (w / 4) .. + 63 of each tile.
+// The inputs of the leaf filter (one CTA = 8 warps over 128 rows of a leaf; warp
+// w reads TMEM lanes 32 (w % 4) .. + 31, its rows, and columns 64 (w / 4) .. +
+// 63 of each tile) and of the scan.
 struct FilterParams {
     const __nv_bfloat16* qb;  // query rows, bf16, dp wide
     const float* q32;         // query rows, FP32, stride xs
@@ -173,7 +175,6 @@ struct FilterParams {
     int exclude_self;         // skip j == query row (self top-K)
     const uint32_t* rows;     // query rows to process (null: 0 .. nrows-1)
     uint64_t nrows;
-    uint64_t split_len;       // base rows per grid.y slice (multiple of 128)
     uint32_t* cnt;            // per query row: hits (atomic; may exceed cap)
     uint32_t cap;
     uint32_t* out_id;         // row * cap + slot
@@ -252,8 +253,8 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     const uint32_t tile_bytes = kTile * (kWide ? kWideK : p.dp) * 2;
     unsigned char* sa = sm;
     unsigned char* sb = sm + (size_t)(kWide ? kWideStages : 1) * tile_bytes;
-    float* col = reinterpret_cast<float*>(sb + (size_t)(kWide ? kWideStages : kStages) * tile_bytes);  // kStages x 4 x 128
-    uint8_t* colint = reinterpret_cast<uint8_t*>(col + kStages * 4 * kTile);    // kStages x 128
+    float* col = reinterpret_cast<float*>(sb + (size_t)(kWide ? kWideStages : kStages) * tile_bytes);  // kStages x 3 x 128
+    uint8_t* colint = reinterpret_cast<uint8_t*>(col + kStages * 3 * kTile);    // kStages x 128
     uint64_t* rowid = reinterpret_cast<uint64_t*>(colint + kStages * kTile);    // 128 (aligned: 2*... bytes)
     uint32_t* colid = reinterpret_cast<uint32_t*>(rowid + kTile);                // kStages x 128 (leaf mode)
     __shared__ uint64_t bar[2];
@@ -264,23 +265,16 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     const uint32_t r = (warp & 3u) * 32 + lane;  // this thread's tile row / TMEM lane
     const uint32_t half = warp >> 2;             // column half of each tile
 
-    const bool leaf = p.leaf_tiles != nullptr;
-    const LeafTile lt = leaf ? p.leaf_tiles[blockIdx.x] : LeafTile{0, 0, 0};
-    const uint32_t* mem = leaf ? p.members + lt.off : nullptr;
-    // query rows of this tile
+    const LeafTile lt = p.leaf_tiles[blockIdx.x];
+    const uint32_t* mem = p.members + lt.off;
+    // rows of this tile
     if (threadIdx.x < kTile) {
-        if (leaf) {
-            const uint32_t t = lt.rb * kTile + threadIdx.x;
-            rowid[threadIdx.x] = t < lt.cnt ? (uint64_t)mem[t] : ~0ull;
-        } else {
-            const uint64_t t = (uint64_t)blockIdx.x * kTile + threadIdx.x;
-            rowid[threadIdx.x] = t < p.nrows ? (p.rows ? p.rows[t] : t) : ~0ull;
-        }
+        const uint32_t t = lt.rb * kTile + threadIdx.x;
+        rowid[threadIdx.x] = t < lt.cnt ? (uint64_t)mem[t] : ~0ull;
     }
-    // base columns: positions [js, je) of the base rows, or of the leaf's members
-    const uint64_t js = leaf ? 0 : (uint64_t)blockIdx.y * p.split_len;
-    const uint64_t je = leaf ? (uint64_t)lt.cnt : min_u64(p.n, js + p.split_len);
-    const uint32_t T = js < je ? (uint32_t)((je - js + kTile - 1) / kTile) : 0u;
+    // columns: the leaf's members
+    const uint64_t je = lt.cnt;
+    const uint32_t T = (lt.cnt + kTile - 1) / kTile;
     if (warp == 0) tc::tmem_alloc(&tslot, 256);
     if (threadIdx.x == 0) {
         tc::mbar_init(&bar[0], 1);
@@ -303,25 +297,24 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     // base tile t -> stage t % kStages (operand + per-column data)
     auto prefetch = [&](uint32_t t) {
         const uint32_t st = t % kStages;
-        const uint64_t j0 = js + (uint64_t)t * kTile;
+        const uint64_t j0 = (uint64_t)t * kTile;
         unsigned char* dst = sb + (size_t)st * tile_bytes;
         for (uint32_t i = threadIdx.x; i < kTile * chunks; i += blockDim.x) {  // (no operand in the wide form)
             const uint32_t rr = i % kTile, c = i / kTile;
             const uint64_t pos = j0 + rr;
             const bool ok = pos < je;
-            const uint64_t row = ok ? (leaf ? (uint64_t)mem[pos] : pos) : 0;
+            const uint64_t row = ok ? (uint64_t)mem[pos] : 0;
             tc::cp_async16_zfill(dst + (size_t)c * kTile * 16 + rr * 16, p.xb + row * p.dp + 8 * c, ok ? 16u : 0u);
         }
         if (threadIdx.x < kTile) {
             const uint64_t pos = j0 + threadIdx.x;
             const bool ok = pos < je;
-            const uint64_t j = ok ? (leaf ? (uint64_t)mem[pos] : pos) : 0;
-            if (leaf) colid[st * kTile + threadIdx.x] = (uint32_t)j;
-            float* cs = col + (size_t)st * 4 * kTile;
+            const uint64_t j = ok ? (uint64_t)mem[pos] : 0;
+            colid[st * kTile + threadIdx.x] = (uint32_t)j;
+            float* cs = col + (size_t)st * 3 * kTile;
             cs[threadIdx.x] = ok ? p.xn[j] : __int_as_float(0x7f800000);
             cs[kTile + threadIdx.x] = ok ? p.xnorm[j] : 0.f;
             cs[2 * kTile + threadIdx.x] = ok ? p.xerr[j] : 0.f;
-            cs[3 * kTile + threadIdx.x] = ok ? (p.thr_col ? p.thr_col[j] : 0.f) : -__int_as_float(0x7f800000);
             colint[st * kTile + threadIdx.x] = ok ? p.xint[j] : 0;
         }
     };
@@ -338,8 +331,8 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     const float qnm = row_ok ? p.qnorm[my_row] : 0.f;
     const float qer = row_ok ? p.qerr[my_row] : 0.f;
     const bool qexact = row_ok && p.qint[my_row] && p.d <= 128;
-    float thr_r = (row_ok && p.thr_row) ? p.thr_row[my_row] : 0.f;
-    if (leaf && row_ok)
+    float thr_r = 0.f;
+    if (row_ok)
         thr_r = p.list_sz[my_row] >= p.list_k ? p.list_kd[my_row * p.list_k + p.list_k - 1]
                                                 : __int_as_float(0x7f800000);
     const float u = 5.9604645e-8f;        // 2^-24
@@ -357,7 +350,6 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
         return l2k ? __fsub_rn(__fadd_rn(qn, xnc), __fmul_rn(2.0f, acc))
                    : (p.key_mode == 1 ? __fsub_rn(1.0f, acc) : -__fadd_rn(acc, 0.0f));  // +0 as the reference's
     };
-    const float* qrow = p.q32 + (row_ok ? my_row : 0) * p.xs;
     // eps <= epsmax for every column of this row (eps grows with the column's
     // |x|, |x - bf16(x)| and norm; exact rows against all-exact columns: 0)
     const float epsmax = (qexact && p.all_exact) ? 0.f : fmaf(ca, p.bx_norm, fmaf(cb, p.bx_err, fmaf(cc, p.bx_n, cd)));
@@ -366,62 +358,46 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     // in stage e % kStages): each thread its row, each warp half the columns
     auto epilogue = [&](uint32_t e, uint32_t tmem) {
         const uint32_t st = e % kStages;
-        const float* cs = col + (size_t)st * 4 * kTile;
-        const uint64_t j0 = js + (uint64_t)e * kTile;
+        const float* cs = col + (size_t)st * 3 * kTile;
         for (uint32_t c0 = half * 64; c0 < half * 64 + 64; c0 += 32) {
             float v[32];
             tc::tmem_ld32(tmem + (((warp & 3u) * 32u) << 16) + (e & 1u) * kTile + c0, v);
             if (!row_ok) continue;
-            // columns that survive the row's eps bound, without branches:
-            // 4 norms (and thresholds) per shared load
-            const bool rowthr = p.thr_row || leaf;
+            // columns that survive the row's eps bound, without branches: 4
+            // norms per shared load (+inf past the leaf, which makes eps below
+            // infinite or no number, so such a column is dropped there)
             uint32_t keep = 0;
 #pragma unroll
             for (uint32_t k = 0; k < 32; k += 4) {
                 const float4 xn4 = *reinterpret_cast<const float4*>(cs + c0 + k);
-                const float4 th4 = rowthr ? make_float4(thr_r, thr_r, thr_r, thr_r)
-                                          : *reinterpret_cast<const float4*>(cs + 3 * kTile + c0 + k);
-                const float xa[4] = {xn4.x, xn4.y, xn4.z, xn4.w}, ta[4] = {th4.x, th4.y, th4.z, th4.w};
+                const float xa[4] = {xn4.x, xn4.y, xn4.z, xn4.w};
 #pragma unroll
                 for (uint32_t q = 0; q < 4; q++) {
                     const float approx = approx_key(xa[q], v[k + q]);
-                    keep |= (approx - epsmax <= ta[q] ? 1u : 0u) << (k + q);
+                    keep |= (approx - epsmax <= thr_r ? 1u : 0u) << (k + q);
                 }
             }
             for (; keep; keep &= keep - 1) {
                 const uint32_t k = __ffs(keep) - 1;
                 const uint32_t cj = c0 + k;
-                const uint64_t j = leaf ? (uint64_t)colid[st * kTile + cj] : j0 + cj;
+                const uint64_t j = colid[st * kTile + cj];
                 const float xn = cs[cj];
                 float vk = 0.f;
 #pragma unroll
                 for (uint32_t q = 0; q < 32; q++)
                     if (q == k) vk = v[q];
                 const float approx = approx_key(xn, vk);
-                const float thr = rowthr ? thr_r : cs[3 * kTile + cj];
                 const bool exact = qexact && colint[st * kTile + cj];
                 const float eps =
                     exact ? 0.f : fmaf(ca, cs[kTile + cj], fmaf(cb, cs[2 * kTile + cj], fmaf(cc, xn, cd)));
-                if (!(approx - eps <= thr)) continue;
-                if (p.exclude_self && j == my_row) continue;
-                if (leaf) {
-                    // the merge recomputes flagged keys in FP32 and keeps <= its K-th;
-                    // slots are indexed by the row's position in the batch of leaves
-                    const uint64_t cs0 = lt.off + (uint64_t)lt.rb * kTile + r - p.pos_base;
-                    const uint32_t pos = atomicAdd(p.cnt + cs0, 1u);
-                    if (pos < p.cap) {
-                        p.out_id[cs0 * p.cap + pos] = (uint32_t)j | (exact ? 0u : kRecheck);
-                        p.out_key[cs0 * p.cap + pos] = approx;
-                    }
-                    continue;
-                }
-                const bool later = p.defer_recheck && !exact;
-                const float key = (exact || later) ? approx : ref_key(qrow, p.x32 + j * p.xs, p.d, qn, xn, p.key_mode);
-                if (!later && !(key <= thr)) continue;
-                const uint32_t pos = atomicAdd(p.cnt + my_row, 1u);
+                if (!(approx - eps <= thr_r) || j == my_row) continue;
+                // the merge recomputes flagged keys in FP32 and keeps <= its K-th;
+                // slots are indexed by the row's position in the batch of leaves
+                const uint64_t cs0 = lt.off + (uint64_t)lt.rb * kTile + r - p.pos_base;
+                const uint32_t pos = atomicAdd(p.cnt + cs0, 1u);
                 if (pos < p.cap) {
-                    p.out_id[my_row * p.cap + pos] = (uint32_t)j | (later ? kRecheck : 0u);
-                    p.out_key[my_row * p.cap + pos] = key;
+                    p.out_id[cs0 * p.cap + pos] = (uint32_t)j | (exact ? 0u : kRecheck);
+                    p.out_key[cs0 * p.cap + pos] = approx;
                 }
             }
         }
@@ -472,7 +448,7 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
         for (uint32_t t = 0; t <= T && !stop; t++) {
             const uint32_t tmem = tslot;
             if (t < T) {
-                const uint64_t j0 = js + (uint64_t)t * kTile;
+                const uint64_t j0 = (uint64_t)t * kTile;
                 for (uint32_t c = 0; c < nc; c++, it++) {
                     const uint32_t slot = it % kWideStages;
                     if (it >= kWideStages &&
@@ -491,7 +467,7 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
                                              p.qb + (oka ? row : 0) * p.dp + c * kWideK + 8 * q, oka ? 16u : 0u);
                         const uint64_t pos = j0 + rr;
                         const bool okb = pos < je;
-                        const uint64_t brow = okb ? (leaf ? (uint64_t)mem[pos] : pos) : 0;
+                        const uint64_t brow = okb ? (uint64_t)mem[pos] : 0;
                         tc::cp_async16_zfill(db + (size_t)q * kTile * 16 + rr * 16,
                                              p.xb + brow * p.dp + c * kWideK + 8 * q, okb ? 16u : 0u);
                     }
@@ -536,24 +512,376 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     if (warp == 0) tc::tmem_free(tslot, 256);
 }
 
+// ------------------------------------------------------------- scan
+// The filter over whole matrices (exact top-K, RkNN CSR): a CTA per SM walks
+// 128-row query tiles against 256-row base tiles, roles split by warp.
+//   warp 8   one thread moves operands in by bulk copies: the matrices are
+//            packed once into the tile layout of tc.cuh (pack_tiles_kernel), so
+//            64 K elements of a tile are one contiguous block and one copy;
+//   warp 9   one thread issues the MMAs (M = 128, N = 256) into one of two
+//            256-column TMEM accumulators;
+//   warps 0-7  read the other accumulator back and test it.
+// The query tile stays resident up to 512 padded dimensions and streams with
+// the base tile above.  The test costs three instructions a pair: base-tile
+// column constants C (the norm, or norm minus threshold rounded down) come with
+// the tile, a row constant R holds the rest of the inequality less eps over all
+// columns and a rounding margin, and the sign of C + R + f acc is shifted into a
+// mask.  Survivors go to a queue per warp; 32 of them at a time take the exact
+// test and the output slot's atomic, so its latency is paid once per 32.
+// At 100,000 x 300 (unit rows, top-100, then three CSRs of 2,000 queries) the
+// scans take 10.1 ms; tiles that were copied 16 bytes a thread and waited for
+// chunk by chunk took 60.7 ms.
+// N = 256: a 128 x 128 step would read both operands from shared memory at the
+// full rate of its port.
+struct ScanParams {
+    FilterParams f;
+    const unsigned char* qpack;  // query tiles of 128 rows
+    const unsigned char* xpack;  // base tiles of 256 rows
+    const float* cpack;          // column constants C, 256 per base tile (+inf past n)
+    const float* cmax;           // the largest finite |C|
+    uint32_t qtiles, xtiles, slices, slots;
+};
+
+constexpr uint32_t kScanN = 256;
+constexpr uint32_t kScanK = 64;              // K elements per ring slot
+constexpr uint32_t kScanResident = 512;      // padded dimension up to which the query tile stays
+constexpr uint32_t kScanThreads = 320;
+constexpr uint32_t kScanCols = 4;            // ring of column constants
+constexpr uint32_t kScanMaxSlots = 8;
+constexpr uint32_t kScanQueue = 64;          // survivors a warp holds: up to 31 waiting and 32 new
+
+__host__ __device__ constexpr uint32_t scan_slot_bytes(uint32_t dp) {
+    return (kScanN + (dp > kScanResident ? kTile : 0u)) * kScanK * 2;
+}
+__host__ __device__ constexpr uint32_t scan_fixed_bytes(uint32_t dp) {
+    return (dp > kScanResident ? 0u : kTile * dp * 2) + kScanCols * kScanN * 4 + 8 * kScanQueue * 12;
+}
+
+__global__ void __launch_bounds__(kScanThreads, 1) tc_scan_kernel(ScanParams sp) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    const FilterParams& p = sp.f;
+    const bool res = p.dp <= kScanResident;
+    const uint32_t slot_bytes = scan_slot_bytes(p.dp), S = sp.slots;
+    unsigned char* sa = sm;                                        // the resident query tile
+    unsigned char* ring = sm + (res ? (size_t)kTile * p.dp * 2 : 0);  // slots: base chunk, then query chunk if streamed
+    float* scol = reinterpret_cast<float*>(ring + (size_t)S * slot_bytes);
+    uint32_t* q_col = reinterpret_cast<uint32_t*>(scol + kScanCols * kScanN);  // 8 warps x kScanQueue each
+    uint32_t* q_row = q_col + 8 * kScanQueue;
+    float* q_acc = reinterpret_cast<float*>(q_row + 8 * kScanQueue);
+    __shared__ uint64_t full[kScanMaxSlots], empty[kScanMaxSlots], colfull[kScanCols], colempty[kScanCols];
+    __shared__ uint64_t accfull[2], accempty[2], afull, aempty, drained;
+    __shared__ uint32_t tslot;
+    __shared__ volatile int s_abort;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    if (warp == 9) tc::tmem_alloc(&tslot, 2 * kScanN);
+    if (threadIdx.x == 0) {
+        for (uint32_t k = 0; k < S; k++) {
+            tc::mbar_init(&full[k], 1);
+            tc::mbar_init(&empty[k], 1);
+        }
+        for (uint32_t k = 0; k < kScanCols; k++) {
+            tc::mbar_init(&colfull[k], 1);
+            tc::mbar_init(&colempty[k], 8);
+        }
+        for (uint32_t k = 0; k < 2; k++) {
+            tc::mbar_init(&accfull[k], 1);
+            tc::mbar_init(&accempty[k], 8);
+        }
+        tc::mbar_init(&afull, 1);
+        tc::mbar_init(&aempty, 1);
+        tc::mbar_init(&drained, 1);
+        tc::fence_mbar_init();
+        s_abort = 0;
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tslot;
+    const uint32_t items = sp.qtiles * sp.slices;
+    const uint32_t per = (sp.xtiles + sp.slices - 1) / sp.slices;  // base tiles per item
+    const uint32_t nc = (p.dp + kScanK - 1) / kScanK;
+    // every wait is bounded; one that runs out makes all roles leave
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (!s_abort && tc::mbar_wait(bar, parity, kWaitPolls)) return true;
+        s_abort = 1;
+        atomicExch(p.err, 8u);
+        return false;
+    };
+    bool ok = true;
+    if (warp == 8 && lane == 0) {
+        uint32_t it = 0, tt = 0, ai = 0;
+        for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t qt = item / sp.slices, t0 = item % sp.slices * per, t1 = min(sp.xtiles, t0 + per);
+            if (t0 >= t1) continue;
+            const unsigned char* qsrc = sp.qpack + (size_t)qt * kTile * p.dp * 2;
+            if (res) {
+                if (ai > 0 && !(ok = wait(&aempty, (ai - 1) & 1u))) break;
+                tc::mbar_expect(&afull, kTile * p.dp * 2);
+                tc::bulk_load(sa, qsrc, kTile * p.dp * 2, &afull);
+                ai++;
+            }
+            for (uint32_t t = t0; t < t1 && ok; t++, tt++) {
+                const uint32_t cs = tt % kScanCols;
+                if (tt >= kScanCols && !(ok = wait(&colempty[cs], (tt / kScanCols - 1) & 1u))) break;
+                tc::mbar_expect(&colfull[cs], kScanN * 4);
+                tc::bulk_load(scol + cs * kScanN, sp.cpack + (size_t)t * kScanN, kScanN * 4, &colfull[cs]);
+                const unsigned char* xsrc = sp.xpack + (size_t)t * kScanN * p.dp * 2;
+                for (uint32_t c = 0; c < nc; c++, it++) {
+                    const uint32_t sl = it % S, w = min(kScanK, p.dp - c * kScanK);
+                    if (it >= S && !(ok = wait(&empty[sl], (it / S - 1) & 1u))) break;
+                    unsigned char* dst = ring + (size_t)sl * slot_bytes;
+                    const uint32_t xb = kScanN * w * 2, qb = res ? 0u : kTile * w * 2;
+                    tc::mbar_expect(&full[sl], xb + qb);
+                    tc::bulk_load(dst, xsrc + (size_t)c * kScanN * kScanK * 2, xb, &full[sl]);
+                    if (qb) tc::bulk_load(dst + kScanN * kScanK * 2, qsrc + (size_t)c * kTile * kScanK * 2, qb, &full[sl]);
+                }
+            }
+        }
+        if (!ok) {
+            // copies still in flight land before the block leaves
+            for (uint32_t k = it > S ? it - S : 0; k < it; k++) tc::mbar_wait(&full[k % S], (k / S) & 1u, kWaitPolls);
+            for (uint32_t k = tt > kScanCols ? tt - kScanCols : 0; k < tt; k++)
+                tc::mbar_wait(&colfull[k % kScanCols], (k / kScanCols) & 1u, kWaitPolls);
+            if (ai) tc::mbar_wait(&afull, (ai - 1) & 1u, kWaitPolls);
+        }
+    } else if (warp == 9 && lane == 0) {
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(kTile, kScanN);
+        uint32_t it = 0, tt = 0, ai = 0;
+        for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t t0 = item % sp.slices * per, t1 = min(sp.xtiles, t0 + per);
+            if (t0 >= t1) continue;
+            if (res && !(ok = wait(&afull, ai & 1u))) break;
+            ai++;
+            for (uint32_t t = t0; t < t1 && ok; t++, tt++) {
+                const uint32_t b = tt & 1u;
+                if (tt >= 2 && !(ok = wait(&accempty[b], (tt / 2 - 1) & 1u))) break;
+                tc::fence_after_sync();
+                for (uint32_t c = 0; c < nc; c++, it++) {
+                    const uint32_t sl = it % S, w = min(kScanK, p.dp - c * kScanK);
+                    if (!(ok = wait(&full[sl], (it / S) & 1u))) break;
+                    tc::fence_after_sync();
+                    const uint32_t xs = tc::smem_u32(ring + (size_t)sl * slot_bytes);
+                    const uint32_t qs = res ? tc::smem_u32(sa) + c * kTile * kScanK * 2 : xs + kScanN * kScanK * 2;
+                    for (uint32_t s = 0; s < w / 16; s++)
+                        tc::mma_bf16(tmem + b * kScanN, tc::smem_desc(qs + 2 * s * kTile * 16, kTile * 16, 128),
+                                     tc::smem_desc(xs + 2 * s * kScanN * 16, kScanN * 16, 128), idesc,
+                                     (c > 0 || s > 0) ? 1u : 0u);
+                    tc::mma_commit(&empty[sl]);
+                }
+                if (ok) tc::mma_commit(&accfull[b]);
+            }
+            if (res && ok) tc::mma_commit(&aempty);
+        }
+        if (!ok) {
+            // so do the MMAs
+            tc::mma_commit(&drained);
+            tc::mbar_wait(&drained, 0, kWaitPolls);
+        }
+    } else if (warp < 8) {
+        const uint32_t quarter = warp & 3u, half = warp >> 2;
+        uint32_t* wq_col = q_col + warp * kScanQueue;
+        uint32_t* wq_row = q_row + warp * kScanQueue;
+        float* wq_acc = q_acc + warp * kScanQueue;
+        const bool l2k = p.key_mode == 0;
+        const float f = l2k ? -2.f : -1.f;
+        const float u = 5.9604645e-8f;  // 2^-24
+        const float g = 2.0f * p.dp * u;
+        const float kh = l2k ? 1.f : 0.5f;
+        const float cc = l2k ? 4.f * u : 0.f;
+        const float cmax = *sp.cmax;
+        uint32_t tt = 0;
+        for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            const uint32_t qt = item / sp.slices, t0 = item % sp.slices * per, t1 = min(sp.xtiles, t0 + per);
+            if (t0 >= t1) continue;
+            // the row's error bound (tc_filter_kernel) and test constants
+            const uint64_t qi = (uint64_t)qt * kTile + quarter * 32 + lane;
+            const bool row_ok = qi < p.nrows;
+            const uint32_t my_row = row_ok ? (p.rows ? p.rows[qi] : (uint32_t)qi) : 0u;
+            const float qn = row_ok ? p.qn[my_row] : 0.f;
+            const float qnm = row_ok ? p.qnorm[my_row] : 0.f;
+            const float qer = row_ok ? p.qerr[my_row] : 0.f;
+            const bool qexact = row_ok && p.qint[my_row] && p.d <= 128;
+            const float thr_r = (row_ok && p.thr_row) ? p.thr_row[my_row] : 0.f;
+            const float ca = kh * (2.f * qer + 4.f * g * (qnm + qer) + 4.f * g * qnm + 8.f * u * qnm);
+            const float cb = kh * (2.f * qnm + 2.f * qer + 4.f * g * (qnm + qer));
+            const float cd = l2k ? 4.f * u * qn : 4.f * u;
+            const float epsmax =
+                (qexact && p.all_exact) ? 0.f : fmaf(ca, p.bx_norm, fmaf(cb, p.bx_err, fmaf(cc, p.bx_n, cd)));
+            // C + R + f acc <= 0 for every pair with key~ - epsmax <= threshold:
+            // the margin covers the roundings of R, C + R and the test's FMA
+            const float q0 = l2k ? qn : (p.key_mode == 1 ? 1.f : 0.f);
+            const float margin = 16.f * u * (fabsf(q0) + (p.thr_row ? fabsf(thr_r) : 0.f) + epsmax + cmax + p.bx_n) + 1e-37f;
+            float R = q0 - thr_r - epsmax - margin;
+            if (p.thr_row && thr_r == __int_as_float(0x7f800000)) R = -__int_as_float(0x7f800000);
+            uint32_t nq = 0;  // survivors waiting in the warp's queue (uniform)
+            auto flush = [&](uint32_t m) {
+                // entry `lane` of the first m: the exact test, then its output slot
+                const bool has = lane < m;
+                const uint32_t src = has ? wq_row[lane] : 0u;
+                const uint32_t j = has ? wq_col[lane] : 0u;
+                const float acc = has ? wq_acc[lane] : 0.f;
+                const uint32_t row = __shfl_sync(0xFFFFFFFFu, my_row, src);
+                const float eqn = __shfl_sync(0xFFFFFFFFu, qn, src);
+                const float eca = __shfl_sync(0xFFFFFFFFu, ca, src), ecb = __shfl_sync(0xFFFFFFFFu, cb, src);
+                const float ecd = __shfl_sync(0xFFFFFFFFu, cd, src), ethr = __shfl_sync(0xFFFFFFFFu, thr_r, src);
+                const bool eint = __shfl_sync(0xFFFFFFFFu, qexact ? 1 : 0, src) != 0;
+                if (has && j < p.n && !(p.exclude_self && j == row)) {
+                    const float xn = p.xn[j];
+                    const float approx = l2k ? __fsub_rn(__fadd_rn(eqn, xn), __fmul_rn(2.0f, acc))
+                                             : (p.key_mode == 1 ? __fsub_rn(1.0f, acc) : -__fadd_rn(acc, 0.0f));
+                    const float thr = p.thr_row ? ethr : p.thr_col[j];
+                    const bool exact = eint && p.xint[j];
+                    const float eps = exact ? 0.f : fmaf(eca, p.xnorm[j], fmaf(ecb, p.xerr[j], fmaf(cc, xn, ecd)));
+                    if (approx - eps <= thr) {
+                        const bool later = p.defer_recheck && !exact;
+                        const float key = (exact || later)
+                                              ? approx
+                                              : ref_key(p.q32 + (uint64_t)row * p.xs, p.x32 + (uint64_t)j * p.xs, p.d,
+                                                        eqn, xn, p.key_mode);
+                        if (later || key <= thr) {
+                            const uint32_t pos = atomicAdd(p.cnt + row, 1u);
+                            if (pos < p.cap) {
+                                p.out_id[(uint64_t)row * p.cap + pos] = j | (later ? kRecheck : 0u);
+                                p.out_key[(uint64_t)row * p.cap + pos] = key;
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            };
+            for (uint32_t t = t0; t < t1; t++, tt++) {
+                const uint32_t b = tt & 1u, cs = tt % kScanCols;
+                if (!(ok = wait(&accfull[b], (tt / 2) & 1u)) || !(ok = wait(&colfull[cs], (tt / kScanCols) & 1u))) {
+                    ok = false;
+                }
+                ok = __all_sync(0xFFFFFFFFu, ok);
+                if (!ok) break;
+                tc::fence_after_sync();
+                const float* C = scol + cs * kScanN;
+                for (uint32_t c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
+                    float v[32];
+                    tc::tmem_ld32(tmem + ((quarter * 32u) << 16) + b * kScanN + c0, v);
+                    uint32_t keep = 0;  // bit 31 - k: column k
+#pragma unroll
+                    for (uint32_t k = 0; k < 32; k += 4) {
+                        const float4 c4 = *reinterpret_cast<const float4*>(C + c0 + k);
+                        const float ca4[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; e++)
+                            keep = __funnelshift_l(__float_as_uint(fmaf(f, v[k + e], ca4[e] + R)), keep, 1);
+                    }
+                    if (!row_ok) keep = 0;
+                    while (true) {
+                        const unsigned any = __ballot_sync(0xFFFFFFFFu, keep != 0);
+                        if (!any) break;
+                        if (keep) {
+                            const uint32_t k = __clz(keep);
+                            keep &= ~(0x80000000u >> k);
+                            float vk = v[0];
+#pragma unroll
+                            for (uint32_t e = 1; e < 32; e++)
+                                if (e == k) vk = v[e];
+                            const uint32_t at = nq + __popc(any & lane_lt_mask());
+                            wq_row[at] = lane;
+                            wq_col[at] = t * kScanN + c0 + k;
+                            wq_acc[at] = vk;
+                        }
+                        nq += __popc(any);
+                        __syncwarp();
+                        if (nq >= 32) {
+                            flush(32);
+                            // the rest moves to the front
+                            nq -= 32;
+                            uint32_t mr = 0, mc = 0;
+                            float ma = 0.f;
+                            if (lane < nq) {
+                                mr = wq_row[32 + lane];
+                                mc = wq_col[32 + lane];
+                                ma = wq_acc[32 + lane];
+                            }
+                            __syncwarp();
+                            if (lane < nq) {
+                                wq_row[lane] = mr;
+                                wq_col[lane] = mc;
+                                wq_acc[lane] = ma;
+                            }
+                            __syncwarp();
+                        }
+                    }
+                }
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    tc::mbar_arrive(&accempty[b]);
+                    tc::mbar_arrive(&colempty[cs]);
+                }
+            }
+            if (nq) flush(nq);
+        }
+    }
+    __syncwarp();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 9) tc::tmem_free(tmem, 2 * kScanN);
+}
+
+// Rows of a bf16 matrix (dp wide) in tiles of `tile` rows, each in the layout
+// of tc.cuh: 16-byte K groups, the tile's rows in each.  rows: the source row of
+// each output row (null: itself); rows past nrows are zero.
+__global__ void pack_tiles_kernel(const __nv_bfloat16* __restrict__ src, const uint32_t* __restrict__ rows,
+                                  uint64_t nrows, uint32_t dp, uint32_t tile, uint64_t total,
+                                  uint4* __restrict__ out) {
+    const uint32_t groups = dp / 8;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+         e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)(e % tile);
+        const uint64_t q = e / tile;
+        const uint32_t c = (uint32_t)(q % groups);
+        const uint64_t row = q / groups * tile + r;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (row < nrows) v = *reinterpret_cast<const uint4*>(src + (rows ? rows[row] : row) * dp + 8 * c);
+        out[e] = v;
+    }
+}
+
+// The scan's column constants: the norm (l2) less the column's threshold if it
+// has one, rounded down; +inf past n.  *cmax: the largest finite magnitude.
+__global__ void scan_columns_kernel(const float* __restrict__ xn, const float* __restrict__ thr_col, uint64_t n,
+                                    uint64_t padded, uint32_t key_mode, float* __restrict__ C, float* cmax) {
+    float mx = 0.f;
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < padded;
+         j += (uint64_t)gridDim.x * blockDim.x) {
+        float c = __int_as_float(0x7f800000);
+        if (j < n) {
+            c = key_mode == 0 ? xn[j] : 0.f;
+            if (thr_col) c = __fsub_rd(c, thr_col[j]);
+            if (fabsf(c) <= 3.4028235e38f) mx = fmaxf(mx, fabsf(c));
+        }
+        C[j] = c;
+    }
+    atomicMax(reinterpret_cast<uint32_t*>(cmax), __float_as_uint(mx));
+}
+
 // Upper bound of each row's K-th smallest key: the largest reference FP32 key
 // to K distinct other rows (the hints, e.g. the AKNN lists).  Warp per row.
 __global__ void hint_bound_kernel(const float* __restrict__ x, const float* __restrict__ xn, uint64_t n,
                                   uint32_t xs, uint32_t d, const uint32_t* __restrict__ hints, uint32_t hk,
                                   uint32_t K, float* __restrict__ tau, uint32_t mode) {
-    const uint32_t lane = threadIdx.x & 31u;
+    // a 4-thread group per pair, eight pairs a pass: the rows are read in whole
+    // 64-byte pieces (a thread per pair read them 4 bytes at a time)
+    const uint32_t lane = threadIdx.x & 31u, gt = lane & 3u, gw = lane >> 2;
     const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = w; i < n; i += nw) {
         float mx = -__int_as_float(0x7f800000);
         bool bad = false;
-        for (uint32_t k = lane; k < K; k += 32) {
-            const uint32_t j = hints[i * hk + k];
-            if (j >= n || j == i) {
-                bad = true;
-                continue;
-            }
-            mx = fmaxf(mx, ref_key(x + i * xs, x + (uint64_t)j * xs, d, xn[i], xn[j], mode));
+        for (uint32_t k0 = 0; k0 < K; k0 += 8) {
+            const bool in = k0 + gw < K;
+            const uint32_t j = in ? hints[i * hk + k0 + gw] : kEmpty;
+            const bool ok = j < n && j != i;
+            bad |= in && !ok;
+            const float ip = group_ip(x + i * xs, x + (ok ? (uint64_t)j : i) * xs, d, gt, 0xFFFFFFFFu);
+            if (ok) mx = fmaxf(mx, mode == 2 ? -ip : __fsub_rn(__fadd_rn(xn[i], xn[j]), __fmul_rn(2.0f, ip)));
         }
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
         bad = __any_sync(0xFFFFFFFFu, bad);
@@ -693,7 +1021,7 @@ __global__ void take_first_k_kernel(const uint64_t* __restrict__ off, uint64_t n
 
 size_t filter_smem(uint32_t dp) {
     const size_t operands = dp > kMaxDp ? (size_t)2 * kWideStages * kTile * kWideK * 2 : (size_t)(1 + kStages) * kTile * dp * 2;
-    return operands + (size_t)kStages * 4 * kTile * 4 + kStages * kTile + kTile * 8 + (size_t)kStages * kTile * 4;
+    return operands + (size_t)kStages * 3 * kTile * 4 + kStages * kTile + kTile * 8 + (size_t)kStages * kTile * 4;
 }
 
 // The padded dimension of the tensor path for d: a multiple of 16 with the
@@ -714,20 +1042,44 @@ int filter_kernel_for(Ctx* c, uint32_t dp, void (**kern)(FilterParams), size_t* 
     return ANQI_OK;
 }
 
-int launch_filter(Ctx* c, FilterParams p, uint64_t nrows) {
+// The scan of p over nrows query rows (p.rows: which; null: the first nrows).
+// The packed operands take the context's init_knn buffers, idle outside a build.
+int launch_scan(Ctx* c, FilterParams p, uint64_t nrows) {
     if (nrows == 0) return ANQI_OK;
-    void (*kern)(FilterParams) = nullptr;
-    size_t smem = 0;
-    int rc = filter_kernel_for(c, p.dp, &kern, &smem);
-    if (rc) return rc;
-    const uint64_t gx = (nrows + kTile - 1) / kTile;
-    const uint64_t tiles = (p.n + kTile - 1) / kTile;
-    uint64_t gy = std::max<uint64_t>(1, ((uint64_t)2 * c->sm_count + gx - 1) / gx);
-    gy = std::min<uint64_t>(gy, tiles);
-    p.split_len = (tiles + gy - 1) / gy * kTile;
+    ScanParams sp{};
     p.nrows = nrows;
-    dim3 grid((unsigned)gx, (unsigned)gy);
-    kern<<<grid, kFilterThreads, smem, c->stream>>>(p);
+    sp.qtiles = (uint32_t)((nrows + kTile - 1) / kTile);
+    sp.xtiles = (uint32_t)((p.n + kScanN - 1) / kScanN);
+    const size_t qbytes = (size_t)sp.qtiles * kTile * p.dp * 2, xbytes = (size_t)sp.xtiles * kScanN * p.dp * 2;
+    const size_t cbytes = (size_t)sp.xtiles * kScanN * 4;
+    int rc;
+    if ((rc = ensure(c, c->init_cid, qbytes)) || (rc = ensure(c, c->init_key, xbytes)) ||
+        (rc = ensure(c, c->init_cnt, cbytes + 16)))
+        return rc;
+    float* cpack = c->init_cnt.as<float>();
+    float* cmax = cpack + (size_t)sp.xtiles * kScanN;
+    const uint32_t blocks = c->sm_count * 8;
+    ANQI_CUDA(c, cudaMemsetAsync(cmax, 0, 4, c->stream));
+    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.qb, p.rows, nrows, p.dp, kTile, qbytes / 16, c->init_cid.as<uint4>());
+    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.xb, nullptr, p.n, p.dp, kScanN, xbytes / 16, c->init_key.as<uint4>());
+    scan_columns_kernel<<<blocks, 256, 0, c->stream>>>(p.xn, p.thr_col, p.n, (uint64_t)sp.xtiles * kScanN, p.key_mode,
+                                                       cpack, cmax);
+    ANQI_CUDA(c, cudaGetLastError());
+    sp.f = p;
+    sp.qpack = c->init_cid.as<unsigned char>();
+    sp.xpack = c->init_key.as<unsigned char>();
+    sp.cpack = cpack;
+    sp.cmax = cmax;
+    // items of one query tile and a slice of the base tiles, at least eight per
+    // SM while a slice keeps 16 tiles, so that the last wave is short
+    sp.slices = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>((8ull * c->sm_count + sp.qtiles - 1) / sp.qtiles, (sp.xtiles + 15) / 16));
+    const uint32_t fixed = scan_fixed_bytes(p.dp), slot = scan_slot_bytes(p.dp);
+    sp.slots = std::min<uint32_t>(kScanMaxSlots, (226 * 1024 - fixed) / slot);
+    const size_t smem = fixed + (size_t)sp.slots * slot;
+    ANQI_CUDA(c, cudaFuncSetAttribute(tc_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(c->sm_count, (uint64_t)sp.qtiles * sp.slices);
+    tc_scan_kernel<<<grid, kScanThreads, smem, c->stream>>>(sp);
     ANQI_CUDA(c, cudaGetLastError());
     return ANQI_OK;
 }
@@ -749,7 +1101,7 @@ int filter_to_csr(Ctx* c, FilterParams p, uint64_t nq, uint32_t cap, std::vector
     p.out_key = okey.as<float>();
     p.rows = nullptr;
     p.err = c->err.as<uint32_t>();
-    if ((rc = launch_filter(c, p, nq))) return rc;
+    if ((rc = launch_scan(c, p, nq))) return rc;
     if ((rc = check_device_error(c, "tensor-core filter"))) return rc;
     std::vector<uint32_t> hc(nq);
     if ((rc = d2h(c, hc.data(), cnt, nq * 4)) || (rc = sync(c))) return rc;
@@ -780,7 +1132,7 @@ int filter_to_csr(Ctx* c, FilterParams p, uint64_t nq, uint32_t cap, std::vector
         q.cap = cap2;
         q.out_id = oid2.as<uint32_t>();
         q.out_key = okey2.as<float>();
-        if ((rc = launch_filter(c, q, no))) return rc;
+        if ((rc = launch_scan(c, q, no))) return rc;
         if ((rc = check_device_error(c, "tensor-core filter (capacity rerun)"))) return rc;
     }
     hoff.assign(nq + 1, 0);
@@ -988,7 +1340,6 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     p.xs = xs;
     p.d = d;
     p.dp = tp.dp;
-    p.exclude_self = 1;
     p.cnt = cnt;
     p.cap = cap;
     p.out_id = out_id;
@@ -1006,7 +1357,6 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     p.bx_n = tp.bn;
     p.all_exact = tp.all_exact;
     p.nrows = ntiles * kTile;
-    p.split_len = 0;
     void (*kern)(FilterParams) = nullptr;
     size_t smem = 0;
     int rc;
