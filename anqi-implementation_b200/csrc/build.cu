@@ -866,6 +866,24 @@ __global__ void label_init_kernel(uint32_t* lab, uint64_t n) {
         lab[i] = (uint32_t)i;
 }
 
+// cnt[label] += 1 per row, one atomic per warp whose lanes agree; then the
+// largest count.
+__global__ void label_count_kernel(const uint32_t* __restrict__ lab, uint64_t n, uint32_t* __restrict__ cnt) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n + 31) / 32 * 32;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t l = i < n ? lab[i] : kEmpty;
+        const unsigned peers = __match_any_sync(kAll, l);
+        if (l < n && (threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1) atomicAdd(cnt + l, (uint32_t)__popc(peers));
+    }
+}
+__global__ void label_max_kernel(const uint32_t* __restrict__ cnt, uint64_t n, uint32_t* __restrict__ out) {
+    uint32_t m = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        m = max(m, cnt[i]);
+    m = __reduce_max_sync(kAll, m);
+    if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
+}
+
 __global__ void inverse_perm_kernel(const uint32_t* __restrict__ perm, uint64_t n, uint32_t* __restrict__ inv) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         inv[perm[i]] = (uint32_t)i;
@@ -1223,9 +1241,11 @@ static int build_reverse(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K, 
 // and inv (original -> new).  order: tree 0's permutation.
 // ranges receives the components of at most kCompMaxRows rows (none when the
 // propagation was cut off, whose labels are not whole components), in_ranges
-// how many rows they hold.
+// how many rows they hold.  only_small: when some component is larger, stop
+// after the labels, with in_ranges = 0 and no numbering.
 static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K, const uint32_t* d_order, DevBuf& perm,
-                          DevBuf& inv, std::vector<CompRange>& ranges, uint64_t& in_ranges) {
+                          DevBuf& inv, std::vector<CompRange>& ranges, uint64_t& in_ranges,
+                          bool only_small = false) {
     TmpBuf lab(c), flag(c);
     int rc;
     if ((rc = ensure(c, lab, n * 4)) || (rc = ensure(c, flag, 4)) || (rc = ensure(c, perm, n * 4)) ||
@@ -1245,6 +1265,18 @@ static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K,
         uint32_t changed = 0;
         if ((rc = d2h(c, &changed, flag, 4)) || (rc = sync(c))) return rc;
         whole = !changed;
+    }
+    in_ranges = 0;
+    if (only_small) {
+        if (!whole) return ANQI_OK;
+        ANQI_CUDA(c, cudaMemsetAsync(inv.p, 0, n * 4, c->stream));
+        ANQI_CUDA(c, cudaMemsetAsync(flag.p, 0, 4, c->stream));
+        label_count_kernel<<<blocks, 256, 0, c->stream>>>(lab.as<uint32_t>(), n, inv.as<uint32_t>());
+        label_max_kernel<<<blocks, 256, 0, c->stream>>>(inv.as<uint32_t>(), n, flag.as<uint32_t>());
+        ANQI_CUDA(c, cudaGetLastError());
+        uint32_t most = 0;
+        if ((rc = d2h(c, &most, flag, 4)) || (rc = sync(c))) return rc;
+        if (most > kCompMaxRows) return ANQI_OK;
     }
     std::vector<uint32_t> hl(n), ho(n), start(n + 1, 0), out(n);
     ANQI_CUDA(c, cudaMemcpyAsync(ho.data(), d_order, n * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1514,8 +1546,61 @@ static int run_select_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_
                              float alpha, DevBuf& O, DevBuf& Odeg, DevBuf* links, DevBuf* deg, uint64_t* pool_total,
                              const uint32_t* row_order = nullptr, double* kernel_ms = nullptr) {
     TmpBuf roff(c), rev(c);
-    int rc = build_reverse(c, hid.as<uint32_t>(), n, K, roff, rev);
-    if (rc) return rc;
+    int rc;
+    // lists that fall into small components everywhere: search and prune on the
+    // components' tables (ANQI_B200_GRAPH_COMPONENTS=0: the general gather)
+    const char* comp_env = std::getenv("ANQI_B200_GRAPH_COMPONENTS");
+    if (links && row_order && !c->edge.active && !(comp_env && comp_env[0] == '0')) {
+        TmpBuf perm(c), inv(c), ids(c), vals(c), rows(c), norm(c), pool(c);
+        std::vector<CompRange> ranges;
+        uint64_t in_ranges = 0;
+        if ((rc = locality_order(c, hid.as<uint32_t>(), n, K, row_order, perm, inv, ranges, in_ranges, true))) return rc;
+        if (in_ranges == n) {
+            const int blocks = c->sm_count * 8;
+            if ((rc = ensure(c, ids, n * K * 4)) || (rc = ensure(c, vals, n * K * 4)) ||
+                (rc = ensure(c, rows, n * stride * 4ull)) || (rc = ensure(c, norm, n * 4)) || (rc = ensure(c, pool, 8)) ||
+                (rc = ensure(c, *links, n * M * 4)) || (rc = ensure(c, *deg, n * 4)))
+                return rc;
+            renumber_lists_kernel<<<blocks, 256, 0, c->stream>>>(hid.as<uint32_t>(), hval.as<float>(),
+                                                                perm.as<uint32_t>(), inv.as<uint32_t>(), n, K,
+                                                                ids.as<uint32_t>(), vals.as<float>());
+            permute_rows_kernel<<<blocks, 256, 0, c->stream>>>(dx.as<float>(), rows.as<float>(), perm.as<uint32_t>(), n,
+                                                               stride, 0u);
+            permute_vals_kernel<<<blocks, 256, 0, c->stream>>>(dn.as<float>(), norm.as<float>(), perm.as<uint32_t>(), n);
+            ANQI_CUDA(c, cudaGetLastError());
+            ANQI_CUDA(c, cudaMemsetAsync(pool.p, 0, 8, c->stream));
+            if ((rc = build_reverse(c, ids.as<uint32_t>(), n, K, roff, rev))) return rc;
+            CompGather g{};
+            g.x = rows.as<float>();
+            g.norms = norm.as<float>();
+            g.n = n;
+            g.stride = stride;
+            g.dim = dim;
+            g.g_ids = ids.as<uint32_t>();
+            g.K = K;
+            g.rev_off = roff.as<uint64_t>();
+            g.rev_ids = rev.as<uint32_t>();
+            g.ef = ef;
+            g.cap = cap;
+            g.perm = perm.as<uint32_t>();
+            g.pool_total = pool.as<unsigned long long>();
+            bool any_bad = false;
+            ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+            if ((rc = run_component_select_commit(c, g, ranges, M, alpha, links->as<uint32_t>(), deg->as<uint32_t>(),
+                                                  &any_bad)))
+                return rc;
+            ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+            if ((rc = sync(c))) return rc;
+            if (!any_bad) {
+                float ms = 0;
+                ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+                if (kernel_ms) *kernel_ms += ms;
+                if (pool_total) ANQI_CUDA(c, cudaMemcpy(pool_total, pool.p, 8, cudaMemcpyDeviceToHost));
+                return ANQI_OK;
+            }
+        }
+    }
+    if ((rc = build_reverse(c, hid.as<uint32_t>(), n, K, roff, rev))) return rc;
     const uint64_t mr = max_reverse(c, roff, n);
     if ((rc = ensure(c, O, n * M * 4)) || (rc = ensure(c, Odeg, n * 4))) return rc;
     GatherParams p = base_params(dx, dn, n, stride, dim);

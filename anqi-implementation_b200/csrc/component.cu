@@ -28,6 +28,14 @@
 // At 1M x 128 in clusters of 1,000 the gather takes 38.6 ms on the device (Gram
 // 14.3, bitmaps 0.5, search 23.8) instead of the general gather's 599 ms, whose
 // rows each read 1,000 vectors and walked 120,000 list entries.
+//
+// The G48 build's select and commit (gather_candidates, the alpha-RNG prune and
+// commit_edges, include/index.h:267-281, 772-829, 907-930) run on the same
+// tables when every row lies in a small component: comp_select_kernel searches
+// and prunes, comp_commit_kernel prunes each row's chosen and reverse edges.
+// Both prune against rows of the distance matrix instead of recomputing a
+// product per candidate and selected edge.  200k x 130 in clusters of 200:
+// 5.9 ms (with the tables) instead of 74.2 ms.
 #include <algorithm>
 #include <cfloat>
 #include <vector>
@@ -501,26 +509,214 @@ int launch_search(Ctx* c, const CompSearchParams& p, uint32_t blocks) {
     return ANQI_OK;
 }
 
-}  // namespace
+struct CompSelectParams {
+    uint64_t row_lo, row_hi;
+    const uint32_t* row_comp;
+    const CompDesc* comps;
+    uint32_t first, ncomps;
+    const float* G;
+    const uint32_t* adj;
+    const uint32_t* bad;
+    const uint32_t* g_ids;
+    uint32_t K, ef, cap, M;
+    float alpha;
+    const uint32_t* perm;
+    uint32_t* edges;  // select: chosen edges and their reverse, bitmaps laid out as adj (zeroed before)
+    uint32_t* links;  // commit: n x M and degrees, original numbering
+    uint32_t* deg;
+    unsigned long long* pool_total;
+};
 
-int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, DevBuf& row_comp,
-                         DevBuf& bad, bool* any_bad) {
-    *any_bad = false;
-    if (ranges.empty()) return ANQI_OK;
+// Lane l's bits of W bitmap words (word j bit l -> bit j), the words spread over
+// the lanes (word j in words[j / 32] of lane j % 32).
+template <int W>
+__device__ __forceinline__ uint64_t lane_bits(const uint32_t (&words)[(W + 31) / 32], uint32_t lane) {
+    uint64_t m = 0;
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+        const uint32_t w = __shfl_sync(kAll, words[j / 32], j % 32);
+        m |= (uint64_t)((w >> lane) & 1u) << j;
+    }
+    return m;
+}
+
+// The best (dist, original id) of the lanes' marked entries: its component row,
+// or kEmpty when nothing is marked.  Warp-collective.
+template <int W>
+__device__ __forceinline__ uint32_t best_marked(const float (&v)[W], uint64_t mark, const uint32_t* perm,
+                                                uint32_t lane) {
+    float bd = 0.f;
+    uint32_t be = kEmpty;
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+        if (!((mark >> j) & 1u)) continue;
+        const uint32_t e = 32 * j + lane;
+        if (be == kEmpty || v[j] < bd || (v[j] == bd && perm[e] < perm[be])) {
+            bd = v[j];
+            be = e;
+        }
+    }
+    const uint32_t key = be == kEmpty ? kPad : key_of(bd);
+    const uint32_t kmin = __reduce_min_sync(kAll, key);
+    if (kmin == kPad) return kEmpty;
+    unsigned b = __ballot_sync(kAll, key == kmin);
+    if (b & (b - 1)) {
+        const uint32_t p = key == kmin ? perm[be] : kPad;
+        b = __ballot_sync(kAll, p == __reduce_min_sync(kAll, p) && key == kmin);
+    }
+    return __shfl_sync(kAll, be, __ffs(b) - 1);
+}
+
+// alpha-RNG prune (index.h:267-281) of the marked entries of a row with
+// distances v into sel: the best one left is taken and drops every entry it
+// occludes, found in its row of the distance matrix.
+template <int W>
+__device__ __forceinline__ uint32_t comp_prune(const float (&v)[W], uint64_t alive, const CompDesc& cd,
+                                               const float* G, const uint32_t* perm, uint32_t M, float alpha,
+                                               uint32_t* sel, uint32_t lane) {
+    uint32_t nsel = 0;
+    while (nsel < M) {
+        const uint32_t c = best_marked<W>(v, alive, perm, lane);
+        if (c == kEmpty) break;
+        if (lane == 0) sel[nsel] = c;
+        nsel++;
+        if (lane == (c & 31u)) alive &= ~(1ull << (c >> 5));
+        const float* crow = G + cd.goff + (uint64_t)c * (cd.words * 32);
+#pragma unroll
+        for (int j = 0; j < W; j++)
+            if ((alive >> j) & 1u)
+                if (__fmul_rn(alpha, crow[32 * j + lane]) < v[j]) alive &= ~(1ull << j);
+    }
+    __syncwarp();
+    return nsel;
+}
+
+// Select: the row's search (as comp_search_kernel's, the next row to expand
+// found by a scan of the marked distances: the queue here is short) and the
+// prune of everything it visited.  Warp per row.
+template <int W>
+__global__ void __launch_bounds__(128) comp_select_kernel(CompSelectParams p) {
+    __shared__ uint32_t s_words[4][kCompMaxWords], s_sel[4][64];
+    constexpr int NL = (W + 31) / 32;
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const uint64_t row = p.row_lo + (uint64_t)blockIdx.x * 4 + wib;
+    if (row >= p.row_hi) return;
+    const uint32_t ci = p.row_comp[row] - p.first;
+    if (ci >= p.ncomps) return;
+    const CompDesc cd = p.comps[ci];
+    if (p.bad[cd.index]) return;
+    uint32_t* words = s_words[wib];
+    uint32_t* sel = s_sel[wib];
+    const uint32_t li = (uint32_t)row - cd.start;
+    const uint32_t* perm = p.perm + cd.start;
+    const float* drow = p.G + cd.goff + (uint64_t)li * (cd.words * 32);
+    float v[W];
+#pragma unroll
+    for (int j = 0; j < W; j++) v[j] = 32 * j + lane < cd.size ? drow[32 * j + lane] : 0.f;
+    for (uint32_t w = lane; w < NL * 32; w += 32) words[w] = 0u;
+    __syncwarp();
+    for (uint32_t t = lane; t < p.K; t += 32) {
+        const uint32_t e = p.g_ids[row * p.K + t] - cd.start;
+        if (e < cd.size) atomicOr(words + (e >> 5), 1u << (e & 31u));
+    }
+    __syncwarp();
+    uint64_t vis = 0;  // the lane's visited entries
+#pragma unroll
+    for (int j = 0; j < W; j++) vis |= (uint64_t)((words[j] >> lane) & 1u) << j;
+    uint64_t front = vis;  // visited, not expanded
+    uint32_t npool = __reduce_add_sync(kAll, (uint32_t)__popcll(vis)), nexp = 0;
+    while (npool < cd.size) {
+        const uint32_t node = best_marked<W>(v, front, perm, lane);
+        if (node == kEmpty) break;
+        if (nexp >= p.ef) {
+            // its rank among the visited: the expanded rows closer than it
+            const float nd = drow[node];
+            const uint32_t np = perm[node];
+            uint32_t closer = 0;
+#pragma unroll
+            for (int j = 0; j < W; j++)
+                if (((vis & ~front) >> j) & 1u)
+                    closer += v[j] < nd || (v[j] == nd && perm[32 * j + lane] < np) ? 1u : 0u;
+            if (__reduce_add_sync(kAll, closer) >= p.ef) break;
+        }
+        const uint32_t* arow = p.adj + cd.aoff + (uint64_t)node * cd.words;
+        uint32_t aw[NL];
+#pragma unroll
+        for (int w = 0; w < NL; w++) aw[w] = lane + 32 * w < cd.words ? arow[lane + 32 * w] : 0u;
+        const uint64_t fresh = lane_bits<W>(aw, lane) & ~vis;
+        vis |= fresh;
+        front |= fresh;
+        if (lane == (node & 31u)) front &= ~(1ull << (node >> 5));
+        npool += __reduce_add_sync(kAll, (uint32_t)__popcll(fresh));
+        nexp++;
+        if (npool >= p.cap) break;
+    }
+    if (lane == (li & 31u)) vis &= ~(1ull << (li >> 5));  // never the row itself
+    const uint32_t nsel = comp_prune<W>(v, vis, cd, p.G, perm, p.M, p.alpha, sel, lane);
+    uint32_t* edges = p.edges + cd.aoff;
+    for (uint32_t t = lane; t < nsel; t += 32) {
+        const uint32_t c = sel[t];
+        atomicOr(edges + (uint64_t)li * cd.words + (c >> 5), 1u << (c & 31u));
+        atomicOr(edges + (uint64_t)c * cd.words + (li >> 5), 1u << (li & 31u));
+    }
+    if (lane == 0) atomicAdd(p.pool_total, (unsigned long long)npool);
+}
+
+// Commit: prunes each row's chosen and reverse edges into its final links.
+template <int W>
+__global__ void __launch_bounds__(128) comp_commit_kernel(CompSelectParams p) {
+    __shared__ uint32_t s_sel[4][64];
+    constexpr int NL = (W + 31) / 32;
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+    const uint64_t row = p.row_lo + (uint64_t)blockIdx.x * 4 + wib;
+    if (row >= p.row_hi) return;
+    const uint32_t ci = p.row_comp[row] - p.first;
+    if (ci >= p.ncomps) return;
+    const CompDesc cd = p.comps[ci];
+    if (p.bad[cd.index]) return;
+    uint32_t* sel = s_sel[wib];
+    const uint32_t li = (uint32_t)row - cd.start;
+    const uint32_t* perm = p.perm + cd.start;
+    const float* drow = p.G + cd.goff + (uint64_t)li * (cd.words * 32);
+    const uint32_t* erow = p.edges + cd.aoff + (uint64_t)li * cd.words;
+    uint32_t ew[NL];
+#pragma unroll
+    for (int w = 0; w < NL; w++) ew[w] = lane + 32 * w < cd.words ? erow[lane + 32 * w] : 0u;
+    const uint64_t cand = lane_bits<W>(ew, lane);
+    float v[W];
+#pragma unroll
+    for (int j = 0; j < W; j++) v[j] = (cand >> j) & 1u ? drow[32 * j + lane] : 0.f;
+    const uint32_t nsel = comp_prune<W>(v, cand, cd, p.G, perm, p.M, p.alpha, sel, lane);
+    const uint64_t orow = perm[li];
+    for (uint32_t t = lane; t < p.M; t += 32) p.links[orow * p.M + t] = t < nsel ? perm[sel[t]] : kEmpty;
+    if (lane == 0) p.deg[orow] = nsel;
+}
+
+template <int W>
+int launch_select(Ctx* c, const CompSelectParams& p, uint32_t blocks) {
+    comp_select_kernel<W><<<blocks, 128, 0, c->stream>>>(p);
+    comp_commit_kernel<W><<<blocks, 128, 0, c->stream>>>(p);
+    ANQI_CUDA(c, cudaGetLastError());
+    return ANQI_OK;
+}
+
+// Components in batches whose matrices fit the context's init_knn key buffer
+// (kept between builds and idle here; at least 256 MB are allowed), with each
+// row's component.
+struct CompBatch {
+    size_t c0, c1;
+    uint32_t tiles, words;
+    uint64_t aoff;
+};
+
+int plan_batches(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, std::vector<CompBatch>& batches,
+                 TmpBuf& descs_d, DevBuf& row_comp, DevBuf& bad) {
     int rc;
-    std::vector<uint32_t> rc_host(g.n, kEmpty);
+    std::vector<uint32_t> rows(g.n, kEmpty);
     std::vector<CompDesc> descs(ranges.size());
-    // batches of components whose matrices fit the context's init_knn key
-    // buffer (up to 512 MB, idle by now): a few launches at 1M rows
-    const uint64_t budget = std::max<uint64_t>(c->init_key.bytes, 64ull << 20) / 4;
-    struct Range {
-        size_t c0, c1;
-        uint32_t tiles, words;
-        uint64_t aoff;
-    };
-    std::vector<Range> batches;
+    const uint64_t budget = std::max<uint64_t>(c->init_key.bytes, 256ull << 20) / 4;
     for (size_t k = 0; k < ranges.size();) {
-        Range b{k, k, 0, 1, 0};
+        CompBatch b{k, k, 0, 1, 0};
         uint64_t goff = 0;
         while (b.c1 < ranges.size()) {
             const CompRange& r = ranges[b.c1];
@@ -533,38 +729,64 @@ int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRang
             b.words = std::max(b.words, words);
             goff += need;
             b.aoff += (uint64_t)r.size * words;
-            for (uint32_t t = 0; t < r.size; t++) rc_host[r.start + t] = (uint32_t)b.c1;
+            for (uint32_t t = 0; t < r.size; t++) rows[r.start + t] = (uint32_t)b.c1;
             b.c1++;
         }
-        if ((rc = ensure(c, c->init_key, std::max(goff * 4, (uint64_t)c->init_key.bytes))) ||
-            (rc = ensure(c, c->init_cid, std::max(b.aoff * 4, (uint64_t)c->init_cid.bytes))))
-            return rc;
+        if ((rc = ensure(c, c->init_key, goff * 4)) || (rc = ensure(c, c->init_cid, b.aoff * 4))) return rc;
         batches.push_back(b);
         k = b.c1;
     }
-    TmpBuf dc(c);
-    if ((rc = h2d(c, row_comp, rc_host.data(), g.n * 4)) ||
-        (rc = h2d(c, dc, descs.data(), descs.size() * sizeof(CompDesc))) ||
+    if ((rc = h2d(c, row_comp, rows.data(), g.n * 4)) ||
+        (rc = h2d(c, descs_d, descs.data(), descs.size() * sizeof(CompDesc))) ||
         (rc = ensure(c, bad, (ranges.size() + 1) * 4)))
         return rc;
     ANQI_CUDA(c, cudaMemsetAsync(bad.p, 0, (ranges.size() + 1) * 4, c->stream));
-    for (const Range& b : batches) {
+    return sync(c);  // the host arrays go out of scope
+}
+
+// The distance matrices and adjacency bitmaps of a batch's components.
+int launch_tables(Ctx* c, const CompGather& g, const CompBatch& b, const CompDesc* comps, uint64_t lo, uint64_t hi,
+                  const DevBuf& row_comp, const DevBuf& bad) {
+    const uint32_t nc = (uint32_t)(b.c1 - b.c0);
+    comp_gram_kernel<<<b.tiles, 256, 0, c->stream>>>(g.x, g.norms, g.stride, g.dim, g.cols, comps, nc,
+                                                     c->init_key.as<float>(), bad.as<uint32_t>());
+    comp_adj_kernel<<<(unsigned)((hi - lo + 3) / 4), 128, 0, c->stream>>>(
+        lo, hi, row_comp.as<uint32_t>(), comps, (uint32_t)b.c0, nc, g.g_ids, g.K, g.rev_off, g.rev_ids,
+        c->init_cid.as<uint32_t>());
+    ANQI_CUDA(c, cudaGetLastError());
+    return ANQI_OK;
+}
+
+int any_flag(Ctx* c, const DevBuf& bad, size_t n, bool* any) {
+    std::vector<uint32_t> hb(n);
+    int rc;
+    if ((rc = d2h(c, hb.data(), bad, hb.size() * 4)) || (rc = sync(c))) return rc;
+    for (uint32_t f : hb) *any |= f != 0;
+    return ANQI_OK;
+}
+
+}  // namespace
+
+int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, DevBuf& row_comp,
+                         DevBuf& bad, bool* any_bad) {
+    *any_bad = false;
+    if (ranges.empty()) return ANQI_OK;
+    int rc;
+    std::vector<CompBatch> batches;
+    TmpBuf dc(c);
+    if ((rc = plan_batches(c, g, ranges, batches, dc, row_comp, bad))) return rc;
+    for (const CompBatch& b : batches) {
         const CompDesc* comps = dc.as<CompDesc>() + b.c0;
-        const uint32_t nc = (uint32_t)(b.c1 - b.c0);
         const uint64_t lo = ranges[b.c0].start, hi = (uint64_t)ranges[b.c1 - 1].start + ranges[b.c1 - 1].size;
         const uint32_t blocks = (uint32_t)((hi - lo + 3) / 4);
-        comp_gram_kernel<<<b.tiles, 256, 0, c->stream>>>(g.x, g.norms, g.stride, g.dim, g.cols, comps, nc,
-                                                         c->init_key.as<float>(), bad.as<uint32_t>());
-        comp_adj_kernel<<<blocks, 128, 0, c->stream>>>(lo, hi, row_comp.as<uint32_t>(), comps, (uint32_t)b.c0, nc,
-                                                       g.g_ids, g.K, g.rev_off, g.rev_ids, c->init_cid.as<uint32_t>());
-        ANQI_CUDA(c, cudaGetLastError());
+        if ((rc = launch_tables(c, g, b, comps, lo, hi, row_comp, bad))) return rc;
         CompSearchParams p{};
         p.row_lo = lo;
         p.row_hi = hi;
         p.row_comp = row_comp.as<uint32_t>();
         p.comps = comps;
         p.first = (uint32_t)b.c0;
-        p.ncomps = nc;
+        p.ncomps = (uint32_t)(b.c1 - b.c0);
         p.G = c->init_key.as<float>();
         p.adj = c->init_cid.as<uint32_t>();
         p.bad = bad.as<uint32_t>();
@@ -586,10 +808,53 @@ int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRang
                              : launch_search<kCompMaxWords>(c, p, blocks);
         if (rc) return rc;
     }
-    std::vector<uint32_t> hb(ranges.size());
-    if ((rc = d2h(c, hb.data(), bad, hb.size() * 4)) || (rc = sync(c))) return rc;
-    for (uint32_t f : hb) *any_bad |= f != 0;
-    return ANQI_OK;
+    return any_flag(c, bad, ranges.size(), any_bad);
+}
+
+int run_component_select_commit(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, uint32_t M,
+                                float alpha, uint32_t* links, uint32_t* deg, bool* any_bad) {
+    *any_bad = false;
+    int rc;
+    std::vector<CompBatch> batches;
+    TmpBuf dc(c), row_comp(c), bad(c), edges(c);
+    if ((rc = plan_batches(c, g, ranges, batches, dc, row_comp, bad))) return rc;
+    uint64_t most = 0;
+    for (const CompBatch& b : batches) most = std::max(most, b.aoff);
+    if ((rc = ensure(c, edges, most * 4))) return rc;
+    for (const CompBatch& b : batches) {
+        const CompDesc* comps = dc.as<CompDesc>() + b.c0;
+        const uint64_t lo = ranges[b.c0].start, hi = (uint64_t)ranges[b.c1 - 1].start + ranges[b.c1 - 1].size;
+        const uint32_t blocks = (uint32_t)((hi - lo + 3) / 4);
+        if ((rc = launch_tables(c, g, b, comps, lo, hi, row_comp, bad))) return rc;
+        ANQI_CUDA(c, cudaMemsetAsync(edges.p, 0, b.aoff * 4, c->stream));
+        CompSelectParams p{};
+        p.row_lo = lo;
+        p.row_hi = hi;
+        p.row_comp = row_comp.as<uint32_t>();
+        p.comps = comps;
+        p.first = (uint32_t)b.c0;
+        p.ncomps = (uint32_t)(b.c1 - b.c0);
+        p.G = c->init_key.as<float>();
+        p.adj = c->init_cid.as<uint32_t>();
+        p.bad = bad.as<uint32_t>();
+        p.g_ids = g.g_ids;
+        p.K = g.K;
+        p.ef = g.ef;
+        p.cap = g.cap;
+        p.M = M;
+        p.alpha = alpha;
+        p.perm = g.perm;
+        p.edges = edges.as<uint32_t>();
+        p.links = links;
+        p.deg = deg;
+        p.pool_total = g.pool_total;
+        rc = b.words <= 8    ? launch_select<8>(c, p, blocks)
+             : b.words <= 20 ? launch_select<20>(c, p, blocks)
+             : b.words <= 36 ? launch_select<36>(c, p, blocks)
+                             : launch_select<kCompMaxWords>(c, p, blocks);
+        if (rc) return rc;
+    }
+    return any_flag(c, bad, ranges.size(), any_bad);
 }
 
 }  // namespace anqi

@@ -48,4 +48,10 @@ struct CompGather {
 int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, DevBuf& row_comp,
                          DevBuf& bad, bool* any_bad);
 
+// Select and commit of the G48 build when `ranges` cover every row (g.out_* and
+// g.g_vals unused): final links (n x M) and degrees in the original numbering.
+// With any_bad set the outputs are incomplete and the general path is to run.
+int run_component_select_commit(Ctx* c, const CompGather& g, const std::vector<CompRange>& ranges, uint32_t M,
+                                float alpha, uint32_t* links, uint32_t* deg, bool* any_bad);
+
 }  // namespace anqi
