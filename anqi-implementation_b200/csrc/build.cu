@@ -657,13 +657,10 @@ __global__ void warm_start_kernel(const float* __restrict__ x, const float* __re
             if (idx < width && gt == 0) cd[idx] = norm_d2(norms[i], norms[jj], ip);
         }
         __syncwarp();
-        if (lane == 0) {
-            for (uint32_t t = 0; t < width; t++) {
-                const uint32_t j = cid[t];
-                if (j != (uint32_t)i && j < n) heap_push(hi, hv, K, j, cd[t]);
-            }
+        for (uint32_t t = 0; t < width; t++) {
+            const uint32_t j = cid[t];
+            if (j != (uint32_t)i && j < n) heap_push(hi, hv, K, j, cd[t], lane);
         }
-        __syncwarp();
         for (uint32_t t = lane; t < K; t += 32) {
             hid[i * K + t] = hi[t];
             hval[i * K + t] = hv[t];
@@ -757,9 +754,7 @@ __global__ void __launch_bounds__(128) join_apply_kernel(const float* __restrict
                 if (ok && gt == 0) bd[idx] = norm_d2(nt, norms[w], ip);
             }
             __syncwarp();
-            if (lane == 0)
-                for (uint32_t q = 0; q < m; q++) local_upd += heap_push(hi, hv, K, bi[q], bd[q]);
-            __syncwarp();
+            for (uint32_t q = 0; q < m; q++) local_upd += heap_push(hi, hv, K, bi[q], bd[q], lane) ? 1u : 0u;
             m = 0;
         };
         for (uint32_t e = 0; e < s; e++) {

@@ -136,31 +136,38 @@ __device__ __forceinline__ void warp_sort_batch64(float* nd, uint32_t* ni, uint3
     __syncwarp();
 }
 
-// heap.h:162-186 push_nolock / check_push (no reverse edges), by one lane.
-__device__ __forceinline__ bool heap_push(uint32_t* ids, float* vals, uint32_t K, uint32_t node, float value) {
+// heap.h:162-186 push_nolock / check_push (no reverse edges), warp-collective:
+// the lanes look for a duplicate together (one of them scanning the heap took
+// most of the time of the kernels that push), lane 0 sifts.
+__device__ __forceinline__ bool heap_push(uint32_t* ids, float* vals, uint32_t K, uint32_t node, float value,
+                                          uint32_t lane) {
     if (value > vals[0]) return false;
-    for (uint32_t i = 0; i < K; i++)
-        if (ids[i] == node) return false;
-    uint32_t cur = 0, sw;
-    for (;;) {
-        const uint32_t l = 2 * cur + 1, r = l + 1;
-        if (l >= K) break;
-        if (r >= K) {
-            if (vals[l] > value) sw = l;
-            else break;
-        } else if (vals[l] >= vals[r]) {
-            if (vals[l] > value) sw = l;
-            else break;
-        } else {
-            if (vals[r] > value) sw = r;
-            else break;
+    bool dup = false;
+    for (uint32_t i = lane; i < K; i += 32) dup |= ids[i] == node;
+    if (__any_sync(kAll, dup)) return false;
+    if (lane == 0) {
+        uint32_t cur = 0, sw;
+        for (;;) {
+            const uint32_t l = 2 * cur + 1, r = l + 1;
+            if (l >= K) break;
+            if (r >= K) {
+                if (vals[l] > value) sw = l;
+                else break;
+            } else if (vals[l] >= vals[r]) {
+                if (vals[l] > value) sw = l;
+                else break;
+            } else {
+                if (vals[r] > value) sw = r;
+                else break;
+            }
+            ids[cur] = ids[sw];
+            vals[cur] = vals[sw];
+            cur = sw;
         }
-        ids[cur] = ids[sw];
-        vals[cur] = vals[sw];
-        cur = sw;
+        ids[cur] = node;
+        vals[cur] = value;
     }
-    ids[cur] = node;
-    vals[cur] = value;
+    __syncwarp();
     return true;
 }
 
