@@ -2,6 +2,7 @@
 // Context lifetime, device memory, error reporting, and small shared kernels.
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 #include <thread>
 
 #include "common.cuh"
@@ -23,17 +24,88 @@ int cuda_check(Ctx* c, cudaError_t e, const char* what) {
     return fail(c, ANQI_ERR_DEVICE, "CUDA error in %s: %s", what, cudaGetErrorString(e));
 }
 
+// The pool temporary buffers come from: one per device, shared by its contexts
+// and given back with the last of them.  A build allocates and frees dozens of
+// buffers of up to hundreds of megabytes; through cudaMalloc and cudaFree that
+// took 196 ms of a 576 ms source build at 1M x 128.  Up to kPoolKeep bytes stay
+// cached between calls; allocation and release follow the context's stream.
+constexpr uint64_t kPoolKeep = 8ull << 30;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+};
+// never destroyed: contexts may outlive static objects at process exit
+static std::mutex& g_pool_lock = *new std::mutex;
+static std::unordered_map<int, DevicePool>& g_pools = *new std::unordered_map<int, DevicePool>;
+
+static cudaMemPool_t pool_acquire(int device) {
+    std::lock_guard<std::mutex> lock(g_pool_lock);
+    DevicePool& d = g_pools[device];
+    if (!d.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            d.pool = nullptr;
+            return nullptr;  // no pools here: temporary buffers use cudaMalloc
+        }
+        uint64_t keep = kPoolKeep;
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    d.contexts++;
+    return d.pool;
+}
+
+static void pool_release(int device) {
+    std::lock_guard<std::mutex> lock(g_pool_lock);
+    DevicePool& d = g_pools[device];
+    if (d.pool && --d.contexts == 0) {
+        cudaMemPoolDestroy(d.pool);
+        d.pool = nullptr;
+    }
+}
+
+size_t free_device_bytes(Ctx* c) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return 8ull << 30;
+    }
+    uint64_t reserved = 0, used = 0;
+    if (c->pool && cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+        free_b += reserved - used;
+    return free_b;
+}
+
+static void free_buf(Ctx* c, DevBuf& b) {
+    if (b.pooled && c->pool) cudaFreeAsync(b.p, c->stream);
+    else cudaFree(b.p);
+    c->device_bytes -= b.bytes;
+    b.p = nullptr;
+    b.bytes = 0;
+}
+
 int ensure(Ctx* c, DevBuf& b, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (b.bytes >= bytes) return ANQI_OK;
-    if (b.p) {
-        cudaFree(b.p);
-        c->device_bytes -= b.bytes;
-        b.p = nullptr;
-        b.bytes = 0;
+    if (b.p) free_buf(c, b);
+    const bool pooled = b.pooled && c->pool;
+    auto alloc = [&] {
+        return pooled ? cudaMallocFromPoolAsync(&b.p, bytes, c->pool, c->stream) : cudaMalloc(&b.p, bytes);
+    };
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && c->pool) {
+        // the cached part of the pool back to the device, then once more
+        cudaGetLastError();
+        cudaStreamSynchronize(c->stream);
+        cudaMemPoolTrimTo(c->pool, 0);
+        e = alloc();
     }
-    cudaError_t e = cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         b.p = nullptr;
         return fail(c, ANQI_ERR_DEVICE, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
     }
@@ -43,12 +115,7 @@ int ensure(Ctx* c, DevBuf& b, size_t bytes) {
 }
 
 void release(Ctx* c, DevBuf& b) {
-    if (b.p) {
-        cudaFree(b.p);
-        c->device_bytes -= b.bytes;
-    }
-    b.p = nullptr;
-    b.bytes = 0;
+    if (b.p) free_buf(c, b);
 }
 
 // Large copies between pageable host memory and the device go through the
@@ -456,6 +523,7 @@ int anqi_ctx_create(int device, anqi_ctx** out) {
     }
     cudaMemsetAsync(c->err.p, 0, 64, c->stream);
     cudaStreamSynchronize(c->stream);
+    c->pool = pool_acquire(device);
     *out = h;
     return ANQI_OK;
 }
@@ -478,7 +546,11 @@ void anqi_ctx_destroy(anqi_ctx* h) {
         if (c->stage[s]) cudaFreeHost(c->stage[s]);
         if (c->stage_ev[s]) cudaEventDestroy(c->stage_ev[s]);
     }
-    if (c->stream) cudaStreamDestroy(c->stream);
+    if (c->stream) {
+        cudaStreamSynchronize(c->stream);  // releases to the pool
+        cudaStreamDestroy(c->stream);
+    }
+    if (c->pool) pool_release(c->device);
     delete h;
 }
 

@@ -14,10 +14,12 @@
 
 namespace anqi {
 
-// A growable device allocation owned by the context.
+// A growable device allocation owned by the context.  Pooled ones (temporary
+// buffers) come from the device's pool, in the order of the context's stream.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool pooled = false;
     template <class T>
     T* as() const { return static_cast<T*>(p); }
 };
@@ -89,7 +91,10 @@ struct GraphBuild {
     uint64_t n = 0, rows_done = 0;
     uint32_t dim = 0, xs = 0;
     anqi_graph_params gp{};
-    DevBuf dx, dn, hid, hv, order;
+    DevBuf dx, dn, hid, hv, order;  // freed after every build
+    GraphBuild() {
+        for (DevBuf* b : {&dx, &dn, &hid, &hv, &order}) b->pooled = true;
+    }
     std::vector<uint8_t> seen;  // rows delivered
     double forest_ms = 0, warm_ms = 0;
     // the edge policy of anqi_graph_params.edge, copied at begin
@@ -118,6 +123,7 @@ struct Ctx {
     int sm_count = 0;
     uint32_t inject = 0;  // ANQI_FAULT_* flags (anqi_inject_fault)
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;  // the device's pool of temporary buffers (shared by its contexts), or null
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
     cudaEvent_t tev0 = nullptr, tev1 = nullptr;  // anqi_timer_*
     std::string last_error;
@@ -180,11 +186,14 @@ struct Ctx {
 // Grow buf to at least bytes (contents not preserved).
 int ensure(Ctx* c, DevBuf& b, size_t bytes);
 void release(Ctx* c, DevBuf& b);
+// Device memory a large temporary buffer may count on: what the device has free
+// and what the pool holds unused.
+size_t free_device_bytes(Ctx* c);
 
 // A temporary device allocation released when it goes out of scope.
 struct TmpBuf : DevBuf {
     Ctx* c;
-    explicit TmpBuf(Ctx* ctx) : c(ctx) {}
+    explicit TmpBuf(Ctx* ctx) : c(ctx) { pooled = true; }
     ~TmpBuf() { release(c, *this); }
     TmpBuf(const TmpBuf&) = delete;
     TmpBuf& operator=(const TmpBuf&) = delete;
@@ -223,6 +232,7 @@ struct ForestOut {
     std::vector<uint32_t> n_nodes, left, right, leaf_off, leaf_cnt;
     std::vector<float> offset;
     DevBuf perm, hyper;  // device; released by the caller
+    ForestOut() { perm.pooled = hyper.pooled = true; }
 };
 int build_forest(Ctx* c, const float* d_x, uint64_t n, uint32_t dim, uint32_t stride, uint32_t trees, uint32_t leaf,
                  uint32_t max_depth, uint64_t seed, uint32_t cap_nodes, ForestOut& out, int angular = 0);
@@ -250,6 +260,7 @@ struct TcPrep {
     uint32_t dp = 0;
     float bnorm = 0, berr = 0, bn = 0;  // maxima of |x|, |x - bf16(x)|, the FP32 norm
     int all_exact = 0;                  // every row exact-integer
+    TcPrep() { bf.pooled = nrm.pooled = err.pooled = xint.pooled = true; }
 };
 // Padded row length of the tensor path for dimension d: resident query tiles
 // up to 256, the wide (K-chunked) form up to 1024; 0 above.

@@ -50,7 +50,9 @@ int anqi_ctx_create(int device, anqi_ctx** out);
 void anqi_ctx_destroy(anqi_ctx* ctx);
 const char* anqi_last_error(const anqi_ctx* ctx);
 int anqi_version(void);
-/* Bytes of device memory the context currently holds. */
+/* Bytes of device memory the context currently holds.  Temporary buffers come
+ * from a pool per device that keeps up to 8 GB cached while any context lives
+ * (not counted here). */
 uint64_t anqi_device_bytes(const anqi_ctx* ctx);
 /* Test hook, no counterpart in the reference: makes the device waits of this
  * context run out without any fault.  ANQI_FAULT_DROP_ROW_COPIES: the search
