@@ -579,6 +579,278 @@ __global__ void __launch_bounds__(128, kVam ? 5 : 7) gather_kernel(GatherParams 
     }
 }
 
+// ------------------------------------------------ AKNN gather, block per row
+// The AKNN mode of gather_kernel with one block per row, for rows that are not
+// in a small component and collections whose visited bitmap fits an SM several
+// times.  There a search visits thousands of rows, and a warp alone spends it
+// waiting: a table probe and an atomic in L2 per id, eight rows fetched at a
+// time, 19 rounds to shift a 600-entry beam.  A block keeps the bitmap over all
+// rows in shared memory, takes a chunk of an expansion's ids with a thread each,
+// fetches a row per 4-thread group and merges the kept ones into the beam in one
+// step between two buffers.  The beam, the pool count and the order are
+// gather_kernel's, so the lists are.  Bound by the latency of that chain and its
+// barriers, so by blocks in flight: 128 threads (ten blocks an SM by registers)
+// for l2; the ip metric's sequential sums need more rows per fetch, 256 threads
+// and five blocks.  Unit rows, 64 trees, ef = 600: 100,000 x 128 l2 181 -> 52 ms
+// (58 with 256 threads), 100,000 x 100 ip 151 -> 80 (115 with 128), 5,003 x 37
+// 10.0 -> 6.5.
+template <bool kIp>
+constexpr uint32_t kGbThreads = kIp ? 256 : 128;
+constexpr uint32_t kGbTile = 36;  // ip: staged row stride (32 floats; conflict-free by rows and by columns)
+
+__host__ __device__ __forceinline__ size_t gather_block_words(uint64_t n, uint32_t ef, uint32_t stride, bool ip) {
+    return (size_t)((n + 127) / 128) * 4 + 4 * (size_t)((ef + 3) & ~3u) +
+           4 * (ip ? kGbThreads<true> : kGbThreads<false>) + 32 + stride + (ip ? 64 * kGbTile : 0);
+}
+
+// 1 - <x_i, x_j> of up to 64 rows ids[0..m) in ip_dist_seq's order: 32 floats of
+// every row at a time through shared memory, so rows are read in whole lines,
+// then a thread per row adds its products in sequence.  Block-collective.
+__device__ __forceinline__ void block_ip64(const GatherParams& p, const float* xi, const uint32_t* ids, float* out,
+                                           uint32_t m, float* tile) {
+    constexpr uint32_t kRows = kGbThreads<true> / 8, kPass = 64 / kRows;  // rows a pass, passes
+    const uint32_t t = threadIdx.x, q = 4 * (t & 7u), r = t >> 3;
+    const uint32_t d8 = p.dim & ~7u;
+    float4 v[kPass];
+    auto fetch = [&](uint32_t c0) {
+#pragma unroll
+        for (uint32_t k = 0; k < kPass; k++) {
+            const uint32_t row = r + kRows * k;
+            v[k] = row < m && c0 + q < p.dim
+                       ? *reinterpret_cast<const float4*>(p.x + (uint64_t)ids[row] * p.stride + c0 + q)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float acc = 0.f;
+    fetch(0);
+    for (uint32_t c0 = 0; c0 < p.dim; c0 += 32) {
+#pragma unroll
+        for (uint32_t k = 0; k < kPass; k++) *reinterpret_cast<float4*>(tile + (r + kRows * k) * kGbTile + q) = v[k];
+        __syncthreads();
+        if (c0 + 32 < p.dim) fetch(c0 + 32);
+        if (t < m) {
+            const uint32_t w = min(32u, p.dim - c0);
+            for (uint32_t j = 0; j < w; j += 4) {
+                const float4 b = *reinterpret_cast<const float4*>(tile + t * kGbTile + j);
+                const float4 a = *reinterpret_cast<const float4*>(xi + c0 + j);
+                if (c0 + j < d8) {
+                    acc = __fadd_rn(acc, __fmul_rn(a.x, b.x));
+                    acc = __fadd_rn(acc, __fmul_rn(a.y, b.y));
+                    acc = __fadd_rn(acc, __fmul_rn(a.z, b.z));
+                    acc = __fadd_rn(acc, __fmul_rn(a.w, b.w));
+                } else {
+                    // the last dim mod 8 products by fused multiply-adds
+                    acc = __fmaf_rn(a.x, b.x, acc);
+                    if (j + 1 < w) acc = __fmaf_rn(a.y, b.y, acc);
+                    if (j + 2 < w) acc = __fmaf_rn(a.z, b.z, acc);
+                    if (j + 3 < w) acc = __fmaf_rn(a.w, b.w, acc);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (t < m) out[t] = __fsub_rn(1.0f, acc);
+}
+
+template <bool kIp>
+__global__ void __launch_bounds__(kGbThreads<kIp>, kIp ? 5 : 10) gather_block_kernel(GatherParams p) {
+    constexpr uint32_t T = kGbThreads<kIp>;
+    const uint32_t t = threadIdx.x, lane = t & 31u, gt = t & 3u, grp = t >> 2;
+    const uint32_t words4 = (uint32_t)((p.n + 127) / 128), efp = (p.ef + 3) & ~3u;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(g_build_smem);
+    float* beams = reinterpret_cast<float*>(bits + 4 * words4);  // two buffers: distances, then ids
+    float* nd = beams + 4 * efp;                                 // fresh rows ...
+    uint32_t* ni = reinterpret_cast<uint32_t*>(nd + T);
+    float* sd = reinterpret_cast<float*>(ni + T);  // ... those that enter the beam, sorted
+    uint32_t* si = reinterpret_cast<uint32_t*>(sd + T);
+    uint32_t* s_u = si + T;  // block scalars
+    float* xi = reinterpret_cast<float*>(s_u + 32);
+    float* tile = xi + p.stride;
+    enum { kRow = 0, kM = 1 /* three of them */, kKept = 4, kFirst = 5 };
+    const PermOrder ord{p.perm};
+    auto bdist = [&](uint32_t b) { return beams + 2 * efp * b; };
+    auto bids = [&](uint32_t b) { return reinterpret_cast<uint32_t*>(beams + 2 * efp * b + efp); };
+
+    for (;;) {
+        __syncthreads();
+        if (t == 0) {
+            uint32_t w;
+            uint64_t i;
+            do {  // rows left to this kernel
+                w = atomicAdd(p.next_row, 1u);
+                i = w < p.n ? (p.row_order ? p.row_order[w] : w) : p.n;
+            } while (w < p.n && (i >= p.n || (p.row_comp && p.row_comp[i] != kEmpty && !p.comp_bad[p.row_comp[i]])));
+            s_u[kRow] = w < p.n ? (uint32_t)i : kEmpty;
+            s_u[kM] = s_u[kM + 1] = s_u[kM + 2] = s_u[kKept] = 0;
+        }
+        for (uint32_t w = t; w < words4; w += T) reinterpret_cast<uint4*>(bits)[w] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        const uint32_t row = s_u[kRow];
+        if (row == kEmpty) break;
+        const uint64_t i = row;
+        for (uint32_t j = t; j < p.stride; j += T) xi[j] = p.x[i * p.stride + j];
+        const float ni_norm = kIp ? 0.f : p.norms[i];
+        uint32_t buf = 0, size = 0, lo = 0, mc = 0;  // mc: which kM counter the next chunk uses
+        uint64_t npool = 0;
+
+        // the fresh ids of a chunk, one per thread, to ni (order does not
+        // matter); returns how many
+        auto visit = [&](uint32_t id, float v, bool vals) -> uint32_t {
+            const bool f = id < p.n && visit_first(bits, id);
+            const unsigned b = __ballot_sync(kAll, f);
+            uint32_t at = 0;
+            if (lane == 0 && b) at = atomicAdd(s_u + kM + mc, __popc(b));
+            at = __shfl_sync(kAll, at, 0) + __popc(b & lane_lt_mask());
+            if (f) {
+                ni[at] = id;
+                if (vals) nd[at] = v;
+            }
+            // the next chunk's counter: last read two chunks ago, before the
+            // last chunk's barrier
+            if (t == 0) s_u[kM + (mc + 1) % 3] = 0;
+            __syncthreads();
+            const uint32_t m = s_u[kM + mc];
+            mc = (mc + 1) % 3;
+            return m;
+        };
+        // the m fresh rows of nd / ni into the beam
+        auto insert = [&](uint32_t m) {
+            const float* bd = bdist(buf);
+            const uint32_t* bi = bids(buf);
+            const bool full = size >= p.ef;
+            float dv = 0.f;
+            uint32_t iv = kEmpty;
+            bool keep = false;
+            if (t < m) {
+                dv = nd[t];
+                iv = ni[t];
+                keep = !full || ord(dv, iv, bd[p.ef - 1], bi[p.ef - 1]);
+            }
+            const unsigned b = __ballot_sync(kAll, keep);
+            uint32_t at = 0;
+            if (lane == 0 && b) at = atomicAdd(s_u + kKept, __popc(b));
+            at = __shfl_sync(kAll, at, 0) + __popc(b & lane_lt_mask());
+            __syncthreads();  // nd / ni read by every thread
+            const uint32_t mk = s_u[kKept];
+            if (mk == 0) return;
+            if (keep) {
+                nd[at] = dv;
+                ni[at] = iv;
+            }
+            __syncthreads();
+            if (t == 0) s_u[kKept] = 0;
+            if (t < mk) {
+                dv = nd[t];
+                iv = ni[t];
+                uint32_t rank = 0;
+                for (uint32_t x = 0; x < mk; x++) rank += ord(nd[x], ni[x], dv, iv) ? 1u : 0u;
+                sd[rank] = dv;
+                si[rank] = iv;
+            }
+            __syncthreads();
+            // fresh entry r lands at r + (beam entries before it), beam entry j
+            // at j + (fresh entries before it), in the other buffer
+            const uint32_t ns = min(p.ef, size + mk);
+            float* od = bdist(buf ^ 1u);
+            uint32_t* oi = bids(buf ^ 1u);
+            if (t < mk) {
+                const uint32_t r0 = lower_rank(bd, bi, size, sd[t], si[t], ord);
+                if (t == 0) s_u[kFirst] = r0;
+                if (t + r0 < ns) {
+                    od[t + r0] = sd[t];
+                    oi[t + r0] = si[t];
+                }
+            }
+            for (uint32_t j = t; j < size; j += T) {
+                const float jd = bd[j];
+                const uint32_t ji = bi[j];
+                const uint32_t pos = j + lower_rank(sd, si, mk, jd, ji, ord);
+                if (pos < ns) {
+                    od[pos] = jd;
+                    oi[pos] = ji;
+                }
+            }
+            __syncthreads();
+            lo = min(lo, s_u[kFirst]);
+            size = ns;
+            buf ^= 1u;
+        };
+
+        // seeds: the row's own list with its stored distances
+        for (uint32_t c0 = 0; c0 < p.K; c0 += T) {
+            const bool has = c0 + t < p.K;
+            const uint32_t m = visit(has ? p.g_ids[i * p.K + c0 + t] : kEmpty, has ? p.g_vals[i * p.K + c0 + t] : 0.f, true);
+            npool += m;
+            if (m) insert(m);
+        }
+        // expansions: the closest unexpanded entry, its forward then reverse list
+        for (;;) {
+            uint32_t* bi = bids(buf);
+            uint32_t cur = size;
+            for (uint32_t s0 = lo; s0 < size; s0 += 32) {
+                const uint32_t idx = s0 + lane;
+                const unsigned b = __ballot_sync(kAll, idx < size && !(bi[idx] & kExpanded));
+                if (b) {
+                    cur = s0 + __ffs(b) - 1;
+                    break;
+                }
+            }
+            if (cur >= size) break;
+            const uint32_t node = bi[cur] & kIdMask;
+            const uint64_t r0 = p.rev_off[node], r1 = p.rev_off[node + 1];
+            const uint32_t tot = p.K + (uint32_t)(r1 - r0);
+            lo = cur + 1;
+            bool marked = false;
+            for (uint32_t c0 = 0; c0 < tot; c0 += T) {
+                const uint32_t pa = c0 + t;
+                const uint32_t id = pa >= tot ? kEmpty
+                                              : (pa < p.K ? p.g_ids[(uint64_t)node * p.K + pa] : p.rev_ids[r0 + (pa - p.K)]);
+                const uint32_t m = visit(id, 0.f, false);
+                if (!marked) {  // every thread has read the cursor before visit's barrier
+                    if (t == 0) bi[cur] = node | kExpanded;
+                    marked = true;
+                }
+                if (m == 0) continue;
+                npool += m;
+                if constexpr (kIp) {
+                    for (uint32_t a = 0; a < m; a += 64) block_ip64(p, xi, ni + a, nd + a, min(64u, m - a), tile);
+                } else {
+                    for (uint32_t a = 0; a < m; a += T / 4) {
+                        const uint32_t e = a + grp;
+                        if ((e & ~7u) < m) {  // the warp's eight groups share the branch
+                            const uint32_t j = ni[min(e, m - 1)];
+                            const float* xj = p.x + (uint64_t)j * p.stride;
+                            const float ip = p.cols ? group_ip_cols<128>(xi, xj, gt, kAll)
+                                                    : group_ip(xi, xj, p.dim, gt, kAll);
+                            if (e < m && gt == 0) nd[e] = norm_d2(ni_norm, p.norms[j], ip);
+                        }
+                    }
+                }
+                __syncthreads();
+                insert(m);
+            }
+            __syncthreads();  // the mark, before the cursor is looked for again
+            if (npool >= p.cap) break;
+        }
+        if (t == 0) atomicAdd(p.pool_total, (unsigned long long)npool);
+        // index.h:1355-1361: sorted pool, first K ids != i
+        const float* ld = bdist(buf);
+        const uint32_t* li = bids(buf);
+        uint32_t self_pos = kEmpty;
+        for (uint32_t e = lane; e < min(size, p.out_k + 1); e += 32)
+            if ((li[e] & kIdMask) == row) self_pos = e;
+        self_pos = __reduce_min_sync(kAll, self_pos);
+        const uint64_t orow = p.perm ? (uint64_t)p.perm[i] : i;
+        for (uint32_t e = t; e < p.out_k; e += T) {
+            const uint32_t src = (self_pos != kEmpty && e >= self_pos) ? e + 1 : e;
+            const bool ok = src < size;
+            const uint32_t id = ok ? (li[src] & kIdMask) : kEmpty;
+            p.out_ids[orow * p.out_k + e] = (p.perm && ok) ? p.perm[id] : id;
+            p.out_d[orow * p.out_k + e] = ok ? ld[src] : FLT_MAX;
+        }
+    }
+}
+
 // ------------------------------------------------------- Vamana entries
 
 // The entry of each row for the Vamana refine (rptrees.h:108-123): the RP-tree
@@ -1463,6 +1735,41 @@ static int run_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_t
         *kernel_ms += ms;
     }
     if (pool_total) ANQI_CUDA(c, cudaMemcpy(pool_total, p.pool_total, 8, cudaMemcpyDeviceToHost));
+    return ANQI_OK;
+}
+
+// The AKNN gather of rows without a component: a block per row where at least
+// three blocks share an SM (up to about 480,000 rows; above, the bitmap leaves
+// one block and the warp-per-row kernel keeps more searches in flight), else
+// gather_kernel.  ANQI_B200_GATHER_BLOCK=0 turns it off.
+static int run_aknn_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_total, double* kernel_ms) {
+    const char* env = std::getenv("ANQI_B200_GATHER_BLOCK");
+    const size_t smem = gather_block_words(p.n, p.ef, p.stride, p.ip != 0) * 4;
+    auto kern = p.ip ? gather_block_kernel<true> : gather_block_kernel<false>;
+    const int threads = p.ip ? kGbThreads<true> : kGbThreads<false>;
+    int per_sm = 0;
+    if (!(env && env[0] == '0') && p.ef > p.out_k && smem <= 227 * 1024) {
+        ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    }
+    if (per_sm < 3) return run_gather(c, p, max_rev, pool_total, kernel_ms);
+    ANQI_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
+    p.next_row = c->counters.as<uint32_t>();
+    p.pool_total = reinterpret_cast<unsigned long long*>(c->counters.as<uint32_t>() + 2);
+    p.err = c->err.as<uint32_t>();
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>((uint64_t)per_sm * c->sm_count, p.n);
+    ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+    kern<<<blocks, threads, smem, c->stream>>>(p);
+    ANQI_CUDA(c, cudaGetLastError());
+    ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+    unsigned long long pooled = 0;
+    ANQI_CUDA(c, cudaMemcpyAsync(&pooled, p.pool_total, 8, cudaMemcpyDeviceToHost, c->stream));
+    int rc = check_device_error(c, "gather");  // synchronizes
+    if (rc) return rc;
+    float ms = 0;
+    ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+    *kernel_ms += ms;
+    *pool_total = pooled;
     return ANQI_OK;
 }
 
@@ -2688,7 +2995,7 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
     }
     if (rest) {
         uint64_t pooled = 0;
-        if ((rc = run_gather(c, p, max_reverse(c, roff, n), &pooled, &gather_kernel_ms))) return rc;
+        if ((rc = run_aknn_gather(c, p, max_reverse(c, roff, n), &pooled, &gather_kernel_ms))) return rc;
         pool_total += pooled;
     }
     const double gather_ms = ms_since(t);
