@@ -69,6 +69,10 @@ __device__ __forceinline__ float group_l2sqr(const float* __restrict__ a, const 
                                              uint32_t dim, uint32_t gt, unsigned mask) {
     const uint32_t q16 = dim >> 4, rem = dim & 15u;
     float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
+    // a far row's tail is requested with its first chunks
+    constexpr bool kFar = kUnroll > 4;
+    float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kFar && 4 * gt < rem) tail = *reinterpret_cast<const float4*>(a + 16 * q16 + 4 * gt);
 #pragma unroll kUnroll
     for (uint32_t c = 0; c < q16; c++) {
         float4 x = *reinterpret_cast<const float4*>(a + 16 * c + 4 * gt);
@@ -84,7 +88,7 @@ __device__ __forceinline__ float group_l2sqr(const float* __restrict__ a, const 
         float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
         const uint32_t base = 16 * q16 + 4 * gt;
         if (4 * gt < rem) {
-            float4 x = *reinterpret_cast<const float4*>(a + base);
+            const float4 x = kFar ? tail : *reinterpret_cast<const float4*>(a + base);
             float4 y = *reinterpret_cast<const float4*>(b + base);
             float d0 = __fsub_rn(x.x, y.x), d1 = __fsub_rn(x.y, y.y), d2 = __fsub_rn(x.z, y.z), d3 = __fsub_rn(x.w, y.w);
             p0 = __fmul_rn(d0, d0);
@@ -98,11 +102,15 @@ __device__ __forceinline__ float group_l2sqr(const float* __restrict__ a, const 
 }
 
 // Inner product (distance.h:89-116; NormSIMD16ExtAVX512__ is ip(a, a)).
+template <int kUnroll = 4>
 __device__ __forceinline__ float group_ip(const float* __restrict__ a, const float* __restrict__ b,
                                           uint32_t dim, uint32_t gt, unsigned mask) {
     const uint32_t q16 = dim >> 4, rem = dim & 15u;
     float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
-#pragma unroll 4
+    constexpr bool kFar = kUnroll > 4;
+    float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kFar && 4 * gt < rem) tail = *reinterpret_cast<const float4*>(a + 16 * q16 + 4 * gt);
+#pragma unroll kUnroll
     for (uint32_t c = 0; c < q16; c++) {
         float4 x = *reinterpret_cast<const float4*>(a + 16 * c + 4 * gt);
         float4 y = *reinterpret_cast<const float4*>(b + 16 * c + 4 * gt);
@@ -116,7 +124,7 @@ __device__ __forceinline__ float group_ip(const float* __restrict__ a, const flo
         float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
         const uint32_t base = 16 * q16 + 4 * gt;
         if (4 * gt < rem) {
-            float4 x = *reinterpret_cast<const float4*>(a + base);
+            const float4 x = kFar ? tail : *reinterpret_cast<const float4*>(a + base);
             float4 y = *reinterpret_cast<const float4*>(b + base);
             p0 = __fmul_rn(x.x, y.x);
             p1 = (4 * gt + 1 < rem) ? __fmul_rn(x.y, y.y) : 0.f;
@@ -196,13 +204,13 @@ __device__ __forceinline__ float group_l2sqr_w(const float* __restrict__ a, cons
 }
 
 // Inner product (distance.h:89-116) by a group of G = 8 or 16 threads.
-template <int G>
+template <int G, int kUnroll = 4>
 __device__ __forceinline__ float group_ip_w(const float* __restrict__ a, const float* __restrict__ b, uint32_t dim,
                                             uint32_t gt, unsigned mask) {
     const uint32_t q16 = dim >> 4, rem = dim & 15u;
     constexpr uint32_t NL = 16 / G;
     float c0 = 0.f, c1 = 0.f;
-#pragma unroll 4
+#pragma unroll kUnroll
     for (uint32_t c = 0; c < q16; c++) {
         if constexpr (NL == 2) {
             const float2 x = *reinterpret_cast<const float2*>(a + 16 * c + 2 * gt);

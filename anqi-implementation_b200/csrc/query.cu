@@ -855,43 +855,45 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
 }
 
 // Query lift and RP-tree entry (rknn_query.cpp:2724-2729, rptrees.h:108-124;
-// |margin| <= EPS goes left): every 4-lane group of a warp descends for its
-// own query (qpw queries per warp, 8 unless the rows are long), staging each
-// hyperplane with cp.async and reducing in the reference's lane order.
-// Writes the entry object and the leaf node reached; the leaf orders the
-// search's work list.
+// |margin| <= EPS goes left): every group of G lanes descends for its own query,
+// reading each hyperplane straight from L2 into registers in the reference's lane
+// order, its children and offset on their way at the same time (G = 4, eight
+// queries a warp; 16 for long rows).  Writes the entry object and the leaf node
+// reached; the leaf orders the search's work list.  Bound by the latency of a
+// row read per level; rows copied through shared memory 16 bytes a lane were
+// bound by its port: 30,000 queries, 1M x 128: 184 us then, 68 now.
+template <int G>
 __global__ void __launch_bounds__(128) rknn_entry_kernel(SearchParams p, uint32_t* __restrict__ enode,
-                                                         uint32_t* __restrict__ entry, uint32_t qpw) {
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5, gt = lane & 3u, gw = lane >> 2;
-    float* qhat = reinterpret_cast<float*>(g_smem) + ((size_t)wib * qpw + (gw < qpw ? gw : 0)) * 2 * p.lstride;
-    float* stage = qhat + p.lstride;
+                                                         uint32_t* __restrict__ entry) {
+    constexpr uint32_t kPerWarp = 32 / G;
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5, gt = lane & (G - 1), gw = lane / G;
+    float* qhat = reinterpret_cast<float*>(g_smem) + ((size_t)wib * kPerWarp + gw) * p.lstride;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t q0 = (blockIdx.x * (blockDim.x >> 5) + wib) * qpw; q0 < p.nq; q0 += warps * qpw) {
+    for (uint32_t q0 = (blockIdx.x * (blockDim.x >> 5) + wib) * kPerWarp; q0 < p.nq; q0 += warps * kPerWarp) {
         const uint32_t qi = q0 + gw;
-        const bool ok = gw < qpw && qi < p.nq;
-        if (ok) {
-            const float* q = p.queries + (size_t)qi * p.bstride;
-            for (uint32_t j = gt; j < p.lstride; j += 4) {
-                float v = 0.0f;
-                if (j < p.d) v = __double2float_rn(__dmul_rn((double)q[j], p.scale));
-                else if (j == p.d) v = 1.0f;
-                qhat[j] = v;
-            }
+        const bool ok = qi < p.nq;
+        const float* q = p.queries + (size_t)(ok ? qi : q0) * p.bstride;
+        for (uint32_t j = gt; j < p.lstride; j += G) {
+            float v = 0.0f;
+            if (j < p.d) v = __double2float_rn(__dmul_rn((double)q[j], p.scale));
+            else if (j == p.d) v = 1.0f;
+            qhat[j] = v;
         }
         __syncwarp();
         uint32_t v = p.troot;
         bool done = !ok;
         for (uint32_t depth = 0; depth < 4096; depth++) {
-            if (!done && p.tleft[v] == kEmpty) done = true;
+            const uint32_t left = p.tleft[v], right = p.tright[v];
+            const float off = p.toffset[v];
+            const float* h = p.thyper + (size_t)v * p.lstride;
+            float ip;
+            if constexpr (G == 4) ip = group_ip<8>(h, qhat, p.dim, gt, kFull);
+            else ip = group_ip_w<16, 20>(h, qhat, p.dim, gt, kFull);
+            if (!done && left == kEmpty) done = true;
             if (__all_sync(kFull, done)) break;
-            if (!done) stage_row_async(stage, p.thyper + (size_t)v * p.lstride, p.lstride, gt, 4);
-            cp_async_wait_all();
-            __syncwarp();
-            const float ip = group_ip(done ? qhat : stage, qhat, p.dim, gt, kFull);
-            __syncwarp();
             if (!done) {
-                const float margin = __fsub_rn(ip, p.toffset[v]);
-                v = (margin < -kSplitEps) ? p.tleft[v] : (margin > kSplitEps ? p.tright[v] : p.tleft[v]);
+                const float margin = __fsub_rn(ip, off);
+                v = (margin < -kSplitEps) ? left : (margin > kSplitEps ? right : left);
             }
         }
         if (ok && gt == 0) {
@@ -902,7 +904,6 @@ __global__ void __launch_bounds__(128) rknn_entry_kernel(SearchParams p, uint32_
             if (p.ip) {
                 // rknn_query.cpp:2724-2729: qn2s sums (q_j s)^2 in index order in
                 // double (multiply, then add); R2 = qn2s + 1 + M*^2
-                const float* q = p.queries + (size_t)qi * p.bstride;
                 double qn2s = 0.0;
                 for (uint32_t j = 0; j < p.d; j++) {
                     const double t = __dmul_rn((double)q[j], p.scale);
@@ -1445,13 +1446,16 @@ static int prepare_entries(Ctx* c, bool order, bool* ordered) {
     p.ip = ix.metric == ANQI_METRIC_IP;
     p.mstar2 = ix.mstar2;
     p.qR2f = p.ip ? b.qr2.as<float>() : nullptr;
-    // 8 queries per warp (one per 4-lane group) while their rows fit 48 KB per block
-    const uint32_t qpw = 4ull * 8 * 2 * ix.lstride * 4 <= 48 * 1024 ? 8u : 1u;
-    const size_t smem = 4ull * qpw * 2 * ix.lstride * 4;
+    // 8 queries per warp (a 4-lane group each) while their lifted vectors fit
+    // 48 KB per block, else 2
+    const bool four = 4ull * 8 * ix.lstride * 4 <= 48 * 1024;
+    const uint32_t qpw = four ? 8u : 2u;
+    const size_t smem = 4ull * qpw * ix.lstride * 4;
+    auto kern = four ? rknn_entry_kernel<4> : rknn_entry_kernel<16>;
     if (smem > 48 * 1024)
-        ANQI_CUDA(c, cudaFuncSetAttribute(rknn_entry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t blocks = std::min<uint32_t>(c->sm_count * 8, (nq + 4 * qpw - 1) / (4 * qpw));
-    rknn_entry_kernel<<<blocks, 128, smem, c->stream>>>(p, b.enode.as<uint32_t>(), b.entry.as<uint32_t>(), qpw);
+    kern<<<blocks, 128, smem, c->stream>>>(p, b.enode.as<uint32_t>(), b.entry.as<uint32_t>());
     const char* env = std::getenv("ANQI_B200_ORDER");
     *ordered = order && !(env && env[0] == '0');
     if (*ordered) {
