@@ -971,6 +971,13 @@ __global__ void join_fill_kernel(const uint32_t* __restrict__ samp, const uint32
     }
 }
 
+// The round's candidates pushed into their targets' heaps, a warp per target.
+// Bound by its chains of loads and its instructions, not by bytes: a target's
+// candidates are mostly ones its heap holds already, so a lane looks for its
+// candidate in the heap first, distances are taken for the others only, and a
+// push follows only where the value is not above the top.  Masks and samples are
+// read 32 at a time instead of list by list.  Three rounds over 200,000 x 130:
+// 27.0 ms pushing one candidate after the other, 13.3 ms this way.
 __global__ void __launch_bounds__(128) join_apply_kernel(const float* __restrict__ x, const float* __restrict__ norms,
                                                          uint64_t n, uint32_t stride, uint32_t dim,
                                                          const uint32_t* __restrict__ samp,
@@ -1016,44 +1023,111 @@ __global__ void __launch_bounds__(128) join_apply_kernel(const float* __restrict
         __syncwarp();
         const float* xt = x + t * stride;
         const float nt = norms[t];
+        // pushes of 32 candidates, a lane each, in lane order: one that the heap holds
+        // needs no value unless a push before it throws it out
+        auto push32 = [&](uint32_t w, bool have, uint32_t* si, float* sd) {
+            bool held = false;
+            for (uint32_t k = 0; k < K; k++) held |= hi[k] == w;
+            const uint32_t fresh = __ballot_sync(kAll, have && !held);
+            const uint32_t rank = __popc(fresh & lane_lt_mask()), nf = __popc(fresh);
+            if (have && !held) si[rank] = w;
+            __syncwarp();
+            for (uint32_t r0 = 0; r0 < nf; r0 += 8) {
+                const uint32_t idx = min(r0 + gw, nf - 1);
+                const uint32_t v = si[idx];
+                const float ip = group_ip(xt, x + (uint64_t)v * stride, dim, gt, kAll);
+                if (gt == 0) sd[idx] = norm_d2(nt, norms[v], ip);
+            }
+            __syncwarp();
+            float value = have && !held ? sd[rank] : 0.0f;
+            uint32_t todo = __ballot_sync(kAll, have);
+            for (;;) {
+                const uint32_t act = __ballot_sync(kAll, !held && !(value > hv[0])) & todo;
+                if (!act) break;
+                const int src = __ffs(act) - 1;
+                todo &= src == 31 ? 0u : ~((2u << src) - 1u);
+                const uint32_t out = hi[0];
+                __syncwarp();
+                if (!heap_push(hi, hv, K, __shfl_sync(kAll, w, src), __shfl_sync(kAll, value, src), lane)) continue;
+                local_upd++;
+                const bool lost = held && w == out;
+                if (__any_sync(kAll, lost && ((todo >> lane) & 1u))) {
+                    const float ip = group_ip(xt, x + (uint64_t)out * stride, dim, gt, kAll);
+                    if (lost) {
+                        value = norm_d2(nt, norms[out], ip);
+                        held = false;
+                    }
+                }
+            }
+            __syncwarp();
+        };
         uint32_t m = 0;
         auto flush = [&]() {
-            for (uint32_t r0 = 0; r0 < m; r0 += 8) {
-                const uint32_t idx = r0 + gw;
-                const bool ok = idx < m;
-                const uint32_t w = bi[ok ? idx : r0];
-                const float ip = group_ip(xt, x + (uint64_t)w * stride, dim, gt, kAll);
-                if (ok && gt == 0) bd[idx] = norm_d2(nt, norms[w], ip);
+            for (uint32_t r0 = 0; r0 < m; r0 += 32) {
+                const bool have = r0 + lane < m;
+                const uint32_t w = have ? bi[r0 + lane] : kEmpty;
+                __syncwarp();
+                push32(w, have, bi + r0, bd + r0);
             }
-            __syncwarp();
-            for (uint32_t q = 0; q < m; q++) local_upd += heap_push(hi, hv, K, bi[q], bd[q], lane) ? 1u : 0u;
             m = 0;
         };
-        for (uint32_t e = 0; e < s; e++) {
-            const uint64_t key = buf[e];
-            const uint64_t u = key >> 8;
-            const uint32_t a = (uint32_t)(key & 0xFF);
-            const uint32_t cu = scnt[u];
-            // candidates: the other sampled ids of u, in sample order
-            if (m + cu > kBatch + 1) flush();
-            if (mask) {
-                // precision form (S <= 32): only the candidates the tensor-core
-                // filter kept; the others would be rejected by the push
-                const uint32_t mk = mask[u * S + a] & (cu >= 32 ? kAll : ((1u << cu) - 1u));
-                if ((mk >> lane) & 1u) bi[m + __popc(mk & lane_lt_mask())] = samp[u * S + lane];
+        if (mask) {
+            // precision form (S <= 32): only the candidates the tensor-core filter
+            // kept; the others would be rejected by the push.  The masks of 32
+            // incoming lists are read at once, and lane j of a group takes the
+            // group's j-th set bit over them: lists and samples in their order.
+            for (uint32_t e0 = 0; e0 < s; e0 += 32) {
+                uint64_t u = 0;
+                uint32_t mk = 0;
+                if (e0 + lane < s) {
+                    const uint64_t key = buf[e0 + lane];
+                    u = key >> 8;
+                    const uint32_t cu = scnt[u];
+                    mk = mask[u * S + (uint32_t)(key & 0xFF)] & (cu >= 32 ? kAll : ((1u << cu) - 1u));
+                }
+                uint32_t end = __popc(mk);  // set bits up to and including the lane's list
+                for (uint32_t o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kAll, end, o);
+                    if (lane >= o) end += v;
+                }
+                const uint32_t total = __shfl_sync(kAll, end, 31);
+                for (uint32_t g = 0; g < total; g += 32) {
+                    const uint32_t pos = g + lane;
+                    const bool have = pos < total;
+                    uint32_t l = 0;  // the first list whose end lies past pos
+                    for (uint32_t o = 16; o; o >>= 1)
+                        if (__shfl_sync(kAll, end, l + o - 1) <= pos) l += o;
+                    const uint32_t lm = __shfl_sync(kAll, mk, l);
+                    const uint64_t lu = __shfl_sync(kAll, u, l);
+                    uint32_t r = pos - (__shfl_sync(kAll, end, l) - __popc(lm)), bit = 0;  // its r-th set bit
+                    for (uint32_t o = 16; o; o >>= 1) {
+                        const uint32_t c = __popc((lm >> bit) & ((1u << o) - 1u));
+                        if (r >= c) {
+                            r -= c;
+                            bit += o;
+                        }
+                    }
+                    push32(have ? samp[lu * S + bit] : kEmpty, have, bi, bd);
+                }
+            }
+        } else {
+            for (uint32_t e = 0; e < s; e++) {
+                const uint64_t key = buf[e];
+                const uint64_t u = key >> 8;
+                const uint32_t a = (uint32_t)(key & 0xFF);
+                const uint32_t cu = scnt[u];
+                // candidates: the other sampled ids of u, in sample order
+                if (m + cu > kBatch + 1) flush();
+                for (uint32_t b = lane; b < cu; b += 32) {
+                    if (b == a) continue;
+                    const uint32_t pos = m + (b < a ? b : b - 1);
+                    bi[pos] = samp[u * S + b];
+                }
                 __syncwarp();
-                m += __popc(mk);
-                continue;
+                m += cu - 1;
             }
-            for (uint32_t b = lane; b < cu; b += 32) {
-                if (b == a) continue;
-                const uint32_t pos = m + (b < a ? b : b - 1);
-                bi[pos] = samp[u * S + b];
-            }
-            __syncwarp();
-            m += cu - 1;
+            flush();
         }
-        flush();
         for (uint32_t k = lane; k < K; k += 32) {
             hid[t * K + k] = hi[k];
             hval[t * K + k] = hv[k];
