@@ -1394,8 +1394,7 @@ __global__ void __launch_bounds__(128) leaf_merge_kernel(const float* __restrict
                                                          uint64_t n, uint32_t stride, uint32_t dim,
                                                          const uint32_t* __restrict__ members, uint64_t pos_base,
                                                          uint64_t nslots, uint32_t* __restrict__ cnt, uint32_t cap,
-                                                         const uint32_t* __restrict__ cid,
-                                                         const float* __restrict__ ckey, uint32_t K,
+                                                         const uint2* __restrict__ cand, uint32_t K,
                                                          float* __restrict__ kd, uint32_t* __restrict__ ki,
                                                          uint32_t* __restrict__ ksz, uint32_t* __restrict__ err,
                                                          uint32_t mode) {
@@ -1431,8 +1430,9 @@ __global__ void __launch_bounds__(128) leaf_merge_kernel(const float* __restrict
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const uint32_t t = c0 + 32 * q + lane;
-                raw[q] = t < m ? cid[sl * cap + t] : (uint32_t)row;
-                key[q] = t < m ? ckey[sl * cap + t] : 0.f;
+                const uint2 pair = t < m ? cand[sl * cap + t] : make_uint2((uint32_t)row, 0u);
+                raw[q] = pair.x;
+                key[q] = __uint_as_float(pair.y);
                 const uint32_t id = raw[q] & ~kRecheck;
                 keep[q] = id != (uint32_t)row && id < n;
             }
@@ -2872,15 +2872,14 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
             // candidate buffers (n x cap entries; GBs at 1M) are kept by the
             // context: allocating them anew for every build cost up to seconds
             DevBuf& ccnt = c->init_cnt;
-            DevBuf& cid = c->init_cid;
-            DevBuf& ckey = c->init_key;
+            DevBuf& cand = c->init_cid;
             const uint32_t cap = round_up(std::max(maxcnt, 2u), 32u);
             // candidate slots for batches of leaves covering up to brows rows (~1 GB)
             uint64_t want = (512ull << 20) / (cap * 4ull);
             if (const char* e = std::getenv("ANQI_B200_INIT_BATCH_ROWS")) want = std::strtoull(e, nullptr, 10);
             const uint64_t brows = std::min<uint64_t>(n, std::max<uint64_t>(maxcnt, want));
             if (!(rc = tc_prep(c, dx.as<float>(), dn.as<float>(), n, xs, d, tp)) && !(rc = ensure(c, ccnt, brows * 4)) &&
-                !(rc = ensure(c, cid, brows * (size_t)cap * 4)) && !(rc = ensure(c, ckey, brows * (size_t)cap * 4))) {
+                !(rc = ensure(c, cand, brows * (size_t)cap * 8))) {
                 auto cu = [&](cudaError_t e, const char* what) { return e == cudaSuccess ? ANQI_OK : cuda_check(c, e, what); };
                 rc = cu(cudaMemsetAsync(ccnt.p, 0, brows * 4, c->stream), "cudaMemsetAsync");
                 const int wpb = 4;
@@ -2907,7 +2906,7 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                         while (l1 < lv.size() && lv[l1].off + lv[l1].cnt - base <= brows) l1++;
                         const std::vector<LeafRef> batch(lv.begin() + l0, lv.begin() + l1);
                         const size_t t0 = tiles.size();
-                        rc = tc_leaf_tiles(c, batch, cap, tiles);
+                        rc = tc_leaf_tiles(c, batch, tp, maxcnt, cap, tiles);
                         plan.push_back({base, lv[l1 - 1].off + lv[l1 - 1].cnt - base, t0, tiles.size() - t0});
                         l0 = l1;
                     }
@@ -2917,14 +2916,14 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                 for (size_t b = 0; b < plan.size() && !rc; b++) {
                     const BatchPlan& bp = plan[b];
                     rc = tc_leaf_filter(c, tp, dx.as<float>(), dn.as<float>(), n, xs, d, f.perm.as<uint32_t>(),
-                                        dtiles.as<LeafTile>() + bp.t0, bp.nt, kd.as<float>(), ksz.as<uint32_t>(), K,
-                                        ccnt.as<uint32_t>(), cap, cid.as<uint32_t>(), ckey.as<float>(), bp.base,
+                                        dtiles.as<LeafTile>() + bp.t0, bp.nt, maxcnt, kd.as<float>(),
+                                        ksz.as<uint32_t>(), K, ccnt.as<uint32_t>(), cap, cand.as<uint2>(), bp.base,
                                         ip ? kKeyIpDist : kKeyL2);
                     if (rc) break;
                     leaf_merge_kernel<<<c->sm_count * 12, 32 * wpb, msmem, c->stream>>>(
                         dx.as<float>(), dn.as<float>(), n, xs, d, f.perm.as<uint32_t>(), bp.base, bp.nslots,
-                        ccnt.as<uint32_t>(), cap, cid.as<uint32_t>(), ckey.as<float>(), K, kd.as<float>(),
-                        ki.as<uint32_t>(), ksz.as<uint32_t>(), c->err.as<uint32_t>(), ip ? kKeyIpDist : kKeyL2);
+                        ccnt.as<uint32_t>(), cap, cand.as<uint2>(), K, kd.as<float>(), ki.as<uint32_t>(),
+                        ksz.as<uint32_t>(), c->err.as<uint32_t>(), ip ? kKeyIpDist : kKeyL2);
                     rc = cu(cudaGetLastError(), "leaf_merge_kernel");
                 }
                 if (!rc) rc = check_device_error(c, "tensor-core init_knn");

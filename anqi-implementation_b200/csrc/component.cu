@@ -714,7 +714,7 @@ int plan_batches(Ctx* c, const CompGather& g, const std::vector<CompRange>& rang
     int rc;
     std::vector<uint32_t> rows(g.n, kEmpty);
     std::vector<CompDesc> descs(ranges.size());
-    const uint64_t budget = std::max<uint64_t>(c->init_key.bytes, 256ull << 20) / 4;
+    const uint64_t budget = std::max<uint64_t>(c->init_cid.bytes, 256ull << 20) / 4;
     for (size_t k = 0; k < ranges.size();) {
         CompBatch b{k, k, 0, 1, 0};
         uint64_t goff = 0;
@@ -732,7 +732,7 @@ int plan_batches(Ctx* c, const CompGather& g, const std::vector<CompRange>& rang
             for (uint32_t t = 0; t < r.size; t++) rows[r.start + t] = (uint32_t)b.c1;
             b.c1++;
         }
-        if ((rc = ensure(c, c->init_key, goff * 4)) || (rc = ensure(c, c->init_cid, b.aoff * 4))) return rc;
+        if ((rc = ensure(c, c->init_cid, goff * 4)) || (rc = ensure(c, c->init_key, b.aoff * 4))) return rc;
         batches.push_back(b);
         k = b.c1;
     }
@@ -749,10 +749,10 @@ int launch_tables(Ctx* c, const CompGather& g, const CompBatch& b, const CompDes
                   const DevBuf& row_comp, const DevBuf& bad) {
     const uint32_t nc = (uint32_t)(b.c1 - b.c0);
     comp_gram_kernel<<<b.tiles, 256, 0, c->stream>>>(g.x, g.norms, g.stride, g.dim, g.cols, comps, nc,
-                                                     c->init_key.as<float>(), bad.as<uint32_t>());
+                                                     c->init_cid.as<float>(), bad.as<uint32_t>());
     comp_adj_kernel<<<(unsigned)((hi - lo + 3) / 4), 128, 0, c->stream>>>(
         lo, hi, row_comp.as<uint32_t>(), comps, (uint32_t)b.c0, nc, g.g_ids, g.K, g.rev_off, g.rev_ids,
-        c->init_cid.as<uint32_t>());
+        c->init_key.as<uint32_t>());
     ANQI_CUDA(c, cudaGetLastError());
     return ANQI_OK;
 }
@@ -787,8 +787,8 @@ int run_component_gather(Ctx* c, const CompGather& g, const std::vector<CompRang
         p.comps = comps;
         p.first = (uint32_t)b.c0;
         p.ncomps = (uint32_t)(b.c1 - b.c0);
-        p.G = c->init_key.as<float>();
-        p.adj = c->init_cid.as<uint32_t>();
+        p.G = c->init_cid.as<float>();
+        p.adj = c->init_key.as<uint32_t>();
         p.bad = bad.as<uint32_t>();
         p.g_ids = g.g_ids;
         p.g_vals = g.g_vals;
@@ -834,8 +834,8 @@ int run_component_select_commit(Ctx* c, const CompGather& g, const std::vector<C
         p.comps = comps;
         p.first = (uint32_t)b.c0;
         p.ncomps = (uint32_t)(b.c1 - b.c0);
-        p.G = c->init_key.as<float>();
-        p.adj = c->init_cid.as<uint32_t>();
+        p.G = c->init_cid.as<float>();
+        p.adj = c->init_key.as<uint32_t>();
         p.bad = bad.as<uint32_t>();
         p.g_ids = g.g_ids;
         p.K = g.K;

@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <vector>
 
 #include "internal.h"
@@ -179,6 +180,7 @@ struct FilterParams {
     uint32_t cap;
     uint32_t* out_id;         // row * cap + slot
     float* out_key;
+    uint2* out_pair;          // leaf mode: (id, key bits) in place of both
     uint32_t* err;
     // leaf mode (init_knn): CTA x = leaf_tiles[x]; rows members[off + 128 rb ..],
     // columns members[off .. off + cnt); the row threshold is its current
@@ -400,8 +402,8 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
                 const uint64_t cs0 = lt.off + (uint64_t)lt.rb * kTile + r - p.pos_base;
                 const uint32_t pos = atomicAdd(s_cnt + r, 1u);
                 if (pos < p.cap) {
-                    p.out_id[cs0 * p.cap + pos] = (uint32_t)j | (exact ? 0u : kRecheck);
-                    p.out_key[cs0 * p.cap + pos] = approx;
+                    p.out_pair[cs0 * p.cap + pos] =
+                        make_uint2((uint32_t)j | (exact ? 0u : kRecheck), __float_as_uint(approx));
                 }
             }
         }
@@ -516,6 +518,228 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
     if (warp == 0) tc::tmem_free(tslot, 256);
     if (threadIdx.x < kTile && rowid[threadIdx.x] != ~0ull)
         p.cnt[lt.off + (uint64_t)lt.rb * kTile + threadIdx.x - p.pos_base] = s_cnt[threadIdx.x];
+}
+
+// ------------------------------------------------------- whole leaves
+// init_knn's leaves while a leaf's rows fit in shared memory (LeafParams below):
+// a CTA per leaf, or per `parts`-th row block of one where leaves are few.  The
+// rows come in once, a bulk of 16-byte copies per 128-row tile, and serve as both
+// operands; warp 16 issues the 128 x 128 products into a ring of four TMEM
+// accumulators, and warps 0-15 test them: warp w TMEM lanes 32 (w % 4) .. + 31,
+// its rows, and columns 32 (w / 4) .. + 31.  An accumulator is free again as soon
+// as it is in registers.  Rows and columns that are all exact take three
+// instructions a pair; the others the full error bound, with its column terms
+// read four at a time.  Survivors, about a tenth of the pairs once the lists are
+// full, take one slot reservation per 32 pairs and one 8-byte store each, without
+// a loop over set bits (whose length is the warp's longest).
+// Bound by issue and, with one CTA to an SM, by the time its rows take to come in.
+// 64 trees over 1M x 128 (integers): 44.2 ms, the 128-row-tile form 81.6 ms; over
+// 5,003 x 37: 0.93 and 1.69 ms; over 100,000 x 100 (ip, no exact rows): 5.9 and
+// 6.4 ms.
+constexpr uint32_t kLeafWarps = 16;
+constexpr uint32_t kLeafThreads = 32 * (kLeafWarps + 1);
+constexpr uint32_t kLeafTiles = 4;
+constexpr uint32_t kLeafRows = kLeafTiles * kTile;
+
+__host__ __device__ constexpr size_t leaf_smem(uint32_t dp, uint32_t tiles) {
+    return (size_t)tiles * kTile * dp * 2 + 6 * (size_t)kLeafRows * 4;
+}
+
+__global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p, uint32_t tiles) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    const size_t tile_bytes = (size_t)kTile * p.dp * 2;
+    uint32_t* mid = reinterpret_cast<uint32_t*>(sm + tiles * tile_bytes);  // per member: id, norm, |x|, error, threshold
+    float* mn = reinterpret_cast<float*>(mid + kLeafRows);
+    float* mnorm = mn + kLeafRows;
+    float* merr = mnorm + kLeafRows;
+    float* mthr = merr + kLeafRows;
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(mthr + kLeafRows);
+    __shared__ uint64_t full[kLeafTiles], accfull[4], accempty[4], drained;
+    __shared__ uint32_t s_int[kLeafRows / 32];  // exact members, a bit each
+    __shared__ uint32_t tslot;
+    __shared__ volatile int s_abort;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const LeafTile lt = p.leaf_tiles[blockIdx.x];
+    const uint32_t* mem = p.members + lt.off;
+    const uint32_t cnt = lt.cnt, T = (cnt + kTile - 1) / kTile;
+    if (blockIdx.y >= T) return;
+    if (warp == kLeafWarps) {
+        tc::tmem_alloc(&tslot, 512);
+        if (lane == 0) {
+            for (uint32_t k = 0; k < kLeafTiles; k++) tc::mbar_init(&full[k], kLeafWarps);
+            for (uint32_t k = 0; k < 4; k++) {
+                tc::mbar_init(&accfull[k], 1);
+                tc::mbar_init(&accempty[k], kLeafWarps);
+            }
+            tc::mbar_init(&drained, 1);
+            tc::fence_mbar_init();
+            s_abort = 0;
+        }
+    } else {
+        const uint32_t t = threadIdx.x;
+        const bool ok = t < cnt;
+        const uint32_t j = ok ? mem[t] : 0u;
+        mid[t] = j;
+        mn[t] = ok ? p.xn[j] : 0.f;
+        mnorm[t] = ok ? p.xnorm[j] : 0.f;
+        merr[t] = ok ? p.xerr[j] : 0.f;
+        float thr = __int_as_float(0x7f800000);
+        if (ok && p.list_sz[j] >= p.list_k) thr = p.list_kd[(uint64_t)j * p.list_k + p.list_k - 1];
+        mthr[t] = thr;
+        s_cnt[t] = 0;
+        const uint32_t in = __ballot_sync(0xFFFFFFFFu, ok && p.xint[j]);
+        if (lane == 0) s_int[warp] = in;
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tslot;
+    // every wait is bounded; one that runs out makes all roles leave
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (!s_abort && tc::mbar_wait(bar, parity, kWaitPolls)) return true;
+        s_abort = 1;
+        atomicExch(p.err, 8u);
+        return false;
+    };
+    bool ok = true;
+    if (warp == kLeafWarps) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (uint32_t rb = blockIdx.y; rb < T && ok; rb += gridDim.y) {
+                if (!(ok = wait(&full[rb], 0))) break;
+                for (uint32_t t = 0; t < T; t++, it++) {
+                    const uint32_t b = it & 3u;
+                    if (!(ok = wait(&full[t], 0))) break;
+                    if (it >= 4 && !(ok = wait(&accempty[b], (it / 4 - 1) & 1u))) break;
+                    tc::fence_after_sync();
+                    issue_tile_mma(tmem + b * kTile, sm + rb * tile_bytes, sm + t * tile_bytes, p.dp);
+                    tc::mma_commit(&accfull[b]);
+                }
+            }
+            if (!ok) {
+                tc::mma_commit(&drained);
+                tc::mbar_wait(&drained, 0, kWaitPolls);
+            }
+        }
+    } else {
+        // a warp's copy: 16 rows, 32 bytes (two K groups) of each
+        const uint32_t units = 8 * (p.dp / 16);
+        for (uint32_t t = 0; t < T; t++) {
+            unsigned char* dst = sm + t * tile_bytes;
+            for (uint32_t u = warp; u < units; u += kLeafWarps) {
+                const uint32_t rr = 16 * (u & 7u) + (lane >> 1), c = 2 * (u >> 3) + (lane & 1u);
+                const uint32_t pos = t * kTile + rr;
+                tc::cp_async16_zfill(dst + (size_t)c * kTile * 16 + rr * 16, p.xb + (uint64_t)mid[pos] * p.dp + 8 * c,
+                                     pos < cnt ? 16u : 0u);
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        for (uint32_t t = 0; t < T; t++) {
+            switch (T - 1 - t) {
+                case 0: asm volatile("cp.async.wait_group 0;\n" ::: "memory"); break;
+                case 1: asm volatile("cp.async.wait_group 1;\n" ::: "memory"); break;
+                case 2: asm volatile("cp.async.wait_group 2;\n" ::: "memory"); break;
+                default: asm volatile("cp.async.wait_group 3;\n" ::: "memory"); break;
+            }
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&full[t]);
+        }
+        const uint32_t quarter = warp & 3u, cg = warp >> 2;
+        const bool l2k = p.key_mode == 0;
+        const bool plain = p.all_exact && p.d <= 128;  // every key exact: no bound, no recheck
+        const float u = 5.9604645e-8f;  // 2^-24
+        const float g = 2.0f * p.dp * u;
+        const float kh = l2k ? 1.f : 0.5f;
+        const float cc = l2k ? 4.f * u : 0.f;
+        const float f = l2k ? 2.f : 1.f;
+        uint32_t it = 0;
+        for (uint32_t rb = blockIdx.y; rb < T && ok; rb += gridDim.y) {
+            const uint32_t row = rb * kTile + quarter * 32 + lane;
+            const bool row_ok = row < cnt;
+            const bool rows_any = rb * kTile + quarter * 32 < cnt;
+            const float qn = l2k ? mn[row] : 1.f;
+            const float thr = mthr[row];
+            const float qnm = mnorm[row], qer = merr[row];
+            const bool qexact = ((s_int[row >> 5] >> lane) & 1u) && p.d <= 128;
+            // the row's error bound, as in tc_filter_kernel
+            const float ca = kh * (2.f * qer + 4.f * g * (qnm + qer) + 4.f * g * qnm + 8.f * u * qnm);
+            const float cb = kh * (2.f * qnm + 2.f * qer + 4.f * g * (qnm + qer));
+            const float cd = l2k ? 4.f * u * qn : 4.f * u;
+            const float R = thr - qn;
+            uint2* out = p.out_pair + (lt.off + row - p.pos_base) * p.cap;
+            for (uint32_t t = 0; t < T; t++, it++) {
+                const uint32_t b = it & 3u, c0 = t * kTile + cg * 32;
+                ok = __all_sync(0xFFFFFFFFu, wait(&accfull[b], (it / 4) & 1u));
+                if (!ok) break;
+                tc::fence_after_sync();
+                float v[32];
+                tc::tmem_ld32(tmem + ((quarter * 32u) << 16) + b * kTile + cg * 32, v);
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&accempty[b]);
+                if (!rows_any || c0 >= cnt) continue;
+                uint32_t keep = 0, flag = 0;  // bit k: column c0 + k
+                if (plain) {
+                    // key <= thr as the sign of (thr - qn) - xn + 2 acc, exact here
+#pragma unroll
+                    for (uint32_t k = 0; k < 32; k += 4) {
+                        const float4 x4 = *reinterpret_cast<const float4*>(mn + c0 + k);
+                        const float xa[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; e++)
+                            keep = __funnelshift_r(keep, __float_as_uint(fmaf(f, v[k + e], l2k ? R - xa[e] : R)) >> 31, 1);
+                    }
+                    keep = ~keep;
+                } else {
+                    const uint32_t cint = qexact ? s_int[c0 >> 5] : 0u;
+#pragma unroll
+                    for (uint32_t k = 0; k < 32; k += 4) {
+                        const float4 x4 = *reinterpret_cast<const float4*>(mn + c0 + k);
+                        const float4 n4 = *reinterpret_cast<const float4*>(mnorm + c0 + k);
+                        const float4 e4 = *reinterpret_cast<const float4*>(merr + c0 + k);
+                        const float xa[4] = {x4.x, x4.y, x4.z, x4.w}, na[4] = {n4.x, n4.y, n4.z, n4.w};
+                        const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; e++) {
+                            const float approx = fmaf(-f, v[k + e], l2k ? __fadd_rn(qn, xa[e]) : 1.f);
+                            float eps = fmaf(ca, na[e], fmaf(cb, ea[e], fmaf(cc, xa[e], cd)));
+                            if ((cint >> (k + e)) & 1u) eps = 0.f;
+                            if (approx - eps <= thr) keep |= 1u << (k + e);
+                        }
+                    }
+                    flag = ~cint;
+                }
+                const uint32_t left = cnt - c0, self = row - c0;
+                if (left < 32) keep &= (1u << left) - 1u;
+                if (self < 32) keep &= ~(1u << self);
+                if (!row_ok) keep = 0;
+                if (!__any_sync(0xFFFFFFFFu, keep != 0)) continue;
+                uint2* o = out;
+                if (keep) o += atomicAdd(s_cnt + row, __popc(keep));
+#pragma unroll
+                for (uint32_t k = 0; k < 32; k += 4) {
+                    const float4 x4 = *reinterpret_cast<const float4*>(mn + c0 + k);
+                    const uint4 i4 = *reinterpret_cast<const uint4*>(mid + c0 + k);
+                    const float xa[4] = {x4.x, x4.y, x4.z, x4.w};
+                    const uint32_t ia[4] = {i4.x, i4.y, i4.z, i4.w};
+#pragma unroll
+                    for (uint32_t e = 0; e < 4; e++) {
+                        if (keep & (1u << (k + e))) {
+                            const float approx = fmaf(-f, v[k + e], l2k ? __fadd_rn(qn, xa[e]) : 1.f);
+                            *o++ = make_uint2(ia[e] | ((flag >> (k + e)) & 1u ? kRecheck : 0u), __float_as_uint(approx));
+                        }
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == kLeafWarps) tc::tmem_free(tmem, 512);
+    else if (threadIdx.x < cnt && (threadIdx.x / kTile) % gridDim.y == blockIdx.y)
+        p.cnt[lt.off + threadIdx.x - p.pos_base] = s_cnt[threadIdx.x];
 }
 
 // ------------------------------------------------------------- scan
@@ -1320,18 +1544,28 @@ int tc_join_filter(Ctx* c, const TcPrep& tp, const float* d_norms, uint64_t n, c
     return ANQI_OK;
 }
 
-int tc_leaf_tiles(Ctx* c, const std::vector<LeafRef>& leaves, uint32_t cap, std::vector<LeafTile>& tiles) {
+// Whether leaves of up to maxcnt rows run whole (tc_leaf_kernel): their rows, padded
+// to 128, are in shared memory together (four tiles up to 208 dimensions).  It was
+// the faster one at every size tried; longer leaves and rows take the tiles.
+static bool leaf_whole(uint32_t dp, uint32_t maxcnt) {
+    const char* env = std::getenv("ANQI_B200_LEAF_WHOLE");
+    return maxcnt <= kLeafRows && leaf_smem(dp, (maxcnt + kTile - 1) / kTile) <= 226 * 1024 && !(env && env[0] == '0');
+}
+
+int tc_leaf_tiles(Ctx* c, const std::vector<LeafRef>& leaves, const TcPrep& tp, uint32_t maxcnt, uint32_t cap,
+                  std::vector<LeafTile>& tiles) {
+    const bool whole = leaf_whole(tp.dp, maxcnt);
     for (const LeafRef& l : leaves) {
         if (l.cnt > cap + 1) return fail(c, ANQI_ERR_ARGS, "leaf of %u rows exceeds the candidate capacity", l.cnt);
-        for (uint32_t rb = 0; rb * kTile < l.cnt; rb++) tiles.push_back({l.off, l.cnt, rb});
+        for (uint32_t rb = 0; rb * kTile < (whole ? 1 : l.cnt); rb++) tiles.push_back({l.off, l.cnt, rb});
     }
     return ANQI_OK;
 }
 
 int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_norms, uint64_t n, uint32_t xs,
                    uint32_t d, const uint32_t* d_members, const LeafTile* d_tiles, size_t ntiles,
-                   const float* list_kd, const uint32_t* list_sz, uint32_t K, uint32_t* cnt, uint32_t cap,
-                   uint32_t* out_id, float* out_key, uint64_t pos_base, uint32_t key_mode) {
+                   uint32_t maxcnt, const float* list_kd, const uint32_t* list_sz, uint32_t K, uint32_t* cnt,
+                   uint32_t cap, uint2* out_pair, uint64_t pos_base, uint32_t key_mode) {
     if (ntiles == 0) return ANQI_OK;
     if (key_mode > 1) return fail(c, ANQI_ERR_ARGS, "leaf tiles take the l2 or ip distance, not mode %u", key_mode);
     FilterParams p{};
@@ -1347,8 +1581,7 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     p.dp = tp.dp;
     p.cnt = cnt;
     p.cap = cap;
-    p.out_id = out_id;
-    p.out_key = out_key;
+    p.out_pair = out_pair;
     p.err = c->err.as<uint32_t>();
     p.leaf_tiles = d_tiles;
     p.members = d_members;
@@ -1362,6 +1595,16 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     p.bx_n = tp.bn;
     p.all_exact = tp.all_exact;
     p.nrows = ntiles * kTile;
+    if (leaf_whole(p.dp, maxcnt)) {
+        const uint32_t tiles = (maxcnt + kTile - 1) / kTile;
+        const size_t bytes = leaf_smem(p.dp, tiles);
+        ANQI_CUDA(c, cudaFuncSetAttribute(tc_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        // few leaves: their row blocks over several CTAs while SMs are idle
+        const uint32_t parts = (uint32_t)std::max<size_t>(1, std::min<size_t>(tiles, c->sm_count / ntiles));
+        tc_leaf_kernel<<<dim3((unsigned)ntiles, parts), kLeafThreads, bytes, c->stream>>>(p, tiles);
+        ANQI_CUDA(c, cudaGetLastError());
+        return ANQI_OK;
+    }
     void (*kern)(FilterParams) = nullptr;
     size_t smem = 0;
     int rc;
