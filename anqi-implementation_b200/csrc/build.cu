@@ -1379,6 +1379,9 @@ __host__ __device__ __forceinline__ size_t merge_smem_words(uint32_t K) {
     return 2 * (size_t)((K + 3) & ~3u) + 128;
 }
 
+// Brings the line of *p into L2; nothing waits for it.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Merges one tree's tensor-core init_knn candidates (tc_leaf_filter) into every
 // row's list.  After the first trees nearly every candidate is already in the
 // row's list, so those go first, by their key when it is exact (a binary search)
@@ -1388,8 +1391,12 @@ __host__ __device__ __forceinline__ size_t merge_smem_words(uint32_t K) {
 // is recomputed in FP32 in the leaf_topk_kernel arithmetic (mode kKeyL2: the AVX
 // lane order; kKeyIpDist: 1 - <a, b> summed in sequence) and inserted in place.
 // The list stays the K smallest unique (key, id) of all candidates seen,
-// whatever their order.  Resets cnt.  One warp per row.  1M x 128, 64 trees:
-// 110 ms, from 146 ms of sorting and merging every candidate; bound by issue.
+// whatever their order.  Resets cnt.  One warp per row, up to eight rows in a run:
+// their counts and sizes come together, a row's list and first candidates are in
+// flight at once and the next row's are brought into L2, which took 105 ms to 90
+// (1M x 128, 64 trees; sorting and merging every candidate: 146).  The first
+// eight trees, whose candidates mostly enter, are 39 ms of it and bound by issue;
+// the later ones, 0.6 ms each, by the latency of one row after the other.
 __global__ void __launch_bounds__(128) leaf_merge_kernel(const float* __restrict__ x, const float* __restrict__ norms,
                                                          uint64_t n, uint32_t stride, uint32_t dim,
                                                          const uint32_t* __restrict__ members, uint64_t pos_base,
@@ -1406,108 +1413,154 @@ __global__ void __launch_bounds__(128) leaf_merge_kernel(const float* __restrict
     uint32_t* wi = reinterpret_cast<uint32_t*>(wd + 64);
     const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t sl = w0; sl < nslots; sl += nw) {
-        uint32_t m = cnt[sl];
-        if (m == 0) continue;
-        const uint64_t row = members[pos_base + sl];
-        if (m > cap) {
-            if (lane == 0) set_error(err, kDevPoolOverflow);
-            m = cap;
+    // a warp's slots come up to eight in a run, their count, row and list size
+    // read together (fewer where the warps would not all have one)
+    const uint32_t run = (uint32_t)min((uint64_t)8, max((uint64_t)1, nslots / nw));
+    const uint32_t list_lines = (K * 4 + 127) / 128;
+    for (uint64_t s0 = w0 * run; s0 < nslots; s0 += nw * run) {
+        const uint32_t rn = (uint32_t)min((uint64_t)run, nslots - s0);
+        uint32_t cnt_l = 0, row_l = 0, size_l = 0;
+        if (lane < rn) {
+            cnt_l = cnt[s0 + lane];
+            row_l = members[pos_base + s0 + lane];
+            size_l = ksz[row_l];
         }
-        uint32_t size = ksz[row];
-        for (uint32_t t = lane; t < K4; t += 32) {
-            li[t] = t < size ? ki[row * K + t] : kEmpty;
-            if (t < size) ld[t] = kd[row * K + t];
-        }
-        bool changed = false;
-        __syncwarp();
-        const float nr = norms[row];
-        const float* xi = x + row * stride;
-        for (uint32_t c0 = 0; c0 < m; c0 += 64) {
-            uint32_t raw[2], kept = 0;
-            float key[2];
-            bool keep[2];
+        for (uint32_t e = 0; e < rn; e++) {
+            const uint64_t sl = s0 + e;
+            uint32_t m = __shfl_sync(kAll, cnt_l, e);
+            const uint64_t row = __shfl_sync(kAll, row_l, e);
+            uint32_t size = __shfl_sync(kAll, size_l, e);
+            const uint32_t m_next = __shfl_sync(kAll, cnt_l, (e + 1) & 31u);
+            const uint64_t row_next = __shfl_sync(kAll, row_l, (e + 1) & 31u);
+            if (e + 1 < rn && m_next) {
+                const uint32_t t = lane & 15u;
+                if (lane >= 16 && t * 16 < m_next) prefetch_l2(cand + (sl + 1) * cap + t * 16);
+                if (lane < 16 && t < 2 * list_lines) {
+                    const uint32_t at = min((t >> 1) * 32, K - 1);
+                    if (t & 1u) prefetch_l2(kd + row_next * K + at);
+                    else prefetch_l2(ki + row_next * K + at);
+                }
+            }
+            if (m == 0) continue;
+            if (m > cap) {
+                if (lane == 0) set_error(err, kDevPoolOverflow);
+                m = cap;
+            }
+            // the list and the first candidates on their way together
+            uint2 first_c[2];
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                const uint32_t t = c0 + 32 * q + lane;
-                const uint2 pair = t < m ? cand[sl * cap + t] : make_uint2((uint32_t)row, 0u);
-                raw[q] = pair.x;
-                key[q] = __uint_as_float(pair.y);
-                const uint32_t id = raw[q] & ~kRecheck;
-                keep[q] = id != (uint32_t)row && id < n;
+                const uint32_t t = 32 * q + lane;
+                first_c[q] = t < m ? cand[sl * cap + t] : make_uint2((uint32_t)row, 0u);
             }
-            // those already in the list
-            const bool flag = (keep[0] && (raw[0] & kRecheck)) || (keep[1] && (raw[1] & kRecheck));
-            const bool flags = __any_sync(kAll, flag);
-            if (flags) {
-                const uint4* l4 = reinterpret_cast<const uint4*>(li);
-                const uint32_t a = raw[0] & ~kRecheck, b = raw[1] & ~kRecheck;
-                bool in0 = false, in1 = false;
-                for (uint32_t t = 0; 4 * t < size; t++) {
-                    const uint4 x4 = l4[t];
-                    in0 |= x4.x == a || x4.y == a || x4.z == a || x4.w == a;
-                    in1 |= x4.x == b || x4.y == b || x4.z == b || x4.w == b;
-                }
-                keep[0] &= !in0;
-                keep[1] &= !in1;
-            } else {
+            for (uint32_t t0 = 0; t0 < K4; t0 += 128) {
+                uint32_t a[4];
+                float b[4];
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    if (!keep[q]) continue;
-                    const uint32_t pos = lower_rank(ld, li, size, key[q], raw[q]);
-                    keep[q] = !(pos < size && li[pos] == raw[q]);
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint32_t t = t0 + 32 * q + lane;
+                    a[q] = t < size ? ki[row * K + t] : kEmpty;
+                    b[q] = t < size ? kd[row * K + t] : 0.f;
                 }
-            }
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const unsigned b = __ballot_sync(kAll, keep[q]);
-                if (keep[q]) {
-                    const uint32_t w = kept + __popc(b & lane_lt_mask());
-                    wd[w] = key[q];
-                    wi[w] = raw[q];
-                }
-                kept += __popc(b);
-            }
-            __syncwarp();
-            if (kept == 0) continue;
-            if (flags && mode == kKeyIpDist) {
-                // the ip distance in the sequential order of leaf_topk_kernel
-                for (uint32_t t = lane; t < kept; t += 32) {
-                    const uint32_t r = wi[t];
-                    if (r & kRecheck) wd[t] = ip_dist_seq(xi, x + (uint64_t)(r & ~kRecheck) * stride, dim);
-                    wi[t] = r & ~kRecheck;
-                }
-                __syncwarp();
-            } else if (flags) {
-                for (uint32_t r0 = 0; r0 < kept; r0 += 8) {
-                    const uint32_t idx = r0 + gw;
-                    const uint32_t r = wi[idx < kept ? idx : r0], j = r & ~kRecheck;
-                    const bool re = idx < kept && (r & kRecheck);
-                    if (__any_sync(kAll, re)) {
-                        const float ip = group_ip(xi, x + (uint64_t)j * stride, dim, gt, kAll);
-                        __syncwarp();
-                        if (re && gt == 0) {
-                            wd[idx] = norm_d2(nr, norms[j], ip);
-                            wi[idx] = j;
-                        }
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint32_t t = t0 + 32 * q + lane;
+                    if (t < K4) {
+                        li[t] = a[q];
+                        ld[t] = b[q];
                     }
                 }
+            }
+            bool changed = false;
+            __syncwarp();
+            const float nr = norms[row];
+            const float* xi = x + row * stride;
+            for (uint32_t c0 = 0; c0 < m; c0 += 64) {
+                uint32_t raw[2], kept = 0;
+                float key[2];
+                bool keep[2];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const uint32_t t = c0 + 32 * q + lane;
+                    const uint2 pair = c0 == 0 ? first_c[q] : t < m ? cand[sl * cap + t] : make_uint2((uint32_t)row, 0u);
+                    raw[q] = pair.x;
+                    key[q] = __uint_as_float(pair.y);
+                    const uint32_t id = raw[q] & ~kRecheck;
+                    keep[q] = id != (uint32_t)row && id < n;
+                }
+                // those already in the list
+                const bool flag = (keep[0] && (raw[0] & kRecheck)) || (keep[1] && (raw[1] & kRecheck));
+                const bool flags = __any_sync(kAll, flag);
+                if (flags) {
+                    const uint4* l4 = reinterpret_cast<const uint4*>(li);
+                    const uint32_t a = raw[0] & ~kRecheck, b = raw[1] & ~kRecheck;
+                    bool in0 = false, in1 = false;
+                    for (uint32_t t = 0; 4 * t < size; t++) {
+                        const uint4 x4 = l4[t];
+                        in0 |= x4.x == a || x4.y == a || x4.z == a || x4.w == a;
+                        in1 |= x4.x == b || x4.y == b || x4.z == b || x4.w == b;
+                    }
+                    keep[0] &= !in0;
+                    keep[1] &= !in1;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        if (!keep[q]) continue;
+                        const uint32_t pos = lower_rank(ld, li, size, key[q], raw[q]);
+                        keep[q] = !(pos < size && li[pos] == raw[q]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const unsigned b = __ballot_sync(kAll, keep[q]);
+                    if (keep[q]) {
+                        const uint32_t w = kept + __popc(b & lane_lt_mask());
+                        wd[w] = key[q];
+                        wi[w] = raw[q];
+                    }
+                    kept += __popc(b);
+                }
                 __syncwarp();
+                if (kept == 0) continue;
+                if (flags && mode == kKeyIpDist) {
+                    // the ip distance in the sequential order of leaf_topk_kernel
+                    for (uint32_t t = lane; t < kept; t += 32) {
+                        const uint32_t r = wi[t];
+                        if (r & kRecheck) wd[t] = ip_dist_seq(xi, x + (uint64_t)(r & ~kRecheck) * stride, dim);
+                        wi[t] = r & ~kRecheck;
+                    }
+                    __syncwarp();
+                } else if (flags) {
+                    for (uint32_t r0 = 0; r0 < kept; r0 += 8) {
+                        const uint32_t idx = r0 + gw;
+                        const uint32_t r = wi[idx < kept ? idx : r0], j = r & ~kRecheck;
+                        const bool re = idx < kept && (r & kRecheck);
+                        if (__any_sync(kAll, re)) {
+                            const float ip = group_ip(xi, x + (uint64_t)j * stride, dim, gt, kAll);
+                            __syncwarp();
+                            if (re && gt == 0) {
+                                wd[idx] = norm_d2(nr, norms[j], ip);
+                                wi[idx] = j;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+                const uint32_t first = beam_insert(ld, li, size, K, wd, wi, kept, lane);
+                changed |= first < size;  // something entered
             }
-            const uint32_t first = beam_insert(ld, li, size, K, wd, wi, kept, lane);
-            changed |= first < size;  // something entered
-        }
-        if (changed) {
-            for (uint32_t t = lane; t < size; t += 32) {
-                kd[row * K + t] = ld[t];
-                ki[row * K + t] = li[t];
+            if (changed) {
+                for (uint32_t t = lane; t < size; t += 32) {
+                    kd[row * K + t] = ld[t];
+                    ki[row * K + t] = li[t];
+                }
             }
+            if (lane == 0) {
+                if (changed) ksz[row] = size;
+                cnt[sl] = 0;
+            }
+            __syncwarp();
         }
-        if (lane == 0) {
-            if (changed) ksz[row] = size;
-            cnt[sl] = 0;
-        }
-        __syncwarp();
     }
 }
 
@@ -2920,7 +2973,7 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                                         ksz.as<uint32_t>(), K, ccnt.as<uint32_t>(), cap, cand.as<uint2>(), bp.base,
                                         ip ? kKeyIpDist : kKeyL2);
                     if (rc) break;
-                    leaf_merge_kernel<<<c->sm_count * 12, 32 * wpb, msmem, c->stream>>>(
+                    leaf_merge_kernel<<<c->sm_count * 8, 32 * wpb, msmem, c->stream>>>(
                         dx.as<float>(), dn.as<float>(), n, xs, d, f.perm.as<uint32_t>(), bp.base, bp.nslots,
                         ccnt.as<uint32_t>(), cap, cand.as<uint2>(), K, kd.as<float>(), ki.as<uint32_t>(),
                         ksz.as<uint32_t>(), c->err.as<uint32_t>(), ip ? kKeyIpDist : kKeyL2);
