@@ -2902,7 +2902,19 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
     auto t = Clock::now();
     ForestOut f;
     const uint32_t cap_nodes = (uint32_t)std::min<uint64_t>(16 * n / ap->leaf + 1024, 4 * n + 8);
-    rc = build_forest(c, dx.as<float>(), n, d, xs, ap->trees, ap->leaf, 100, ap->seed, cap_nodes, f, ip);
+    // the tensor-core form of the rows, for the forest's sides and the leaf tiles:
+    // query tile resident up to 256 (padded) dimensions, K-chunked up to 1024
+    const bool tensor = ap->precision == 1 && tc_padded_dim(d) != 0;
+    TcPrep tp;
+    struct Release {
+        Ctx* c;
+        TcPrep& tp;
+        ~Release() { tc_release(c, tp); }
+    } release_tp{c, tp};
+    if (tensor && (rc = tc_prep(c, dx.as<float>(), dn.as<float>(), n, xs, d, tp))) return rc;
+    const char* rows_env = std::getenv("ANQI_B200_FOREST_BF16");  // 0: sides from the FP32 rows
+    rc = build_forest(c, dx.as<float>(), n, d, xs, ap->trees, ap->leaf, 100, ap->seed, cap_nodes, f, ip,
+                      tensor && !(rows_env && rows_env[0] == '0') ? &tp : nullptr);
     const double forest_ms = ms_since(t);
     t = Clock::now();
     if (!rc) {
@@ -2917,11 +2929,8 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                     maxcnt = std::max(maxcnt, f.leaf_cnt[g]);
                 }
             }
-        // the tensor-core tiles: query tile resident up to 256 (padded)
-        // dimensions, K-chunked up to 1024
-        if (ap->precision == 1 && tc_padded_dim(d) != 0) {
+        if (tensor) {
             // BF16 tensor-core leaf tiles: candidates per tree, then the merge
-            TcPrep tp;
             // candidate buffers (n x cap entries; GBs at 1M) are kept by the
             // context: allocating them anew for every build cost up to seconds
             DevBuf& ccnt = c->init_cnt;
@@ -2931,8 +2940,7 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
             uint64_t want = (512ull << 20) / (cap * 4ull);
             if (const char* e = std::getenv("ANQI_B200_INIT_BATCH_ROWS")) want = std::strtoull(e, nullptr, 10);
             const uint64_t brows = std::min<uint64_t>(n, std::max<uint64_t>(maxcnt, want));
-            if (!(rc = tc_prep(c, dx.as<float>(), dn.as<float>(), n, xs, d, tp)) && !(rc = ensure(c, ccnt, brows * 4)) &&
-                !(rc = ensure(c, cand, brows * (size_t)cap * 8))) {
+            if (!(rc = ensure(c, ccnt, brows * 4)) && !(rc = ensure(c, cand, brows * (size_t)cap * 8))) {
                 auto cu = [&](cudaError_t e, const char* what) { return e == cudaSuccess ? ANQI_OK : cuda_check(c, e, what); };
                 rc = cu(cudaMemsetAsync(ccnt.p, 0, brows * 4, c->stream), "cudaMemsetAsync");
                 const int wpb = 4;

@@ -15,6 +15,8 @@
 // its hyperplane; 4-thread groups compute point margins over fixed-size chunks
 // of the segments; a stable partition per chunk places points using per-chunk
 // prefix counts.  The host only keeps the small per-node records.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 #include <cfloat>
 
@@ -44,7 +46,7 @@ __global__ void forest_hyperplane_kernel(const float* __restrict__ x, uint32_t s
                                          const uint32_t* __restrict__ perm, const SplitNode* __restrict__ nodes,
                                          uint32_t n_split, uint64_t seed, uint32_t cap_nodes,
                                          float* __restrict__ hyper, float* __restrict__ mid,
-                                         float* __restrict__ offset, int angular) {
+                                         float* __restrict__ offset, float* __restrict__ hnorm, int angular) {
     const uint32_t lane = threadIdx.x & 31u, gt = lane & 3u;
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w >= n_split) return;
@@ -70,7 +72,12 @@ __global__ void forest_hyperplane_kernel(const float* __restrict__ x, uint32_t s
         if (fabsf(hn) < kSplitEps) hn = 1.0f;
         __syncwarp();
         for (uint32_t j = lane; j < dim; j += 32) hp[j] = __fdiv_rn(hp[j], hn);
-        if (lane == 0) offset[w] = 0.0f;
+        __syncwarp();
+        const float h2 = group_ip(hp, hp, dim, gt, kAll);
+        if (lane == 0) {
+            offset[w] = 0.0f;
+            hnorm[w] = __fsqrt_ru(h2) * 1.001f;
+        }
         return;
     }
     for (uint32_t j = lane; j < stride; j += 32) {
@@ -80,7 +87,11 @@ __global__ void forest_hyperplane_kernel(const float* __restrict__ x, uint32_t s
     }
     __syncwarp();
     const float off = group_ip(hp, md, dim, gt, kAll);
-    if (lane == 0) offset[w] = off;
+    const float h2 = group_ip(hp, hp, dim, gt, kAll);
+    if (lane == 0) {
+        offset[w] = off;
+        hnorm[w] = __fsqrt_ru(h2) * 1.001f;  // a bound: FP32 sums of up to 1,024 squares
+    }
 }
 
 // Sides for every point of every chunk; counts lefts per chunk.
@@ -122,6 +133,94 @@ __global__ void forest_sides_kernel(const float* __restrict__ x, uint32_t stride
             sd[p] = s;
             lefts += (s == 0);
         }
+    }
+    for (int o = 16; o > 0; o >>= 1) lefts += __shfl_xor_sync(kAll, lefts, o);
+    if (lane == 0) atomicAdd(&s_cnt, lefts);
+    __syncthreads();
+    if (threadIdx.x == 0) chunk_left[blockIdx.x] = s_cnt;
+}
+
+// The same sides from the rows' bf16 copies (dp wide, zero-padded), half the
+// bytes: the margin differs from the reference's by at most the row's rounding
+// error along the hyperplane and the two sums' own, bounded for all rows by
+// |h| (err_max + 8 dp 2^-24 (norm_max + err_max)), so a margin past that and
+// kSplitEps has the reference's sign; the others (NaN and overflow among them)
+// take the reference's arithmetic on the FP32 row.  A warp most of whose first
+// rows do so (rows of very different lengths) takes it for the rest at once.
+// Every level reads every row of every tree, so it is bound by those bytes:
+// 64 trees over 1M x 128, 72.5 ms from the FP32 rows and 32.7 from these; over
+// 100,000 x 100 (ip; all of it in L2), 2.9 and 2.7; over 5,003 x 37, 0.126 and 0.096.
+__global__ void __launch_bounds__(256) forest_sides_bf16_kernel(
+    const __nv_bfloat16* __restrict__ xb, uint32_t dp, float norm_max, float err_max, const float* __restrict__ x,
+    uint32_t stride, uint32_t dim, uint64_t n, const uint32_t* __restrict__ perm, const SplitNode* __restrict__ nodes,
+    const Chunk* __restrict__ chunks, uint64_t seed, uint32_t cap_nodes, const float* __restrict__ hyper,
+    const float* __restrict__ offset, const float* __restrict__ hnorm, uint8_t* __restrict__ side,
+    uint32_t* __restrict__ chunk_left) {
+    extern __shared__ __align__(16) float s_hp[];
+    __shared__ uint32_t s_cnt;
+    const Chunk ch = chunks[blockIdx.x];
+    const SplitNode nd = nodes[ch.node];
+    const uint64_t key = node_key(seed, nd.tree, nd.local);
+    const uint32_t* pt = perm + (uint64_t)nd.tree * n + nd.start;
+    uint8_t* sd = side + (uint64_t)nd.tree * n + nd.start;
+    const float* hp = hyper + ((uint64_t)nd.tree * cap_nodes + nd.local) * stride;
+    const float off = offset[ch.node];
+    const float g = 4.0f * dp * 5.9604645e-8f;
+    const float bound = hnorm[ch.node] * (err_max + 2.0f * g * (norm_max + err_max)) * 1.001f + 1.001f * kSplitEps;
+    for (uint32_t k = threadIdx.x; k < dp; k += blockDim.x) s_hp[k] = k < dim ? hp[k] : 0.f;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, gt = lane & 3u;
+    const uint32_t group = threadIdx.x >> 2, ngroups = blockDim.x >> 2;
+    const uint32_t units = dp / 8, end = ch.begin + ch.len;
+    uint32_t lefts = 0, redone = 0;
+    const uint32_t iters = (ch.len + ngroups - 1) / ngroups;
+    uint32_t p = ch.begin + group;
+    uint32_t id = pt[min(p, end - 1)];
+    bool direct = false;
+    for (uint32_t it = 0; it < iters; it++, p += ngroups) {
+        const bool ok = p < end;
+        const uint32_t id_next = pt[min(p + ngroups, end - 1)];
+        float m = __int_as_float(0x7fc00000);
+        if (!direct) {
+            const uint4* row = reinterpret_cast<const uint4*>(xb + (uint64_t)id * dp);
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll 4
+            for (uint32_t c = gt; c < units; c += 4) {
+                const uint4 v = row[c];
+                const float4 h0 = *reinterpret_cast<const float4*>(s_hp + 8 * c);
+                const float4 h1 = *reinterpret_cast<const float4*>(s_hp + 8 * c + 4);
+                a0 = fmaf(h0.x, __uint_as_float(v.x << 16), a0);
+                a1 = fmaf(h0.y, __uint_as_float(v.x & 0xFFFF0000u), a1);
+                a0 = fmaf(h0.z, __uint_as_float(v.y << 16), a0);
+                a1 = fmaf(h0.w, __uint_as_float(v.y & 0xFFFF0000u), a1);
+                a0 = fmaf(h1.x, __uint_as_float(v.z << 16), a0);
+                a1 = fmaf(h1.y, __uint_as_float(v.z & 0xFFFF0000u), a1);
+                a0 = fmaf(h1.z, __uint_as_float(v.w << 16), a0);
+                a1 = fmaf(h1.w, __uint_as_float(v.w & 0xFFFF0000u), a1);
+            }
+            a0 += a1;
+            a0 += __shfl_xor_sync(kAll, a0, 1);
+            a0 += __shfl_xor_sync(kAll, a0, 2);
+            m = a0 - off;
+        }
+        const bool redo = !(fabsf(m) * 0.999999f > bound);
+        if (__any_sync(kAll, redo)) {
+            // the groups of the warp step together; those that need no row take hp's
+            const float ip = group_ip(hp, redo ? x + (uint64_t)id * stride : hp, dim, gt, kAll);
+            if (redo) m = __fsub_rn(ip, off);
+            redone += __popc(__ballot_sync(kAll, redo));
+            if (it == 3) direct = redone > 64;  // of 4 x 32 lanes
+        }
+        uint8_t s;
+        if (m < -kSplitEps) s = 0;
+        else if (m > kSplitEps) s = 1;
+        else s = (uint8_t)(hash64(key ^ (((uint64_t)id << 2) | 3)) & 1);
+        if (ok && gt == 0) {
+            sd[p] = s;
+            lefts += (s == 0);
+        }
+        id = id_next;
     }
     for (int o = 16; o > 0; o >>= 1) lefts += __shfl_xor_sync(kAll, lefts, o);
     if (lane == 0) atomicAdd(&s_cnt, lefts);
@@ -187,7 +286,8 @@ __global__ void iota_trees_kernel(uint32_t* perm, uint64_t n, uint32_t trees) {
 }
 
 int build_forest(Ctx* c, const float* d_x, uint64_t n, uint32_t dim, uint32_t stride, uint32_t trees,
-                 uint32_t leaf, uint32_t max_depth, uint64_t seed, uint32_t cap_nodes, ForestOut& out, int angular) {
+                 uint32_t leaf, uint32_t max_depth, uint64_t seed, uint32_t cap_nodes, ForestOut& out, int angular,
+                 const TcPrep* rows) {
     if (n == 0 || trees == 0 || leaf == 0 || cap_nodes < 1) return fail(c, ANQI_ERR_ARGS, "invalid forest arguments");
     if (n >= 0xFFFFFFFFull) return fail(c, ANQI_ERR_ARGS, "forest needs n < 2^32");
     out.trees = trees;
@@ -205,7 +305,7 @@ int build_forest(Ctx* c, const float* d_x, uint64_t n, uint32_t dim, uint32_t st
     int rc;
     if ((rc = ensure(c, out.perm, (size_t)trees * n * 4)) || (rc = ensure(c, out.hyper, tot_nodes * stride * 4)))
         return rc;
-    TmpBuf tmp(c), side(c), dnodes(c), dchunks(c), dmid(c), doff(c), dleft(c), dpre(c), dnl(c);
+    TmpBuf tmp(c), side(c), dnodes(c), dchunks(c), dmid(c), doff(c), dhn(c), dleft(c), dpre(c), dnl(c);
     if ((rc = ensure(c, tmp, (size_t)trees * n * 4)) || (rc = ensure(c, side, (size_t)trees * n)))
         return rc;
     iota_trees_kernel<<<c->sm_count * 8, 256, 0, c->stream>>>(out.perm.as<uint32_t>(), n, trees);
@@ -242,16 +342,22 @@ int build_forest(Ctx* c, const float* d_x, uint64_t n, uint32_t dim, uint32_t st
         const uint32_t nc = (uint32_t)chunks.size();
         if ((rc = h2d(c, dnodes, split.data(), ns * sizeof(SplitNode))) ||
             (rc = h2d(c, dchunks, chunks.data(), nc * sizeof(Chunk))) ||
-            (rc = ensure(c, dmid, (size_t)ns * stride * 4)) || (rc = ensure(c, doff, ns * 4)) ||
+            (rc = ensure(c, dmid, (size_t)ns * stride * 4)) || (rc = ensure(c, doff, ns * 4)) || (rc = ensure(c, dhn, ns * 4)) ||
             (rc = ensure(c, dleft, nc * 4)) || (rc = ensure(c, dpre, nc * 4)) || (rc = ensure(c, dnl, ns * 4)))
             return rc;
         forest_hyperplane_kernel<<<(ns + 3) / 4, 128, 0, c->stream>>>(
             d_x, stride, dim, n, out.perm.as<uint32_t>(), dnodes.as<SplitNode>(), ns, seed, cap_nodes,
-            out.hyper.as<float>(), dmid.as<float>(), doff.as<float>(), angular);
-        forest_sides_kernel<<<nc, 256, 0, c->stream>>>(d_x, stride, dim, n, out.perm.as<uint32_t>(),
-                                                       dnodes.as<SplitNode>(), dchunks.as<Chunk>(), seed, cap_nodes,
-                                                       out.hyper.as<float>(), doff.as<float>(), side.as<uint8_t>(),
-                                                       dleft.as<uint32_t>(), 0);
+            out.hyper.as<float>(), dmid.as<float>(), doff.as<float>(), dhn.as<float>(), angular);
+        if (rows)
+            forest_sides_bf16_kernel<<<nc, 256, rows->dp * 4, c->stream>>>(
+                rows->bf.as<__nv_bfloat16>(), rows->dp, rows->bnorm, rows->berr, d_x, stride, dim, n,
+                out.perm.as<uint32_t>(), dnodes.as<SplitNode>(), dchunks.as<Chunk>(), seed, cap_nodes,
+                out.hyper.as<float>(), doff.as<float>(), dhn.as<float>(), side.as<uint8_t>(), dleft.as<uint32_t>());
+        else
+            forest_sides_kernel<<<nc, 256, 0, c->stream>>>(d_x, stride, dim, n, out.perm.as<uint32_t>(),
+                                                           dnodes.as<SplitNode>(), dchunks.as<Chunk>(), seed, cap_nodes,
+                                                           out.hyper.as<float>(), doff.as<float>(), side.as<uint8_t>(),
+                                                           dleft.as<uint32_t>(), 0);
         ANQI_CUDA(c, cudaGetLastError());
         std::vector<uint32_t> cl(nc);
         std::vector<float> offs(ns);

@@ -234,8 +234,11 @@ struct ForestOut {
     DevBuf perm, hyper;  // device; released by the caller
     ForestOut() { perm.pooled = hyper.pooled = true; }
 };
+// rows: the rows' tensor-core form, if it is there, which halves the bytes of a level.
+struct TcPrep;
 int build_forest(Ctx* c, const float* d_x, uint64_t n, uint32_t dim, uint32_t stride, uint32_t trees, uint32_t leaf,
-                 uint32_t max_depth, uint64_t seed, uint32_t cap_nodes, ForestOut& out, int angular = 0);
+                 uint32_t max_depth, uint64_t seed, uint32_t cap_nodes, ForestOut& out, int angular = 0,
+                 const TcPrep* rows = nullptr);
 // Exclusive scan of n u32 counts into n + 1 u64 offsets (device).
 int device_scan(Ctx* c, const uint32_t* d_in, uint64_t* d_out, uint64_t n);
 
