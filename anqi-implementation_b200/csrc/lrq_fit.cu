@@ -27,7 +27,6 @@ namespace {
 constexpr uint32_t kFitMaxCols = 128;  // nk
 constexpr uint32_t kFitMaxRank = 16;   // rank M
 constexpr uint32_t kStatRows = 1024;   // rows per block of the partial sums
-constexpr uint32_t kSortChunk = 2048;  // elements sorted per block in shared memory
 
 __device__ __forceinline__ double row_value(const float* keys, const uint32_t* ids, uint64_t i, uint32_t nk, uint32_t k) {
     const uint64_t r = ids ? (uint64_t)ids[i] : i;
@@ -211,59 +210,106 @@ __global__ void fit_lohi_init_kernel(double* lohi, uint32_t nk) {
 }
 
 // ---------------------------------------------------------------- sort
+// Every column ascending, by eight stable passes over 8-bit digits: a pass counts
+// each tile's digits, sums the counts over the column (digit by digit, tile by
+// tile) and moves each key to its place.  Sixteen passes over memory in all, where
+// a bitonic network over columns padded to a power of two makes over a hundred, as
+// many as fit in shared memory at once: 100 columns of 120,000, SORT_FIG.
+// Bound by the moves' scattered 8-byte writes and the lanes' digit matching.
+constexpr uint32_t kSortTile = 4096, kSortPer = 16;  // keys a tile of 8 warps; a thread's share
 
-// Copies column k of res (m values) into a padded row of n2 (+inf beyond m).
-__global__ void fit_pad_kernel(const double* __restrict__ res, uint64_t m, uint32_t nk, uint64_t n2,
-                               double* __restrict__ a) {
-    const uint64_t total = (uint64_t)nk * n2;
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = t / n2, i = t % n2;
-        a[t] = i < m ? res[k * m + i] : __longlong_as_double(0x7ff0000000000000ll);
-    }
+// The digit at `shift` of a key's rank among doubles (sign folded in).
+__device__ __forceinline__ uint32_t sort_digit(double v, uint32_t shift) {
+    const uint64_t b = (uint64_t)__double_as_longlong(v);
+    const uint64_t r = b ^ ((b >> 63) ? ~0ull : 0x8000000000000000ull);
+    return (uint32_t)(r >> shift) & 255u;
 }
 
-// Bitonic stages (kk, j) with j >= kSortChunk: one compare-exchange per thread.
-__global__ void fit_bitonic_global_kernel(double* __restrict__ a, uint64_t total, uint64_t n2, uint64_t kk,
-                                          uint64_t j) {
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total / 2;
-         t += (uint64_t)gridDim.x * blockDim.x) {
-        // the t-th pair: i has bit j clear
-        const uint64_t i = (t / j) * 2 * j + (t % j);
-        const uint64_t p = i + j;
-        const uint64_t pos = i % n2;  // position within the column
-        const bool up = (pos & kk) == 0;
-        const double x = a[i], y = a[p];
-        if ((x > y) == up) {
-            a[i] = y;
-            a[p] = x;
-        }
-    }
-}
-
-// Bitonic stages j < kSortChunk for every kk in [kk_lo, kk_hi] inside chunks
-// of kSortChunk elements held in shared memory.
-__global__ void __launch_bounds__(1024) fit_bitonic_shared_kernel(double* __restrict__ a, uint64_t n2, uint64_t kk_lo,
-                                                                  uint64_t kk_hi) {
-    __shared__ double s[kSortChunk];
-    const uint64_t base = (uint64_t)blockIdx.x * kSortChunk;
-    for (uint32_t t = threadIdx.x; t < kSortChunk; t += blockDim.x) s[t] = a[base + t];
+// The tile's keys of this warp (512 in a row, 32 at a time) and their digits,
+// counted per warp in cnt[warp]; past the column's end the digit is 256.
+__device__ __forceinline__ void sort_load(const double* __restrict__ src, uint64_t m, uint32_t shift,
+                                          double (&v)[kSortPer], uint32_t (*cnt)[256]) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t t = threadIdx.x; t < 8 * 256; t += blockDim.x) (&cnt[0][0])[t] = 0;
+    const uint64_t at = (uint64_t)blockIdx.x * kSortTile + warp * 512 + lane;
+#pragma unroll
+    for (uint32_t q = 0; q < kSortPer; q++) v[q] = at + 32 * q < m ? src[at + 32 * q] : 0.0;
     __syncthreads();
-    for (uint64_t kk = kk_lo; kk <= kk_hi; kk <<= 1) {
-        for (uint64_t j = (kk >> 1) < (kSortChunk >> 1) ? (kk >> 1) : (kSortChunk >> 1); j > 0; j >>= 1) {
-            for (uint32_t t = threadIdx.x; t < kSortChunk / 2; t += blockDim.x) {
-                const uint32_t i = (uint32_t)((t / j) * 2 * j + (t % j));
-                const uint32_t p = i + (uint32_t)j;
-                const bool up = (((base + i) % n2) & kk) == 0;
-                const double x = s[i], y = s[p];
-                if ((x > y) == up) {
-                    s[i] = y;
-                    s[p] = x;
-                }
-            }
-            __syncthreads();
-        }
+#pragma unroll
+    for (uint32_t q = 0; q < kSortPer; q++) {
+        const uint32_t d = at + 32 * q < m ? sort_digit(v[q], shift) : 256u;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+        if (d < 256 && lane == __ffs(peers) - 1u) cnt[warp][d] += __popc(peers);
+        __syncwarp();
     }
-    for (uint32_t t = threadIdx.x; t < kSortChunk; t += blockDim.x) a[base + t] = s[t];
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) fit_sort_count_kernel(const double* __restrict__ src, uint64_t m, uint32_t shift,
+                                                             uint64_t* __restrict__ counts) {
+    __shared__ uint32_t cnt[8][256];
+    double v[kSortPer];
+    sort_load(src + blockIdx.y * m, m, shift, v, cnt);
+    uint32_t sum = 0;
+    for (uint32_t w = 0; w < 8; w++) sum += cnt[w][threadIdx.x];
+    counts[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x] = sum;
+}
+
+// A column's counts -> the first place of each tile's digit.
+__global__ void __launch_bounds__(256) fit_sort_scan_kernel(uint64_t* __restrict__ counts, uint64_t tiles) {
+    __shared__ uint64_t s[256];
+    uint64_t* c = counts + blockIdx.x * tiles * 256 + threadIdx.x;
+    uint64_t sum = 0;
+    for (uint64_t t = 0; t < tiles; t++) sum += c[t * 256];
+    s[threadIdx.x] = sum;
+    __syncthreads();
+    for (uint32_t o = 1; o < 256; o <<= 1) {
+        const uint64_t add = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
+        __syncthreads();
+        s[threadIdx.x] += add;
+        __syncthreads();
+    }
+    uint64_t run = s[threadIdx.x] - sum;
+    for (uint64_t t = 0; t < tiles; t++) {
+        const uint64_t here = c[t * 256];
+        c[t * 256] = run;
+        run += here;
+    }
+}
+
+__global__ void __launch_bounds__(256) fit_sort_move_kernel(const double* __restrict__ src, uint64_t m, uint32_t shift,
+                                                            const uint64_t* __restrict__ counts,
+                                                            double* __restrict__ dst) {
+    __shared__ uint32_t cnt[8][256];
+    __shared__ uint64_t first[256];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    double v[kSortPer];
+    first[threadIdx.x] = counts[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x];
+    sort_load(src + blockIdx.y * m, m, shift, v, cnt);
+    // each warp's start within the tile's digit
+    uint32_t run = 0;
+    for (uint32_t w = 0; w < 8; w++) {
+        const uint32_t here = cnt[w][threadIdx.x];
+        cnt[w][threadIdx.x] = run;
+        run += here;
+    }
+    __syncthreads();
+    double* out = dst + blockIdx.y * m;
+    const uint64_t at = (uint64_t)blockIdx.x * kSortTile + warp * 512 + lane;
+#pragma unroll
+    for (uint32_t q = 0; q < kSortPer; q++) {
+        const uint32_t d = at + 32 * q < m ? sort_digit(v[q], shift) : 256u;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+        uint32_t start = 0;
+        if (d < 256) start = cnt[warp][d];
+        __syncwarp();
+        if (d < 256) {
+            if (rank == 0) cnt[warp][d] = start + __popc(peers);
+            out[first[d] + start + rank] = v[q];
+        }
+        __syncwarp();
+    }
 }
 
 // prefix[k][0] = 0, prefix[k][i+1] = prefix[k][i] + s[k][i], in index order
@@ -478,9 +524,7 @@ int anqi_lrq_fit_range(const float* keys, uint64_t n, uint32_t nk, const double*
 }
 
 uint64_t anqi_lrq_fit_codebooks_scratch(uint64_t m, uint32_t nk) {
-    uint64_t n2 = kSortChunk;
-    while (n2 < m) n2 <<= 1;
-    return (uint64_t)nk * n2 + (uint64_t)nk * (m + 1);
+    return (uint64_t)nk * m + (uint64_t)nk * (m + 1) + (uint64_t)nk * ((m + kSortTile - 1) / kSortTile) * 256;
 }
 
 int anqi_lrq_fit_codebooks(const double* res, uint64_t m, uint32_t nk, uint32_t cs, uint32_t iters, double* scratch,
@@ -488,23 +532,21 @@ int anqi_lrq_fit_codebooks(const double* res, uint64_t m, uint32_t nk, uint32_t 
     if (!res || !scratch || !codebooks || m < 2 || nk == 0 || nk > kFitMaxCols || cs < 2 || cs > 256)
         return ANQI_ERR_ARGS;
     if (scratch_doubles < anqi_lrq_fit_codebooks_scratch(m, nk)) return ANQI_ERR_CAPACITY;
-    uint64_t n2 = kSortChunk;
-    while (n2 < m) n2 <<= 1;
+    const uint64_t tiles = (m + kSortTile - 1) / kSortTile;
     double* a = scratch;
-    double* prefix = scratch + (uint64_t)nk * n2;
-    const uint64_t total = (uint64_t)nk * n2;
+    double* prefix = scratch + (uint64_t)nk * m;
+    uint64_t* counts = reinterpret_cast<uint64_t*>(prefix + (uint64_t)nk * (m + 1));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    fit_pad_kernel<<<grid_for(total, 256), 256, 0, st>>>(res, m, nk, n2, a);
-    const uint32_t chunks = (uint32_t)(total / kSortChunk);
-    // every chunk sorted up to size kSortChunk, then the larger merges
-    fit_bitonic_shared_kernel<<<chunks, 1024, 0, st>>>(a, n2, 2, kSortChunk);
-    for (uint64_t kk = 2 * kSortChunk; kk <= n2; kk <<= 1) {
-        for (uint64_t j = kk >> 1; j >= kSortChunk; j >>= 1)
-            fit_bitonic_global_kernel<<<grid_for(total / 2, 256), 256, 0, st>>>(a, total, n2, kk, j);
-        fit_bitonic_shared_kernel<<<chunks, 1024, 0, st>>>(a, n2, kk, kk);
+    const dim3 grid((unsigned)tiles, nk);
+    for (uint32_t pass = 0; pass < 8; pass++) {
+        // between the prefix sums' room and a, which the last pass fills
+        const double* src = pass == 0 ? res : pass & 1u ? prefix : a;
+        fit_sort_count_kernel<<<grid, 256, 0, st>>>(src, m, 8 * pass, counts);
+        fit_sort_scan_kernel<<<nk, 256, 0, st>>>(counts, tiles);
+        fit_sort_move_kernel<<<grid, 256, 0, st>>>(src, m, 8 * pass, counts, pass & 1u ? a : prefix);
     }
-    fit_prefix_kernel<<<nk, 128, 0, st>>>(a, m, n2, prefix);
-    fit_lloyd_kernel<<<nk, 256, 0, st>>>(a, m, n2, prefix, cs, iters, codebooks);
+    fit_prefix_kernel<<<nk, 128, 0, st>>>(a, m, m, prefix);
+    fit_lloyd_kernel<<<nk, 256, 0, st>>>(a, m, m, prefix, cs, iters, codebooks);
     return cudaGetLastError() == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
 }
 
