@@ -1155,6 +1155,29 @@ __global__ void fill_reverse_kernel(const uint32_t* __restrict__ ids, uint64_t n
     }
 }
 
+// out[0]: the longest list of a CSR (zeroed before); its total stays at off[n].
+__global__ void max_list_kernel(const uint64_t* __restrict__ off, uint64_t n, unsigned long long* __restrict__ out) {
+    unsigned long long m = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        m = max(m, (unsigned long long)(off[i + 1] - off[i]));
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(kAll, m, o));
+    if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
+}
+
+// The longest list of a CSR and its total, found on the device: bringing the
+// offsets over and walking them took 5.8 ms at 1M rows and 0.8 ms at 200,000.
+static int list_bounds(Ctx* c, const DevBuf& off, uint64_t n, uint64_t* longest, uint64_t* total) {
+    TmpBuf m(c);
+    int rc;
+    if ((rc = ensure(c, m, 8))) return rc;
+    ANQI_CUDA(c, cudaMemsetAsync(m.p, 0, 8, c->stream));
+    max_list_kernel<<<c->sm_count * 8, 256, 0, c->stream>>>(off.as<uint64_t>(), n, m.as<unsigned long long>());
+    ANQI_CUDA(c, cudaGetLastError());
+    if ((rc = d2h(c, longest, m, 8))) return rc;
+    ANQI_CUDA(c, cudaMemcpyAsync(total, off.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, c->stream));
+    return sync(c);
+}
+
 // ------------------------------------------------------------ locality numbering
 // The AKNN gather's visited tests and row reads stay local when rows that
 // visit one another carry nearby numbers.  Rows are numbered component by
@@ -1728,14 +1751,6 @@ static int locality_order(Ctx* c, const uint32_t* d_ids, uint64_t n, uint32_t K,
     return ANQI_OK;
 }
 
-static uint64_t max_reverse(Ctx* c, const DevBuf& off, uint64_t n) {
-    std::vector<uint64_t> h(n + 1);
-    cudaMemcpy(h.data(), off.p, (n + 1) * 8, cudaMemcpyDeviceToHost);
-    uint64_t m = 0;
-    for (uint64_t i = 0; i < n; i++) m = std::max(m, h[i + 1] - h[i]);
-    return m;
-}
-
 // Runs gather_kernel over all rows.
 static int run_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_total, double* kernel_ms = nullptr) {
     const int warps_per_block = 4;
@@ -1947,11 +1962,8 @@ static int run_localjoin(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n,
                                            hval.as<float>(), K, mask.as<uint32_t>())))
             return rc;
         if ((rc = device_scan(c, incnt.as<uint32_t>(), off.as<uint64_t>(), n))) return rc;
-        std::vector<uint64_t> hoff(n + 1);
-        ANQI_CUDA(c, cudaMemcpy(hoff.data(), off.p, (n + 1) * 8, cudaMemcpyDeviceToHost));
-        uint64_t maxin = 0;
-        for (uint64_t i = 0; i < n; i++) maxin = std::max(maxin, hoff[i + 1] - hoff[i]);
-        if ((rc = ensure(c, inc, hoff[n] * 8 + 8))) return rc;
+        uint64_t maxin = 0, incoming = 0;
+        if ((rc = list_bounds(c, off, n, &maxin, &incoming)) || (rc = ensure(c, inc, incoming * 8 + 8))) return rc;
         join_fill_kernel<<<blocks, 256, 0, c->stream>>>(samp.as<uint32_t>(), scnt.as<uint32_t>(), n, S,
                                                        off.as<uint64_t>(), fill.as<uint32_t>(), inc.as<uint64_t>());
         ANQI_CUDA(c, cudaGetLastError());
@@ -2059,7 +2071,8 @@ static int run_select_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_
         }
     }
     if ((rc = build_reverse(c, hid.as<uint32_t>(), n, K, roff, rev))) return rc;
-    const uint64_t mr = max_reverse(c, roff, n);
+    uint64_t mr = 0, rev_total = 0;
+    if ((rc = list_bounds(c, roff, n, &mr, &rev_total))) return rc;
     if ((rc = ensure(c, O, n * M * 4)) || (rc = ensure(c, Odeg, n * 4))) return rc;
     GatherParams p = base_params(dx, dn, n, stride, dim);
     p.g_ids = hid.as<uint32_t>();
@@ -2090,7 +2103,8 @@ static int run_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n, ui
     DevBuf* deg = &deg_buf;
     TmpBuf roff2(c), rev2(c);
     if ((rc = build_reverse(c, O.as<uint32_t>(), n, M, roff2, rev2))) return rc;
-    const uint64_t mr2 = max_reverse(c, roff2, n);
+    uint64_t mr2 = 0, rev_total = 0;
+    if ((rc = list_bounds(c, roff2, n, &mr2, &rev_total))) return rc;
     if ((rc = ensure(c, *links, n * M * 4)) || (rc = ensure(c, *deg, n * 4))) return rc;
     GatherParams q = base_params(dx, dn, n, stride, dim);
     q.mode = kModeCommit;
@@ -2535,7 +2549,8 @@ int anqi_graph_commit_policy(anqi_ctx* h, const float* x, uint64_t n, uint32_t d
     q.rev_ids = rev.as<uint32_t>();
     q.links = dl.as<uint32_t>();
     q.deg = dd.as<uint32_t>();
-    if ((rc = run_gather(c, q, max_reverse(c, roff, n), nullptr))) return rc;
+    uint64_t longest = 0, rev_total = 0;
+    if ((rc = list_bounds(c, roff, n, &longest, &rev_total)) || (rc = run_gather(c, q, longest, nullptr))) return rc;
     if ((rc = d2h(c, links, dl, n * M * 4)) || (rc = d2h(c, deg, dd, n * 4))) return rc;
     return sync(c);
 }
@@ -2878,7 +2893,8 @@ int anqi_aknn_gather_metric(anqi_ctx* h, const float* x, uint64_t n, uint32_t di
     p.out_k = out_k;
     p.out_ids = oi.as<uint32_t>();
     p.out_d = od.as<float>();
-    if ((rc = run_gather(c, p, max_reverse(c, roff, n), nullptr))) return rc;
+    uint64_t longest = 0, rev_total = 0;
+    if ((rc = list_bounds(c, roff, n, &longest, &rev_total)) || (rc = run_gather(c, p, longest, nullptr))) return rc;
     if ((rc = d2h(c, ids, oi, n * out_k * 4)) || (rc = d2h(c, dists, od, n * out_k * 4))) return rc;
     return sync(c);
 }
@@ -3129,7 +3145,10 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
     }
     if (rest) {
         uint64_t pooled = 0;
-        if ((rc = run_aknn_gather(c, p, max_reverse(c, roff, n), &pooled, &gather_kernel_ms))) return rc;
+        uint64_t longest = 0, rev_total = 0;
+        if ((rc = list_bounds(c, roff, n, &longest, &rev_total)) ||
+            (rc = run_aknn_gather(c, p, longest, &pooled, &gather_kernel_ms)))
+            return rc;
         pool_total += pooled;
     }
     const double gather_ms = ms_since(t);
