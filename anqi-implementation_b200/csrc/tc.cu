@@ -2,12 +2,12 @@
 // exact ground truth (tools/dataset_gt.cpp:206-313) in the precision form.
 //
 // Rows are converted once to bf16 (padded to a multiple of 16).  Whole-matrix
-// work runs in tc_scan_kernel; init_knn's leaves in tc_filter_kernel, where a CTA
-// of 8 warps owns 128 rows of a leaf resident in shared memory and streams the
-// leaf's rows through a two-stage ring, one thread issuing the K = 16
-// tcgen05.mma steps into one of two 128-column TMEM accumulators while all run
-// the epilogue of the previous tile (tcgen05.ld: thread = row, 32 columns per
-// load).
+// work runs in tc_scan_kernel and init_knn's leaves in tc_leaf_kernel; leaves or
+// rows too long for it in tc_filter_kernel, where a CTA of 8 warps owns 128 rows
+// of a leaf resident in shared memory and streams the leaf's rows through a
+// two-stage ring, one thread issuing the K = 16 tcgen05.mma steps into one of two
+// 128-column TMEM accumulators while all run the epilogue of the previous tile
+// (tcgen05.ld: thread = row, 32 columns per load).
 //
 // Epilogue: key~ = |q|^2 + |x|^2 - 2 <q~, x~> with the reference's FP32
 // norms.  A pair is a candidate when key~ - eps <= threshold, where eps bounds
