@@ -533,9 +533,10 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
 // full, take one slot reservation per 32 pairs and one 8-byte store each, without
 // a loop over set bits (whose length is the warp's longest).
 // Bound by issue and, with one CTA to an SM, by the time its rows take to come in.
-// 64 trees over 1M x 128 (integers): 44.2 ms, the 128-row-tile form 81.6 ms; over
-// 5,003 x 37: 0.93 and 1.69 ms; over 100,000 x 100 (ip, no exact rows): 5.9 and
-// 6.4 ms.
+// 64 trees over 1M x 128 (integers): 40.8 ms (44.2 before the exact form was an
+// instance of its own and ip rows' norms zeros), the 128-row-tile form 81.6 ms;
+// over 5,003 x 37: 0.92 and 1.69 ms; over 100,000 x 100 (ip, no exact rows): 5.9
+// and 6.4 ms.
 constexpr uint32_t kLeafWarps = 16;
 constexpr uint32_t kLeafThreads = 32 * (kLeafWarps + 1);
 constexpr uint32_t kLeafTiles = 4;
@@ -545,6 +546,8 @@ __host__ __device__ constexpr size_t leaf_smem(uint32_t dp, uint32_t tiles) {
     return (size_t)tiles * kTile * dp * 2 + 6 * (size_t)kLeafRows * 4;
 }
 
+// kPlain: every row exact and d <= 128, so no bound and no recheck.
+template <bool kPlain>
 __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p, uint32_t tiles) {
     extern __shared__ __align__(128) unsigned char sm[];
     const size_t tile_bytes = (size_t)kTile * p.dp * 2;
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
         const bool ok = t < cnt;
         const uint32_t j = ok ? mem[t] : 0u;
         mid[t] = j;
-        mn[t] = ok ? p.xn[j] : 0.f;
+        mn[t] = ok && p.key_mode == 0 ? p.xn[j] : 0.f;  // ip keys hold no norm
         mnorm[t] = ok ? p.xnorm[j] : 0.f;
         merr[t] = ok ? p.xerr[j] : 0.f;
         float thr = __int_as_float(0x7f800000);
@@ -647,7 +650,6 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
         }
         const uint32_t quarter = warp & 3u, cg = warp >> 2;
         const bool l2k = p.key_mode == 0;
-        const bool plain = p.all_exact && p.d <= 128;  // every key exact: no bound, no recheck
         const float u = 5.9604645e-8f;  // 2^-24
         const float g = 2.0f * p.dp * u;
         const float kh = l2k ? 1.f : 0.5f;
@@ -680,7 +682,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
                 if (lane == 0) tc::mbar_arrive(&accempty[b]);
                 if (!rows_any || c0 >= cnt) continue;
                 uint32_t keep = 0, flag = 0;  // bit k: column c0 + k
-                if (plain) {
+                if constexpr (kPlain) {
                     // key <= thr as the sign of (thr - qn) - xn + 2 acc, exact here
 #pragma unroll
                     for (uint32_t k = 0; k < 32; k += 4) {
@@ -688,7 +690,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
                         const float xa[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
                         for (uint32_t e = 0; e < 4; e++)
-                            keep = __funnelshift_r(keep, __float_as_uint(fmaf(f, v[k + e], l2k ? R - xa[e] : R)) >> 31, 1);
+                            keep = __funnelshift_r(keep, __float_as_uint(fmaf(f, v[k + e], R - xa[e])) >> 31, 1);
                     }
                     keep = ~keep;
                 } else {
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
                         const float ea[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
                         for (uint32_t e = 0; e < 4; e++) {
-                            const float approx = fmaf(-f, v[k + e], l2k ? __fadd_rn(qn, xa[e]) : 1.f);
+                            const float approx = fmaf(-f, v[k + e], __fadd_rn(qn, xa[e]));
                             float eps = fmaf(ca, na[e], fmaf(cb, ea[e], fmaf(cc, xa[e], cd)));
                             if ((cint >> (k + e)) & 1u) eps = 0.f;
                             if (approx - eps <= thr) keep |= 1u << (k + e);
@@ -726,8 +728,9 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
 #pragma unroll
                     for (uint32_t e = 0; e < 4; e++) {
                         if (keep & (1u << (k + e))) {
-                            const float approx = fmaf(-f, v[k + e], l2k ? __fadd_rn(qn, xa[e]) : 1.f);
-                            *o++ = make_uint2(ia[e] | ((flag >> (k + e)) & 1u ? kRecheck : 0u), __float_as_uint(approx));
+                            const float approx = fmaf(-f, v[k + e], __fadd_rn(qn, xa[e]));
+                            const uint32_t id = kPlain ? ia[e] : ia[e] | ((flag >> (k + e)) & 1u ? kRecheck : 0u);
+                            *o++ = make_uint2(id, __float_as_uint(approx));
                         }
                     }
                 }
@@ -1598,10 +1601,11 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     if (leaf_whole(p.dp, maxcnt)) {
         const uint32_t tiles = (maxcnt + kTile - 1) / kTile;
         const size_t bytes = leaf_smem(p.dp, tiles);
-        ANQI_CUDA(c, cudaFuncSetAttribute(tc_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        auto leaf = p.all_exact && p.d <= 128 ? tc_leaf_kernel<true> : tc_leaf_kernel<false>;
+        ANQI_CUDA(c, cudaFuncSetAttribute(leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         // few leaves: their row blocks over several CTAs while SMs are idle
         const uint32_t parts = (uint32_t)std::max<size_t>(1, std::min<size_t>(tiles, c->sm_count / ntiles));
-        tc_leaf_kernel<<<dim3((unsigned)ntiles, parts), kLeafThreads, bytes, c->stream>>>(p, tiles);
+        leaf<<<dim3((unsigned)ntiles, parts), kLeafThreads, bytes, c->stream>>>(p, tiles);
         ANQI_CUDA(c, cudaGetLastError());
         return ANQI_OK;
     }
