@@ -214,8 +214,9 @@ __global__ void fit_lohi_init_kernel(double* lohi, uint32_t nk) {
 // each tile's digits, sums the counts over the column (digit by digit, tile by
 // tile) and moves each key to its place.  Sixteen passes over memory in all, where
 // a bitonic network over columns padded to a power of two makes over a hundred, as
-// many as fit in shared memory at once: 100 columns of 120,000, SORT_FIG.
-// Bound by the moves' scattered 8-byte writes and the lanes' digit matching.
+// many as fit in shared memory at once: 100 columns of 120,000, 3.5 ms that way and
+// 1.77 ms this way (72 us a count, 144 us a move; 15 and 30 by their bytes).
+// Bound by the lanes' digit matching and the moves' scattered 8-byte writes.
 constexpr uint32_t kSortTile = 4096, kSortPer = 16;  // keys a tile of 8 warps; a thread's share
 
 // The digit at `shift` of a key's rank among doubles (sign folded in).
