@@ -527,9 +527,9 @@ __global__ void __launch_bounds__(kFilterThreads, kWide ? 1 : 2) tc_filter_kerne
 // operands; warp 16 issues the 128 x 128 products into a ring of four TMEM
 // accumulators, and warps 0-15 test them: warp w TMEM lanes 32 (w % 4) .. + 31,
 // its rows, and columns 32 (w / 4) .. + 31.  An accumulator is free again as soon
-// as it is in registers.  Rows and columns that are all exact take three
-// instructions a pair; the others the full error bound, with its column terms
-// read four at a time.  Survivors, about a tenth of the pairs once the lists are
+// as it is in registers.  Rows and columns that are all exact, with keys that
+// are too, take three instructions a pair; the others the full error bound, with
+// its column terms read four at a time.  Survivors, about a tenth of the pairs once the lists are
 // full, take one slot reservation per 32 pairs and one 8-byte store each, without
 // a loop over set bits (whose length is the warp's longest).
 // Bound by issue and, with one CTA to an SM, by the time its rows take to come in.
@@ -546,7 +546,8 @@ __host__ __device__ constexpr size_t leaf_smem(uint32_t dp, uint32_t tiles) {
     return (size_t)tiles * kTile * dp * 2 + 6 * (size_t)kLeafRows * 4;
 }
 
-// kPlain: every row exact and d <= 128, so no bound and no recheck.
+// kPlain: every row exact, d <= 128 and no key above 2^24 (leaf_plain), so no bound
+// and no recheck.
 template <bool kPlain>
 __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p, uint32_t tiles) {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -1555,6 +1556,14 @@ static bool leaf_whole(uint32_t dp, uint32_t maxcnt) {
     return maxcnt <= kLeafRows && leaf_smem(dp, (maxcnt + kTile - 1) / kTile) <= 226 * 1024 && !(env && env[0] == '0');
 }
 
+// Whether the whole-leaf kernel may test a pair by the sign of thr - key in one
+// sum: exact rows whose keys FP32 holds exactly.  An l2 key is at most (|q| + |x|)^2
+// <= 4 max |x|^2 and past 2^24 the reference's is rounded, so there a sum that is
+// not would drop ties with the threshold; an ip key, 1 - <a, b>, stays within 2^23.
+static bool leaf_plain(const FilterParams& p) {
+    return p.all_exact && p.d <= 128 && (p.key_mode == 1 || 4.0f * p.bx_n <= 16777216.0f);
+}
+
 int tc_leaf_tiles(Ctx* c, const std::vector<LeafRef>& leaves, const TcPrep& tp, uint32_t maxcnt, uint32_t cap,
                   std::vector<LeafTile>& tiles) {
     const bool whole = leaf_whole(tp.dp, maxcnt);
@@ -1601,7 +1610,7 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
     if (leaf_whole(p.dp, maxcnt)) {
         const uint32_t tiles = (maxcnt + kTile - 1) / kTile;
         const size_t bytes = leaf_smem(p.dp, tiles);
-        auto leaf = p.all_exact && p.d <= 128 ? tc_leaf_kernel<true> : tc_leaf_kernel<false>;
+        auto leaf = leaf_plain(p) ? tc_leaf_kernel<true> : tc_leaf_kernel<false>;
         ANQI_CUDA(c, cudaFuncSetAttribute(leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         // few leaves: their row blocks over several CTAs while SMs are idle
         const uint32_t parts = (uint32_t)std::max<size_t>(1, std::min<size_t>(tiles, c->sm_count / ntiles));
