@@ -197,7 +197,7 @@ __device__ __forceinline__ bool visit_id(Visited& vis, uint32_t* win, uint32_t w
     return vis_first(vis, id, rec, err);
 }
 
-// Of the m (<= 64) fresh (dist, id) entries in nd/ni, keeps those that can
+// Of the m (<= 64) fresh (dist, id) entries in nd/ni (NaN counting as +inf), keeps those that can
 // enter the beam -- all of them while the beam is not full, else those ranking
 // before its last entry (td, tid), since any other would land at rank >= L --
 // and sorts them ascending into nd/ni[0..m').  Returns m'.  Small batches (the
@@ -208,7 +208,7 @@ template <class Ord = IdOrder, bool kCompact = false>
 __device__ __forceinline__ uint32_t sort_fresh_kept(float* nd, uint32_t* ni, uint32_t m, bool full, float td,
                                                     uint32_t tid, uint32_t lane, Ord ord = Ord()) {
     if (m <= 32) {
-        const float dv = lane < m ? nd[lane] : 0.f;
+        const float dv = lane < m ? rank_dist(nd[lane]) : 0.f;
         const uint32_t iv = lane < m ? ni[lane] : kEmpty;
         const bool keep = lane < m && (!full || ord(dv, iv, td, tid));
         const unsigned km = __ballot_sync(kAll, keep);
@@ -240,9 +240,9 @@ __device__ __forceinline__ uint32_t sort_fresh_kept(float* nd, uint32_t* ni, uin
         return __popc(km);
     }
     const float inf = __int_as_float(0x7f800000);
-    float d0 = lane < m ? nd[lane] : inf;
+    float d0 = lane < m ? rank_dist(nd[lane]) : inf;
     uint32_t i0 = lane < m ? ni[lane] : kEmpty;
-    float d1 = lane + 32 < m ? nd[lane + 32] : inf;
+    float d1 = lane + 32 < m ? rank_dist(nd[lane + 32]) : inf;
     uint32_t i1 = lane + 32 < m ? ni[lane + 32] : kEmpty;
     warp_sort64<Ord, kCompact>(d0, i0, d1, i1, ord);
     __syncwarp();

@@ -344,6 +344,12 @@ __device__ __forceinline__ void stage_row_async(float* dst, const float* __restr
     for (uint32_t c = t; c < stride / 4; c += nthreads) cp_async16(dst + 4 * c, src + 4 * c);
 }
 
+// A distance as beams and lists rank it: NaN (a row or query that holds one, or
+// inf - inf of overflowed norms) counts as +inf.  Left in, it would compare false
+// both ways, two entries would take one rank, and a merge by ranks would leave a
+// slot with whatever the memory held, to be followed as an id.
+__device__ __forceinline__ float rank_dist(float d) { return d == d ? d : __int_as_float(0x7f800000); }
+
 // nndindex::d2 (index.h:172-176): (na + nb) - 2 * ip(a, b)
 __device__ __forceinline__ float norm_d2(float na, float nb, float ip) {
     return __fsub_rn(__fadd_rn(na, nb), __fmul_rn(2.0f, ip));

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32 * kWpb, 32 / kWpb) rknn_search_kernel(Searc
         __syncwarp();
         if (lane == 0) {
             win[(ep - wbase) >> 5] |= 1u << ((ep - wbase) & 31u);  // the entry lies in the window
-            bd[0] = dep;
+            bd[0] = rank_dist(dep);
             bi[0] = ep;
         }
         uint32_t nlog = 0, nvis = 1, ncand = 0, nexp = 0, nfl = 0;
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
             const float dep = row_dist(ep);
             if (lane == 0) {
                 bits[ep >> 5] |= 1u << (ep & 31u);
-                beam(0)[0] = dep;
+                beam(0)[0] = rank_dist(dep);
                 reinterpret_cast<uint32_t*>(beam(0) + p.L_max)[0] = ep;
                 const bool in = dep <= r2f;
                 if (in) clist[0] = ep;
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
             }
             if (warp * 8 < m) {
                 const float d = row_dist(ni[min(grp, m - 1)]);
-                if (gt == 0 && grp < m) nd[grp] = d;
+                if (gt == 0 && grp < m) nd[grp] = rank_dist(d);
             }
             __syncthreads();
             if (warp == 7) {

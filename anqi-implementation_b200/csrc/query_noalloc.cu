@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(32 * kWarps) noalloc_search_kernel(NoAllocPara
         if (lane == 0) {
             visit_first(bits, ep);
             vlog[0] = ep;
-            bdA[0] = dep;
+            bdA[0] = rank_dist(dep);
             biA[0] = ep;
         }
         uint32_t nlog = 1, ncand = 0;

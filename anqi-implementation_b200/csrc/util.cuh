@@ -119,13 +119,14 @@ static __device__ uint32_t warp_merge(const float* ld, const uint32_t* li, uint3
     return ns;
 }
 
-// Sorts up to 64 (d, id) entries held in nd/ni[0..m) (pads filled here).
+// Sorts up to 64 (d, id) entries held in nd/ni[0..m) (pads filled here, NaN as
+// +inf).
 __device__ __forceinline__ void warp_sort_batch64(float* nd, uint32_t* ni, uint32_t m) {
     const uint32_t lane = threadIdx.x & 31u;
     const float inf = __int_as_float(0x7f800000);
-    float d0 = lane < m ? nd[lane] : inf;
+    float d0 = lane < m ? rank_dist(nd[lane]) : inf;
     uint32_t i0 = lane < m ? ni[lane] : kEmpty;
-    float d1 = lane + 32 < m ? nd[lane + 32] : inf;
+    float d1 = lane + 32 < m ? rank_dist(nd[lane + 32]) : inf;
     uint32_t i1 = lane + 32 < m ? ni[lane + 32] : kEmpty;
     warp_sort64(d0, i0, d1, i1);
     __syncwarp();
