@@ -1391,8 +1391,9 @@ __global__ void __launch_bounds__(256) leaf_topk_kernel(const float* __restrict_
         const uint32_t r = t / K, k = t % K;
         const uint64_t row = mem[rb + r];
         const uint32_t h = rbuf[r];
-        kd[row * K + k] = ld[(h * kLeafRows + r) * K + k];
-        ki[row * K + k] = li[(h * kLeafRows + r) * K + k];
+        const bool in = k < rsz[r];  // past a short list: empty, as init_lists_kernel left it
+        kd[row * K + k] = in ? ld[(h * kLeafRows + r) * K + k] : FLT_MAX;
+        ki[row * K + k] = in ? li[(h * kLeafRows + r) * K + k] : kEmpty;
     }
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) ksz[mem[rb + r]] = rsz[r];
 }
