@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(128, kVam ? 5 : 7) gather_kernel(GatherParams 
 // rows in shared memory, takes a chunk of an expansion's ids with a thread each,
 // fetches a row per 4-thread group and merges the kept ones into the beam in one
 // step between two buffers.  The beam, the pool count and the order are
-// gather_kernel's, so the lists are.  Bound by the latency of that chain and its
+// gather_kernel's, so the lists are; any row is accepted, NaN distances ranking
+// as +inf.  Bound by the latency of that chain and its
 // barriers, so by blocks in flight: 128 threads (ten blocks an SM by registers)
 // for l2; the ip metric's sequential sums need more rows per fetch, 256 threads
 // and five blocks.  Unit rows, 64 trees, ef = 600: 100,000 x 128 l2 181 -> 52 ms
@@ -649,7 +650,7 @@ __device__ __forceinline__ void block_ip64(const GatherParams& p, const float* x
         }
         __syncthreads();
     }
-    if (t < m) out[t] = __fsub_rn(1.0f, acc);
+    if (t < m) out[t] = rank_dist(__fsub_rn(1.0f, acc));
 }
 
 template <bool kIp>
@@ -703,7 +704,7 @@ __global__ void __launch_bounds__(kGbThreads<kIp>, kIp ? 5 : 10) gather_block_ke
             at = __shfl_sync(kAll, at, 0) + __popc(b & lane_lt_mask());
             if (f) {
                 ni[at] = id;
-                if (vals) nd[at] = v;
+                if (vals) nd[at] = rank_dist(v);
             }
             // the next chunk's counter: last read two chunks ago, before the
             // last chunk's barrier
@@ -822,7 +823,7 @@ __global__ void __launch_bounds__(kGbThreads<kIp>, kIp ? 5 : 10) gather_block_ke
                             const float* xj = p.x + (uint64_t)j * p.stride;
                             const float ip = p.cols ? group_ip_cols<128>(xi, xj, gt, kAll)
                                                     : group_ip(xi, xj, p.dim, gt, kAll);
-                            if (e < m && gt == 0) nd[e] = norm_d2(ni_norm, p.norms[j], ip);
+                            if (e < m && gt == 0) nd[e] = rank_dist(norm_d2(ni_norm, p.norms[j], ip));
                         }
                     }
                 }
@@ -1612,9 +1613,9 @@ __global__ void random_fill_kernel(const float* __restrict__ x, const float* __r
         for (uint32_t t = 0; t < miss; t++) {
             const uint32_t r = (uint32_t)(hash64(hash64(seed + 0x51ED270Bull) ^ (i << 20) ^ t) % n);
             // every lane forms the same key (the ip metric's is one sequential sum)
-            const float v = ip ? ip_dist_seq(x + i * stride, x + (uint64_t)r * stride, dim)
-                               : norm_d2(norms[i], norms[r], group_ip(x + i * stride, x + (uint64_t)r * stride, dim,
-                                                                     gt, kAll));
+            const float v = rank_dist(ip ? ip_dist_seq(x + i * stride, x + (uint64_t)r * stride, dim)
+                                         : norm_d2(norms[i], norms[r],
+                                                   group_ip(x + i * stride, x + (uint64_t)r * stride, dim, gt, kAll)));
             bool dup = false;
             for (uint32_t s = lane; s < size; s += 32) dup |= id[s] == r;
             dup = __any_sync(kAll, dup);
