@@ -1690,8 +1690,12 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
         }
     }
     if (cfgs.empty()) return fail(c, ANQI_ERR_ARGS, "beam width %u needs too much shared memory", b.L_max);
-    uint32_t slots = 0, gslots = 0, gcap_max = 0;
+    // slots: warps of the warp-per-query form, each with a bitmap and a log; lists:
+    // candidate lists, one a warp of that form or one a block of the other
+    uint32_t slots = 0, lists = 0, gslots = 0, gcap_max = 0;
     for (const SearchCfg& g : cfgs) {
+        lists = std::max(lists, g.block ? g.blocks : g.blocks * g.wpb);
+        if (g.block) continue;
         slots = std::max(slots, g.blocks * g.wpb);
         if (g.gcap) gslots = std::max(gslots, g.blocks * g.wpb);
         gcap_max = std::max(gcap_max, g.gcap);
@@ -1710,21 +1714,22 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
         set_l2_window(c, c->vis_gtab.p, (size_t)c->gtab_slots * c->gtab_cap * 4);
         c->l2_window = true;
     }
-    // per-slot scratch (bitmap, log, candidate list) for the largest configuration
+    // scratch (bitmaps and logs, candidate lists) for the largest configuration
     const uint32_t words = (uint32_t)((ix.n + 31) / 32);
     const uint32_t log_cap = (uint32_t)std::min<uint64_t>(ix.n, 16384);
     const uint32_t cand_cap = (uint32_t)std::min<uint64_t>(ix.n, 65536);
-    if (c->vis_slots < slots || c->vis_words != words || c->log_cap != log_cap || c->cand_cap != cand_cap) {
+    if (slots && (c->vis_slots < slots || c->vis_words != words || c->log_cap != log_cap)) {
+        c->vis_slots = 0;  // until both are there
         if ((rc = ensure(c, c->vis_bits, (size_t)slots * words * 4)) ||
-            (rc = ensure(c, c->vis_log, (size_t)slots * log_cap * 4)) ||
-            (rc = ensure(c, c->cand_scratch, (size_t)slots * cand_cap * 4)))
+            (rc = ensure(c, c->vis_log, (size_t)slots * log_cap * 4)))
             return rc;
         ANQI_CUDA(c, cudaMemsetAsync(c->vis_bits.p, 0, (size_t)slots * words * 4, c->stream));
         c->vis_slots = slots;
         c->vis_words = words;
         c->log_cap = log_cap;
-        c->cand_cap = cand_cap;
     }
+    if ((rc = ensure(c, c->cand_scratch, (size_t)lists * cand_cap * 4))) return rc;
+    c->cand_cap = cand_cap;
     if ((rc = prepare_entries(c, !use_block, &b.ordered))) return rc;
     if (b.pred_cap == 0) b.pred_cap = std::max<uint64_t>(1024, (uint64_t)b.nq * 128);
     if (keep_candidates && b.cand_cap == 0) b.cand_cap = std::max<uint64_t>(1024, (uint64_t)b.nq * 256);
