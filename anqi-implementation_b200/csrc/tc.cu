@@ -757,10 +757,11 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
 //   warps 0-7  read the other accumulator back and test it.
 // The query tile stays resident up to 512 padded dimensions and streams with
 // the base tile above.  The test costs three instructions a pair: base-tile
-// column constants C (the norm, or norm minus threshold rounded down) come with
-// the tile, a row constant R holds the rest of the inequality less eps over all
-// columns and a rounding margin, and the sign of C + R + f acc is shifted into a
-// mask.  Survivors go to a queue per warp; 32 of them at a time take the exact
+// column constants C (the norm, or norm minus threshold, less a margin for its
+// own rounding) come with the tile, a row constant R holds the rest of the
+// inequality less eps over all columns and a margin for its terms, and the sign of
+// C + R + f acc is shifted into a mask.  Each column carries its own margin: one
+// of the largest |C| in every row let a single threshold of FLT_MAX keep all pairs.  Survivors go to a queue per warp; 32 of them at a time take the exact
 // test and the output slot's atomic, so its latency is paid once per 32.
 // At 100,000 x 300 (unit rows, top-100, then three CSRs of 2,000 queries) the
 // scans take 10.1 ms; tiles that were copied 16 bytes a thread and waited for
@@ -772,7 +773,6 @@ struct ScanParams {
     const unsigned char* qpack;  // query tiles of 128 rows
     const unsigned char* xpack;  // base tiles of 256 rows
     const float* cpack;          // column constants C, 256 per base tile (+inf past n)
-    const float* cmax;           // the largest finite |C|
     uint32_t qtiles, xtiles, slices, slots;
 };
 
@@ -922,7 +922,6 @@ __global__ void __launch_bounds__(kScanThreads, 1) tc_scan_kernel(ScanParams sp)
         const float g = 2.0f * p.dp * u;
         const float kh = l2k ? 1.f : 0.5f;
         const float cc = l2k ? 4.f * u : 0.f;
-        const float cmax = *sp.cmax;
         uint32_t tt = 0;
         for (uint32_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
             const uint32_t qt = item / sp.slices, t0 = item % sp.slices * per, t1 = min(sp.xtiles, t0 + per);
@@ -941,10 +940,10 @@ __global__ void __launch_bounds__(kScanThreads, 1) tc_scan_kernel(ScanParams sp)
             const float cd = l2k ? 4.f * u * qn : 4.f * u;
             const float epsmax =
                 (qexact && p.all_exact) ? 0.f : fmaf(ca, p.bx_norm, fmaf(cb, p.bx_err, fmaf(cc, p.bx_n, cd)));
-            // C + R + f acc <= 0 for every pair with key~ - epsmax <= threshold:
-            // the margin covers the roundings of R, C + R and the test's FMA
+            // C + R + f acc < 0 for every pair with key~ - epsmax <= threshold: the
+            // margins here and in C cover the roundings of key~, R and C + R
             const float q0 = l2k ? qn : (p.key_mode == 1 ? 1.f : 0.f);
-            const float margin = 16.f * u * (fabsf(q0) + (p.thr_row ? fabsf(thr_r) : 0.f) + epsmax + cmax + p.bx_n) + 1e-37f;
+            const float margin = 16.f * u * (fabsf(q0) + (p.thr_row ? fabsf(thr_r) : 0.f) + epsmax + p.bx_n) + 1e-37f;
             float R = q0 - thr_r - epsmax - margin;
             if (p.thr_row && thr_r == __int_as_float(0x7f800000)) R = -__int_as_float(0x7f800000);
             uint32_t nq = 0;  // survivors waiting in the warp's queue (uniform)
@@ -1079,21 +1078,19 @@ __global__ void pack_tiles_kernel(const __nv_bfloat16* __restrict__ src, const u
 }
 
 // The scan's column constants: the norm (l2) less the column's threshold if it
-// has one, rounded down; +inf past n.  *cmax: the largest finite magnitude.
+// has one, less 2^-20 of that for the roundings it goes through; +inf past n.
 __global__ void scan_columns_kernel(const float* __restrict__ xn, const float* __restrict__ thr_col, uint64_t n,
-                                    uint64_t padded, uint32_t key_mode, float* __restrict__ C, float* cmax) {
-    float mx = 0.f;
+                                    uint64_t padded, uint32_t key_mode, float* __restrict__ C) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < padded;
          j += (uint64_t)gridDim.x * blockDim.x) {
         float c = __int_as_float(0x7f800000);
         if (j < n) {
             c = key_mode == 0 ? xn[j] : 0.f;
             if (thr_col) c = __fsub_rd(c, thr_col[j]);
-            if (fabsf(c) <= 3.4028235e38f) mx = fmaxf(mx, fabsf(c));
+            if (fabsf(c) <= 3.4028235e38f) c = __fsub_rd(c, 9.5367432e-7f * fabsf(c));
         }
         C[j] = c;
     }
-    atomicMax(reinterpret_cast<uint32_t*>(cmax), __float_as_uint(mx));
 }
 
 // Upper bound of each row's K-th smallest key: the largest reference FP32 key
@@ -1288,22 +1285,19 @@ int launch_scan(Ctx* c, FilterParams p, uint64_t nrows) {
     const size_t cbytes = (size_t)sp.xtiles * kScanN * 4;
     int rc;
     if ((rc = ensure(c, c->init_cid, qbytes)) || (rc = ensure(c, c->init_key, xbytes)) ||
-        (rc = ensure(c, c->init_cnt, cbytes + 16)))
+        (rc = ensure(c, c->init_cnt, cbytes)))
         return rc;
     float* cpack = c->init_cnt.as<float>();
-    float* cmax = cpack + (size_t)sp.xtiles * kScanN;
     const uint32_t blocks = c->sm_count * 8;
-    ANQI_CUDA(c, cudaMemsetAsync(cmax, 0, 4, c->stream));
     pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.qb, p.rows, nrows, p.dp, kTile, qbytes / 16, c->init_cid.as<uint4>());
     pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.xb, nullptr, p.n, p.dp, kScanN, xbytes / 16, c->init_key.as<uint4>());
     scan_columns_kernel<<<blocks, 256, 0, c->stream>>>(p.xn, p.thr_col, p.n, (uint64_t)sp.xtiles * kScanN, p.key_mode,
-                                                       cpack, cmax);
+                                                       cpack);
     ANQI_CUDA(c, cudaGetLastError());
     sp.f = p;
     sp.qpack = c->init_cid.as<unsigned char>();
     sp.xpack = c->init_key.as<unsigned char>();
     sp.cpack = cpack;
-    sp.cmax = cmax;
     // items of one query tile and a slice of the base tiles, at least eight per
     // SM while a slice keeps 16 tiles, so that the last wave is short
     sp.slices = (uint32_t)std::max<uint64_t>(
