@@ -1274,7 +1274,7 @@ int filter_kernel_for(Ctx* c, uint32_t dp, void (**kern)(FilterParams), size_t* 
 }
 
 // The scan of p over nrows query rows (p.rows: which; null: the first nrows).
-// The packed operands take the context's init_knn buffers, idle outside a build.
+// The packed operands are temporary: the context holds nothing after the call.
 int launch_scan(Ctx* c, FilterParams p, uint64_t nrows) {
     if (nrows == 0) return ANQI_OK;
     ScanParams sp{};
@@ -1283,21 +1283,19 @@ int launch_scan(Ctx* c, FilterParams p, uint64_t nrows) {
     sp.xtiles = (uint32_t)((p.n + kScanN - 1) / kScanN);
     const size_t qbytes = (size_t)sp.qtiles * kTile * p.dp * 2, xbytes = (size_t)sp.xtiles * kScanN * p.dp * 2;
     const size_t cbytes = (size_t)sp.xtiles * kScanN * 4;
+    TmpBuf qpack(c), xpack(c), cpack(c);
     int rc;
-    if ((rc = ensure(c, c->init_cid, qbytes)) || (rc = ensure(c, c->init_key, xbytes)) ||
-        (rc = ensure(c, c->init_cnt, cbytes)))
-        return rc;
-    float* cpack = c->init_cnt.as<float>();
+    if ((rc = ensure(c, qpack, qbytes)) || (rc = ensure(c, xpack, xbytes)) || (rc = ensure(c, cpack, cbytes))) return rc;
     const uint32_t blocks = c->sm_count * 8;
-    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.qb, p.rows, nrows, p.dp, kTile, qbytes / 16, c->init_cid.as<uint4>());
-    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.xb, nullptr, p.n, p.dp, kScanN, xbytes / 16, c->init_key.as<uint4>());
+    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.qb, p.rows, nrows, p.dp, kTile, qbytes / 16, qpack.as<uint4>());
+    pack_tiles_kernel<<<blocks, 256, 0, c->stream>>>(p.xb, nullptr, p.n, p.dp, kScanN, xbytes / 16, xpack.as<uint4>());
     scan_columns_kernel<<<blocks, 256, 0, c->stream>>>(p.xn, p.thr_col, p.n, (uint64_t)sp.xtiles * kScanN, p.key_mode,
-                                                       cpack);
+                                                       cpack.as<float>());
     ANQI_CUDA(c, cudaGetLastError());
     sp.f = p;
-    sp.qpack = c->init_cid.as<unsigned char>();
-    sp.xpack = c->init_key.as<unsigned char>();
-    sp.cpack = cpack;
+    sp.qpack = qpack.as<unsigned char>();
+    sp.xpack = xpack.as<unsigned char>();
+    sp.cpack = cpack.as<float>();
     // items of one query tile and a slice of the base tiles, at least eight per
     // SM while a slice keeps 16 tiles, so that the last wave is short
     sp.slices = (uint32_t)std::max<uint64_t>(
