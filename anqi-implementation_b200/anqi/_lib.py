@@ -312,7 +312,8 @@ class Context:
 
     def inject_fault(self, flags: int) -> None:
         """Test hook (anqi_inject_fault): 1 = the search issues no row copies, so
-        its bounded waits run out and queries fail with ANQI_ERR_TIMEOUT; 0 = off."""
+        its bounded waits run out and queries fail with ANQI_ERR_TIMEOUT; 2 = device
+        allocations that a build can do without fail; 0 = off."""
         self._check(self.lib.anqi_inject_fault(self.h, flags), "inject_fault")
 
     def timer_start(self) -> None:

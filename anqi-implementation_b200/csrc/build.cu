@@ -2013,65 +2013,79 @@ static int run_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n, ui
                       DevBuf& O, DevBuf& Odeg, uint32_t M, float alpha, DevBuf& links_buf, DevBuf& deg_buf,
                       const uint32_t* row_order, double* kernel_ms);
 
+// Select and commit on the components' tables where the lists fall into small
+// components everywhere (*done; ANQI_B200_GRAPH_COMPONENTS=0: never).  Needs the
+// rows, lists and values once more, renumbered: where these cannot be had the
+// caller takes the general gather.
+static int component_select_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n, uint32_t stride,
+                                   uint32_t dim, const DevBuf& hid, const DevBuf& hval, uint32_t K, uint32_t M,
+                                   uint32_t ef, uint32_t cap, float alpha, DevBuf& links, DevBuf& deg,
+                                   uint64_t* pool_total, const uint32_t* row_order, double* kernel_ms, bool* done) {
+    const char* env = std::getenv("ANQI_B200_GRAPH_COMPONENTS");
+    if (env && env[0] == '0') return ANQI_OK;
+    OptionalPart part(c);
+    TmpBuf perm(c), inv(c), ids(c), vals(c), rows(c), norm(c), pool(c), roff(c), rev(c);
+    std::vector<CompRange> ranges;
+    uint64_t in_ranges = 0;
+    int rc;
+    if ((rc = locality_order(c, hid.as<uint32_t>(), n, K, row_order, perm, inv, ranges, in_ranges, true))) return rc;
+    if (in_ranges != n) return ANQI_OK;
+    const int blocks = c->sm_count * 8;
+    if ((rc = ensure(c, ids, n * K * 4)) || (rc = ensure(c, vals, n * K * 4)) ||
+        (rc = ensure(c, rows, n * stride * 4ull)) || (rc = ensure(c, norm, n * 4)) || (rc = ensure(c, pool, 8)) ||
+        (rc = ensure(c, links, n * M * 4)) || (rc = ensure(c, deg, n * 4)))
+        return rc;
+    renumber_lists_kernel<<<blocks, 256, 0, c->stream>>>(hid.as<uint32_t>(), hval.as<float>(), perm.as<uint32_t>(),
+                                                         inv.as<uint32_t>(), n, K, ids.as<uint32_t>(),
+                                                         vals.as<float>());
+    permute_rows_kernel<<<blocks, 256, 0, c->stream>>>(dx.as<float>(), rows.as<float>(), perm.as<uint32_t>(), n,
+                                                       stride, 0u);
+    permute_vals_kernel<<<blocks, 256, 0, c->stream>>>(dn.as<float>(), norm.as<float>(), perm.as<uint32_t>(), n);
+    ANQI_CUDA(c, cudaGetLastError());
+    ANQI_CUDA(c, cudaMemsetAsync(pool.p, 0, 8, c->stream));
+    if ((rc = build_reverse(c, ids.as<uint32_t>(), n, K, roff, rev))) return rc;
+    CompGather g{};
+    g.x = rows.as<float>();
+    g.norms = norm.as<float>();
+    g.n = n;
+    g.stride = stride;
+    g.dim = dim;
+    g.g_ids = ids.as<uint32_t>();
+    g.K = K;
+    g.rev_off = roff.as<uint64_t>();
+    g.rev_ids = rev.as<uint32_t>();
+    g.ef = ef;
+    g.cap = cap;
+    g.perm = perm.as<uint32_t>();
+    g.pool_total = pool.as<unsigned long long>();
+    bool any_bad = false;
+    ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+    if ((rc = run_component_select_commit(c, g, ranges, M, alpha, links.as<uint32_t>(), deg.as<uint32_t>(), &any_bad)))
+        return rc;
+    ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+    if ((rc = sync(c))) return rc;
+    if (any_bad) return ANQI_OK;
+    float ms = 0;
+    ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+    if (kernel_ms) *kernel_ms += ms;
+    if (pool_total) ANQI_CUDA(c, cudaMemcpy(pool_total, pool.p, 8, cudaMemcpyDeviceToHost));
+    *done = true;
+    return ANQI_OK;
+}
+
 static int run_select_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n, uint32_t stride, uint32_t dim,
                              const DevBuf& hid, const DevBuf& hval, uint32_t K, uint32_t M, uint32_t ef, uint32_t cap,
                              float alpha, DevBuf& O, DevBuf& Odeg, DevBuf* links, DevBuf* deg, uint64_t* pool_total,
                              const uint32_t* row_order = nullptr, double* kernel_ms = nullptr) {
-    TmpBuf roff(c), rev(c);
     int rc;
-    // lists that fall into small components everywhere: search and prune on the
-    // components' tables (ANQI_B200_GRAPH_COMPONENTS=0: the general gather)
-    const char* comp_env = std::getenv("ANQI_B200_GRAPH_COMPONENTS");
-    if (links && row_order && !c->edge.active && !(comp_env && comp_env[0] == '0')) {
-        TmpBuf perm(c), inv(c), ids(c), vals(c), rows(c), norm(c), pool(c);
-        std::vector<CompRange> ranges;
-        uint64_t in_ranges = 0;
-        if ((rc = locality_order(c, hid.as<uint32_t>(), n, K, row_order, perm, inv, ranges, in_ranges, true))) return rc;
-        if (in_ranges == n) {
-            const int blocks = c->sm_count * 8;
-            if ((rc = ensure(c, ids, n * K * 4)) || (rc = ensure(c, vals, n * K * 4)) ||
-                (rc = ensure(c, rows, n * stride * 4ull)) || (rc = ensure(c, norm, n * 4)) || (rc = ensure(c, pool, 8)) ||
-                (rc = ensure(c, *links, n * M * 4)) || (rc = ensure(c, *deg, n * 4)))
-                return rc;
-            renumber_lists_kernel<<<blocks, 256, 0, c->stream>>>(hid.as<uint32_t>(), hval.as<float>(),
-                                                                perm.as<uint32_t>(), inv.as<uint32_t>(), n, K,
-                                                                ids.as<uint32_t>(), vals.as<float>());
-            permute_rows_kernel<<<blocks, 256, 0, c->stream>>>(dx.as<float>(), rows.as<float>(), perm.as<uint32_t>(), n,
-                                                               stride, 0u);
-            permute_vals_kernel<<<blocks, 256, 0, c->stream>>>(dn.as<float>(), norm.as<float>(), perm.as<uint32_t>(), n);
-            ANQI_CUDA(c, cudaGetLastError());
-            ANQI_CUDA(c, cudaMemsetAsync(pool.p, 0, 8, c->stream));
-            if ((rc = build_reverse(c, ids.as<uint32_t>(), n, K, roff, rev))) return rc;
-            CompGather g{};
-            g.x = rows.as<float>();
-            g.norms = norm.as<float>();
-            g.n = n;
-            g.stride = stride;
-            g.dim = dim;
-            g.g_ids = ids.as<uint32_t>();
-            g.K = K;
-            g.rev_off = roff.as<uint64_t>();
-            g.rev_ids = rev.as<uint32_t>();
-            g.ef = ef;
-            g.cap = cap;
-            g.perm = perm.as<uint32_t>();
-            g.pool_total = pool.as<unsigned long long>();
-            bool any_bad = false;
-            ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-            if ((rc = run_component_select_commit(c, g, ranges, M, alpha, links->as<uint32_t>(), deg->as<uint32_t>(),
-                                                  &any_bad)))
-                return rc;
-            ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-            if ((rc = sync(c))) return rc;
-            if (!any_bad) {
-                float ms = 0;
-                ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-                if (kernel_ms) *kernel_ms += ms;
-                if (pool_total) ANQI_CUDA(c, cudaMemcpy(pool_total, pool.p, 8, cudaMemcpyDeviceToHost));
-                return ANQI_OK;
-            }
-        }
+    if (links && row_order && !c->edge.active) {
+        bool done = false;
+        rc = component_select_commit(c, dx, dn, n, stride, dim, hid, hval, K, M, ef, cap, alpha, *links, *deg, pool_total,
+                                     row_order, kernel_ms, &done);
+        if (done) return ANQI_OK;
+        if (rc && !fall_back(c, rc)) return rc;
     }
+    TmpBuf roff(c), rev(c);
     if ((rc = build_reverse(c, hid.as<uint32_t>(), n, K, roff, rev))) return rc;
     uint64_t mr = 0, rev_total = 0;
     if ((rc = list_bounds(c, roff, n, &mr, &rev_total))) return rc;
@@ -3134,16 +3148,22 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
         g.pool_total = comp_pool.as<unsigned long long>();
         bool any_bad = false;
         ANQI_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-        if ((rc = run_component_gather(c, g, ranges, row_comp, comp_bad, &any_bad))) return rc;
-        ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
-        ANQI_CUDA(c, cudaMemcpyAsync(&pool_total, comp_pool.p, 8, cudaMemcpyDeviceToHost, c->stream));
-        if ((rc = sync(c))) return rc;
-        float ms = 0;
-        ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-        gather_kernel_ms += ms;
-        p.row_comp = row_comp.as<uint32_t>();
-        p.comp_bad = comp_bad.as<uint32_t>();
-        rest = in_ranges < n || any_bad;
+        {
+            OptionalPart part(c);
+            rc = run_component_gather(c, g, ranges, row_comp, comp_bad, &any_bad);
+        }
+        if (rc && !fall_back(c, rc)) return rc;
+        if (!rc) {  // else all rows go to the general gather
+            ANQI_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+            ANQI_CUDA(c, cudaMemcpyAsync(&pool_total, comp_pool.p, 8, cudaMemcpyDeviceToHost, c->stream));
+            if ((rc = sync(c))) return rc;
+            float ms = 0;
+            ANQI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+            gather_kernel_ms += ms;
+            p.row_comp = row_comp.as<uint32_t>();
+            p.comp_bad = comp_bad.as<uint32_t>();
+            rest = in_ranges < n || any_bad;
+        }
     }
     if (rest) {
         uint64_t pooled = 0;

@@ -94,6 +94,7 @@ int ensure(Ctx* c, DevBuf& b, size_t bytes) {
     if (b.p) free_buf(c, b);
     const bool pooled = b.pooled && c->pool;
     auto alloc = [&] {
+        if (c->optional && (c->inject & ANQI_FAULT_OPTIONAL_ALLOC)) return cudaErrorMemoryAllocation;
         return pooled ? cudaMallocFromPoolAsync(&b.p, bytes, c->pool, c->stream) : cudaMalloc(&b.p, bytes);
     };
     cudaError_t e = alloc();
@@ -490,7 +491,7 @@ extern "C" {
 int anqi_version(void) { return 1; }
 
 int anqi_inject_fault(anqi_ctx* h, uint32_t flags) {
-    if (!h || (flags & ~ANQI_FAULT_DROP_ROW_COPIES)) return ANQI_ERR_ARGS;
+    if (!h || (flags & ~(ANQI_FAULT_DROP_ROW_COPIES | ANQI_FAULT_OPTIONAL_ALLOC))) return ANQI_ERR_ARGS;
     h->c.inject = flags;
     return ANQI_OK;
 }

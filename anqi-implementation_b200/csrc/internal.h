@@ -122,6 +122,7 @@ struct Ctx {
     int device = 0;
     int sm_count = 0;
     uint32_t inject = 0;  // ANQI_FAULT_* flags (anqi_inject_fault)
+    int optional = 0;     // inside a part with a fallback for failed allocations (OptionalPart)
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;  // the device's pool of temporary buffers (shared by its contexts), or null
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
@@ -198,6 +199,21 @@ struct TmpBuf : DevBuf {
     TmpBuf(const TmpBuf&) = delete;
     TmpBuf& operator=(const TmpBuf&) = delete;
 };
+// Marks a part of a call that its caller falls back from when an allocation in it
+// fails (ANQI_ERR_DEVICE).
+struct OptionalPart {
+    Ctx* c;
+    explicit OptionalPart(Ctx* ctx) : c(ctx) { c->optional++; }
+    ~OptionalPart() { c->optional--; }
+    OptionalPart(const OptionalPart&) = delete;
+    OptionalPart& operator=(const OptionalPart&) = delete;
+};
+// Whether an OptionalPart's status is one to fall back from; the message it left goes.
+inline bool fall_back(Ctx* c, int rc) {
+    if (rc != ANQI_ERR_DEVICE) return false;
+    c->last_error.clear();
+    return true;
+}
 int h2d(Ctx* c, DevBuf& b, const void* src, size_t bytes);
 // Host <-> device copies of raw ranges on the context's stream (large
 // pageable ranges through pinned staging slots; d2h_raw then returns with the

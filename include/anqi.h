@@ -54,13 +54,16 @@ int anqi_version(void);
  * from a pool per device that keeps up to 8 GB cached while any context lives
  * (not counted here). */
 uint64_t anqi_device_bytes(const anqi_ctx* ctx);
-/* Test hook, no counterpart in the reference: makes the device waits of this
- * context run out without any fault.  ANQI_FAULT_DROP_ROW_COPIES: the search
+/* Test hook, no counterpart in the reference: failures of this context made
+ * without any fault.  ANQI_FAULT_DROP_ROW_COPIES: the search
  * kernel of later anqi_query_run / anqi_rknn_query calls issues no bulk copies
  * of lifted rows, so its bounded waits for them (a fixed number of polls)
  * expire with nothing in flight; the call returns ANQI_ERR_TIMEOUT and the context
- * stays usable.  flags = 0 restores normal operation. */
+ * stays usable.  ANQI_FAULT_OPTIONAL_ALLOC: device allocations that a build can
+ * do without fail, as they would on a full device, and the build takes the form
+ * that needs less memory (same output).  flags = 0 restores normal operation. */
 #define ANQI_FAULT_DROP_ROW_COPIES 1u
+#define ANQI_FAULT_OPTIONAL_ALLOC 2u
 int anqi_inject_fault(anqi_ctx* ctx, uint32_t flags);
 /* Device timer on the context's stream (CUDA events): start, then stop returns
  * the elapsed milliseconds of everything the context ran in between. */
