@@ -2943,10 +2943,26 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
         TcPrep& tp;
         ~Release() { tc_release(c, tp); }
     } release_tp{c, tp};
-    if (tensor && (rc = tc_prep(c, dx.as<float>(), dn.as<float>(), n, xs, d, tp))) return rc;
+    auto prepare_rows = [&] { return tensor ? tc_prep(c, dx.as<float>(), dn.as<float>(), n, xs, d, tp) : ANQI_OK; };
+    auto forest = [&](const TcPrep* rows) {
+        return build_forest(c, dx.as<float>(), n, d, xs, ap->trees, ap->leaf, 100, ap->seed, cap_nodes, f, ip, rows);
+    };
     const char* rows_env = std::getenv("ANQI_B200_FOREST_BF16");  // 0: sides from the FP32 rows
-    rc = build_forest(c, dx.as<float>(), n, d, xs, ap->trees, ap->leaf, 100, ap->seed, cap_nodes, f, ip,
-                      tensor && !(rows_env && rows_env[0] == '0') ? &tp : nullptr);
+    if (tensor && !(rows_env && rows_env[0] == '0')) {
+        {
+            OptionalPart part(c);
+            if (!(rc = prepare_rows())) rc = forest(&tp);
+        }
+        if (rc && fall_back(c, rc)) {
+            // no room for both: the forest first, from the FP32 rows
+            tc_release(c, tp);
+            release(c, f.perm);
+            release(c, f.hyper);
+            if (!(rc = forest(nullptr))) rc = prepare_rows();
+        }
+    } else if (!(rc = forest(nullptr))) {
+        rc = prepare_rows();
+    }
     const double forest_ms = ms_since(t);
     t = Clock::now();
     if (!rc) {
