@@ -1797,7 +1797,7 @@ static int run_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_t
                  : policy                ? gather_kernel<false, false, false, true>
                  : sub                   ? gather_kernel<false, false, false, false, true>
                                          : gather_kernel<false>;
-    ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(kern));
     int per_sm = 0;
     ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps_per_block, smem));
     if (per_sm < 1) return fail(c, ANQI_ERR_DEVICE, "gather kernel does not fit on an SM");
@@ -1893,7 +1893,7 @@ static int run_aknn_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* p
     const int threads = p.ip ? kGbThreads<true> : kGbThreads<false>;
     int per_sm = 0;
     if (!(env && env[0] == '0') && p.ef > p.out_k && smem <= 227 * 1024) {
-        ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ANQI_CUDA(c, allow_smem(kern));
         ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     }
     if (per_sm < 3) return run_gather(c, p, max_rev, pool_total, kernel_ms);
@@ -1971,7 +1971,7 @@ static int run_localjoin(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n,
         ANQI_CUDA(c, cudaGetLastError());
         const int wpb = 4;
         const size_t smem = (size_t)(2 * 512 + 2 * K + 2 * 128) * 4 * wpb;
-        ANQI_CUDA(c, cudaFuncSetAttribute(join_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ANQI_CUDA(c, allow_smem(join_apply_kernel));
         int per_sm = 0;
         ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, join_apply_kernel, 32 * wpb, smem));
         const uint32_t jb = std::max(1, per_sm) * c->sm_count;
@@ -2001,7 +2001,7 @@ static int run_warm_start(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n
     if ((rc = ensure(c, hid, n * K * 4)) || (rc = ensure(c, hval, n * K * 4))) return rc;
     const int wpb = 4;
     const size_t smem = (size_t)(2 * width + 2 * K) * 4 * wpb;
-    ANQI_CUDA(c, cudaFuncSetAttribute(warm_start_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(warm_start_kernel));
     warm_start_kernel<<<c->sm_count * 8, 32 * wpb, smem, c->stream>>>(dx.as<float>(), dn.as<float>(), n, row0, rows,
                                                                       stride, dim, d_cand, cstride, width, K,
                                                                       hid.as<uint32_t>(), hval.as<float>());
@@ -2426,7 +2426,7 @@ static int run_leaf_topk(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_t n,
                          2 * nwarp * 64 + tile_rows + 2 * kLeafRows) * 4;
     if (smem > 227 * 1024) return fail(c, ANQI_ERR_ARGS, "init_knn tile does not fit (dim %u, K %u)", dim, K);
     if (mode > kKeyNegIp) return fail(c, ANQI_ERR_ARGS, "unknown key mode %u", mode);
-    ANQI_CUDA(c, cudaFuncSetAttribute(leaf_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(leaf_topk_kernel));
     TmpBuf dl(c);
     int rc = h2d(c, dl, leaves.data(), leaves.size() * sizeof(LeafRef));
     if (rc) return rc;
@@ -2994,8 +2994,7 @@ int anqi_aknn_build(anqi_ctx* h, const float* base, uint64_t n, uint32_t d, cons
                 const int wpb = 4;
                 const size_t msmem = merge_smem_words(K) * 4 * wpb;
                 if (!rc && msmem > 48 * 1024)
-                    rc = cu(cudaFuncSetAttribute(leaf_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem),
-                            "cudaFuncSetAttribute");
+                    rc = cu(allow_smem(leaf_merge_kernel), "cudaFuncSetAttribute");
                 // every tree's batches planned on the host first, their tiles
                 // uploaded once: the filter and merge launches then follow
                 // each other on the stream without a host round trip

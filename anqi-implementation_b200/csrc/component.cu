@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(128) comp_search_kernel(CompSearchParams p) {
 template <int W>
 int launch_search(Ctx* c, const CompSearchParams& p, uint32_t blocks) {
     const size_t smem = 4ull * 4 * comp_search_words(p.mcap);
-    ANQI_CUDA(c, cudaFuncSetAttribute(comp_search_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(comp_search_kernel<W>));
     comp_search_kernel<W><<<blocks, 128, smem, c->stream>>>(p);
     ANQI_CUDA(c, cudaGetLastError());
     return ANQI_OK;

@@ -112,7 +112,7 @@ int sort_csr_segments(Ctx* c, const uint64_t* d_off, uint64_t nseg, uint32_t* d_
     if ((rc = ensure(c, sd, (size_t)sblocks * 4 * scr_cap * 4)) || (rc = ensure(c, si, (size_t)sblocks * 4 * scr_cap * 4)))
         return rc;
     const size_t ssm = 4 * 2 * 1024 * 4;
-    ANQI_CUDA(c, cudaFuncSetAttribute(sort_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+    ANQI_CUDA(c, allow_smem(sort_segments_kernel));
     sort_segments_kernel<<<sblocks, 128, ssm, c->stream>>>(d_off, nseg, d_ids, d_keys, sd.as<float>(),
                                                            si.as<uint32_t>(), scr_cap);
     ANQI_CUDA(c, cudaGetLastError());
@@ -152,7 +152,7 @@ extern "C" int anqi_rknn_ground_truth_metric(anqi_ctx* h, const float* base, uin
     while (tile > 8 && ((size_t)(kGtQ + tile) * xs + kGtQ) * 4 > 227 * 1024) tile -= 8;
     const size_t smem = ((size_t)(kGtQ + tile) * xs + kGtQ) * 4;
     if (smem > 227 * 1024) return fail(c, ANQI_ERR_ARGS, "dimension %u too large for the ground-truth kernel", d);
-    ANQI_CUDA(c, cudaFuncSetAttribute(rknn_gt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(rknn_gt_kernel));
     const unsigned blocks = (unsigned)((nq + kGtQ - 1) / kGtQ);
     rknn_gt_kernel<<<blocks, 256, smem, c->stream>>>(db.as<float>(), dbn.as<float>(), n, dq.as<float>(), nq, xs, d,
                                                      dr.as<float>(), dcnt.as<uint32_t>(), nullptr, nullptr, nullptr,
@@ -178,7 +178,7 @@ extern "C" int anqi_rknn_ground_truth_metric(anqi_ctx* h, const float* base, uin
     if ((rc = ensure(c, sd, (size_t)sblocks * 4 * scr_cap * 4)) || (rc = ensure(c, si, (size_t)sblocks * 4 * scr_cap * 4)))
         return rc;
     const size_t ssm = 4 * 2 * 1024 * 4;
-    ANQI_CUDA(c, cudaFuncSetAttribute(sort_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+    ANQI_CUDA(c, allow_smem(sort_segments_kernel));
     sort_segments_kernel<<<sblocks, 128, ssm, c->stream>>>(doff.as<uint64_t>(), nq, did.as<uint32_t>(),
                                                            dkey.as<float>(), sd.as<float>(), si.as<uint32_t>(), scr_cap);
     ANQI_CUDA(c, cudaGetLastError());

@@ -199,6 +199,20 @@ struct TmpBuf : DevBuf {
     TmpBuf(const TmpBuf&) = delete;
     TmpBuf& operator=(const TmpBuf&) = delete;
 };
+// Lets a kernel be launched with any dynamic shared memory that fits beside its
+// static share.  The limit belongs to the function, for every thread and context
+// of the process, so it always gets this one value: were it what the launch at
+// hand needs, a thread with a smaller launch could lower it between another's
+// setting and launch.
+template <class... Args>
+cudaError_t allow_smem(void (*kern)(Args...)) {
+    cudaFuncAttributes a{};
+    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                227 * 1024 - (int)a.sharedSizeBytes);
+}
+
 // Marks a part of a call that its caller falls back from when an allocation in it
 // fails (ANQI_ERR_DEVICE).
 struct OptionalPart {

@@ -340,7 +340,7 @@ static int lrq_encode(anqi_ctx* h, const float* keys, uint64_t n, uint32_t nk, u
         return rc;
     const size_t smem = ((size_t)kEncodeRows * nk + nk + (size_t)rankm * nk) * 4;
     if (smem > 200 * 1024) return fail(c, ANQI_ERR_ARGS, "nk too large for the encoder");
-    ANQI_CUDA(c, cudaFuncSetAttribute(lrq_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(lrq_encode_kernel));
     const unsigned blocks = (unsigned)((n + kEncodeRows - 1) / kEncodeRows);
     lrq_encode_kernel<<<blocks, kEncodeRows, smem, c->stream>>>(
         dk.as<float>(), n, nk, rankm, dmu.as<float>(), db.as<float>(), dcb.as<float>(), code_size, bits, policy,

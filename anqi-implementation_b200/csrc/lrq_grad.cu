@@ -407,7 +407,7 @@ cudaError_t launch_forward(ObjParams p, cudaStream_t st) {
     p.bcols = fit >= p.nk ? p.nk : (uint32_t)fit / 32 * 32;
     const size_t smem = fixed + (p.codes_in ? 0 : (size_t)p.bcols * p.bpitch * 8);
     auto kern = lrq_objective_forward_kernel<M, kThreads>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     constexpr uint64_t rows = kThreads / 32 * 4;
     kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
@@ -418,14 +418,14 @@ template <uint32_t M, uint32_t kThreads>
 cudaError_t launch_backward(const GradParams& p, cudaStream_t st) {
     const size_t smem = (size_t)(2 * M + 1) * 32 * kMaxCols * 8;
     auto kern = lrq_objective_backward_kernel<M, kThreads>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern);
     if (e != cudaSuccess) return e;
     constexpr uint64_t rows = kThreads / 32 * 4;
     kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // one block an SM, at least 64 rows a block
     const size_t hist = (size_t)p.cs * 32 * 8;
-    e = cudaFuncSetAttribute(lrq_codebook_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist);
+    e = allow_smem(lrq_codebook_grad_kernel);
     if (e != cudaSuccess) return e;
     const uint32_t groups = (p.nk + 31) / 32;
     const uint64_t rowgroups = std::min<uint64_t>((p.n + 63) / 64, std::max(1u, sm_count() / groups));

@@ -1185,6 +1185,7 @@ struct SearchCfg {
     uint64_t code() const { return hash_cap | (uint64_t)gcap << 24 | (uint64_t)wpb << 48 | (uint64_t)post_rows << 56; }
 };
 
+// (The kernel's allow_smem comes first.)
 static int search_cfg(Ctx* c, uint32_t hash_cap, uint32_t gcap, uint32_t wpb, uint32_t post_rows, SearchCfg& cfg) {
     const Batch& b = c->batch;
     cfg.hash_cap = hash_cap;
@@ -1194,7 +1195,6 @@ static int search_cfg(Ctx* c, uint32_t hash_cap, uint32_t gcap, uint32_t wpb, ui
     cfg.smem = search_smem_per_warp(c, b.L_max, hash_cap) * wpb;
     if (cfg.smem > 227 * 1024) return ANQI_ERR_ARGS;
     auto kern = search_kernel_for(c->ix.dim, wpb);
-    ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem));
     int per_sm = 0;
     ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, cfg.smem));
     if (per_sm < 1) return ANQI_ERR_ARGS;
@@ -1217,7 +1217,7 @@ static int block_cfg(Ctx* c, SearchCfg& cfg, bool* fits) {
     if ((env && env[0] == '0') || c->inject || smem > 227 * 1024 || stage_rows_for(c->ix.lstride, c->ix.bstride) != 8)
         return ANQI_OK;
     auto kern = block_kernel_for(c->ix.dim);
-    ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(kern));
     int per_sm = 0;
     ANQI_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlockThreads, smem));
     if ((uint64_t)per_sm * c->sm_count < b.nq) return ANQI_OK;
@@ -1489,8 +1489,7 @@ static int prepare_entries(Ctx* c, bool order, bool* ordered) {
     const uint32_t qpw = four ? 8u : 2u;
     const size_t smem = 4ull * qpw * ix.lstride * 4;
     auto kern = four ? rknn_entry_kernel<4> : rknn_entry_kernel<16>;
-    if (smem > 48 * 1024)
-        ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) ANQI_CUDA(c, allow_smem(kern));
     const uint32_t blocks = std::min<uint32_t>(c->sm_count * 8, (nq + 4 * qpw - 1) / (4 * qpw));
     kern<<<blocks, 128, smem, c->stream>>>(p, b.enode.as<uint32_t>(), b.entry.as<uint32_t>());
     const char* env = std::getenv("ANQI_B200_ORDER");
@@ -1584,7 +1583,6 @@ static int enqueue_search(Ctx* c, const SearchCfg& cfg, int keep_candidates, boo
     p.drop_row_copies = (c->inject & ANQI_FAULT_DROP_ROW_COPIES) ? 1u : 0u;
     p.post_rows = cfg.post_rows;
     auto kern = cfg.block ? block_kernel_for(ix.dim) : search_kernel_for(ix.dim, cfg.wpb);
-    ANQI_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem));
     // in a captured graph the events become event-record nodes (so the replay
     // is timed like a plain launch)
     const unsigned ef = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -1678,6 +1676,8 @@ static int query_run(anqi_ctx* h, int keep_candidates, anqi_query_stats* st, boo
         if ((rc = block_cfg(c, blk, &use_block))) return rc;
         if (use_block) cfgs.push_back(blk);
     }
+    for (uint32_t w : {2u, 4u, 8u})
+        if (!use_block) ANQI_CUDA(c, allow_smem(search_kernel_for(ix.dim, w)));
     for (const auto& shape : kShapes) {
         if (use_block) break;
         if (fshape && (shape[0] != f_w || (f_t && shape[1] != f_t))) continue;

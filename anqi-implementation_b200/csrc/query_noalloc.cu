@@ -342,8 +342,7 @@ extern "C" int anqi_rknn_query_noalloc(const anqi_device_index* ix, const float*
     const size_t smem = (size_t)(4 * L + 128 + ix->lifted_stride + ix->base_stride) * 4 * wpb;
     if (smem > 227 * 1024) return ANQI_ERR_ARGS;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaFuncSetAttribute(noalloc_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    if (allow_smem(noalloc_search_kernel) != cudaSuccess)
         return ANQI_ERR_DEVICE;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_search_kernel, 32 * wpb, smem) !=

@@ -1269,7 +1269,7 @@ uint32_t tc_dp(uint32_t d) {
 int filter_kernel_for(Ctx* c, uint32_t dp, void (**kern)(FilterParams), size_t* smem) {
     *kern = dp > kMaxDp ? tc_filter_kernel<true> : tc_filter_kernel<false>;
     *smem = filter_smem(dp);
-    ANQI_CUDA(c, cudaFuncSetAttribute(*kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    ANQI_CUDA(c, allow_smem(*kern));
     return ANQI_OK;
 }
 
@@ -1303,7 +1303,7 @@ int launch_scan(Ctx* c, FilterParams p, uint64_t nrows) {
     const uint32_t fixed = scan_fixed_bytes(p.dp), slot = scan_slot_bytes(p.dp);
     sp.slots = std::min<uint32_t>(kScanMaxSlots, (226 * 1024 - fixed) / slot);
     const size_t smem = fixed + (size_t)sp.slots * slot;
-    ANQI_CUDA(c, cudaFuncSetAttribute(tc_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(tc_scan_kernel));
     const uint32_t grid = (uint32_t)std::min<uint64_t>(c->sm_count, (uint64_t)sp.qtiles * sp.slices);
     tc_scan_kernel<<<grid, kScanThreads, smem, c->stream>>>(sp);
     ANQI_CUDA(c, cudaGetLastError());
@@ -1532,7 +1532,7 @@ int tc_join_filter(Ctx* c, const TcPrep& tp, const float* d_norms, uint64_t n, c
     p.mask = mask;
     p.err = c->err.as<uint32_t>();
     const size_t smem = (size_t)kTile * tp.dp * 2;
-    ANQI_CUDA(c, cudaFuncSetAttribute(join_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(join_filter_kernel));
     const uint64_t blocks = (n + 3) / 4;
     if (blocks > 0x7FFFFFFFull) return fail(c, ANQI_ERR_ARGS, "too many rows for the LocalJoin filter");
     join_filter_kernel<<<(unsigned)blocks, 128, smem, c->stream>>>(p);
@@ -1603,7 +1603,7 @@ int tc_leaf_filter(Ctx* c, const TcPrep& tp, const float* d_x, const float* d_no
         const uint32_t tiles = (maxcnt + kTile - 1) / kTile;
         const size_t bytes = leaf_smem(p.dp, tiles);
         auto leaf = leaf_plain(p) ? tc_leaf_kernel<true> : tc_leaf_kernel<false>;
-        ANQI_CUDA(c, cudaFuncSetAttribute(leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        ANQI_CUDA(c, allow_smem(leaf));
         // few leaves: their row blocks over several CTAs while SMs are idle
         const uint32_t parts = (uint32_t)std::max<size_t>(1, std::min<size_t>(tiles, c->sm_count / ntiles));
         leaf<<<dim3((unsigned)ntiles, parts), kLeafThreads, bytes, c->stream>>>(p, tiles);
@@ -1665,7 +1665,7 @@ int anqi_bf16_gram(anqi_ctx* h, const float* a, uint64_t na, const float* b, uin
         return rc;
     ANQI_CUDA(c, cudaMemsetAsync(c->err.p, 0, 4, c->stream));
     const size_t smem = (size_t)2 * kTile * dp * 2;
-    ANQI_CUDA(c, cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ANQI_CUDA(c, allow_smem(gram_kernel));
     dim3 grid((unsigned)((na + kTile - 1) / kTile), (unsigned)((nb + kTile - 1) / kTile));
     gram_kernel<<<grid, 128, smem, c->stream>>>(ab.as<__nv_bfloat16>(), na, bb.as<__nv_bfloat16>(), nb, dp,
                                                 dout.as<float>(), c->err.as<uint32_t>());
