@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) lrq_objective_backward_kernel(Gra
     }
 #pragma unroll
     for (uint32_t mm = 0; mm < M; mm++) {
+        if (mm >= p.m) break;  // zero times an infinite residual there
         const double sv = __shfl_sync(kWarp, ssum, sum_lane<M>(mm));
 #pragma unroll
         for (uint32_t j = 0; j < kMaxCols; j++) gmu[j] = fma(-sG[mm * kRow + 32 * j + lane], sv, gmu[j]);
