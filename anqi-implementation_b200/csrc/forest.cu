@@ -38,6 +38,12 @@ __device__ __forceinline__ uint64_t node_key(uint64_t seed, uint32_t tree, uint3
     return hash64(hash64(seed ^ ((uint64_t)tree << 32)) ^ (uint64_t)node);
 }
 
+// An upper bound of |h| from h2 = <h, h> in FP32: sums of up to 1,024 squares, each
+// up to 2^-149 short where it underflows.
+__device__ __forceinline__ float norm_bound(float h2, uint32_t dim) {
+    return __fsqrt_ru(h2 + 2e-45f * dim) * 1.001f;
+}
+
 // One warp per splitting node: pivots, hyperplane, midpoint, offset.  The
 // angular form (the ip metric, rptrees.h:41-52) splits through the origin by
 // the normalized difference of the unit-scaled pivots: x0/|x0| - x1/|x1|,
@@ -76,7 +82,7 @@ __global__ void forest_hyperplane_kernel(const float* __restrict__ x, uint32_t s
         const float h2 = group_ip(hp, hp, dim, gt, kAll);
         if (lane == 0) {
             offset[w] = 0.0f;
-            hnorm[w] = __fsqrt_ru(h2) * 1.001f;
+            hnorm[w] = norm_bound(h2, dim);
         }
         return;
     }
@@ -90,7 +96,7 @@ __global__ void forest_hyperplane_kernel(const float* __restrict__ x, uint32_t s
     const float h2 = group_ip(hp, hp, dim, gt, kAll);
     if (lane == 0) {
         offset[w] = off;
-        hnorm[w] = __fsqrt_ru(h2) * 1.001f;  // a bound: FP32 sums of up to 1,024 squares
+        hnorm[w] = norm_bound(h2, dim);
     }
 }
 
