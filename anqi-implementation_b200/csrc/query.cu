@@ -571,14 +571,11 @@ __global__ void __launch_bounds__(32 * kWpb, 32 / kWpb) rknn_search_kernel(Searc
 // one step between two buffers, a thread per entry.  Same expansions, same
 // arithmetic, same (dist, original id) order as rknn_search_kernel, so the
 // results are its.  Bound by the latency of its chain per expansion: links,
-// visited test, rows, rank and merge, four block barriers.  One query, 50,000 x
-// 128, L = 128: 827 us a warp per query, 518 us this way; 333 queries, 60,000 x
-// 100 (ip), L = 85: 1,540 us and 472 us.
-// Two things take memory off that chain: the links of every entry that enters the
-// beam or the candidate list are touched into L1 at once, and one warp that has
-// no rows to reduce touches the unvisited neighbours' rows of the next node in
-// line while the current one's are fetched: 518 -> 462 us for the one query;
-// the 333, 2-3 blocks to an SM, stay where they were (481 and 485 us).
+// visited test, rows, rank and merge, four block barriers.  Four blocks to an SM are
+// asked for, so that 64 registers hold a row's loads in flight together (left to
+// itself the compiler takes 48 for d = 128 and issues them in parts).  One query,
+// 50,000 x 128, L = 128: 827 us a warp per query, 516 us this way with 48 registers,
+// 397 us with 64; 333 queries, 60,000 x 100 (ip), L = 85: 1,540 us and 470 us.
 constexpr uint32_t kBlockThreads = 256;
 constexpr uint32_t kBlockCand = 1024;  // candidates kept in shared memory; the rest in the slot's scratch
 
@@ -586,19 +583,8 @@ __device__ __host__ __forceinline__ size_t block_search_words(uint32_t L_max, ui
     return (size_t)lstride + 4 * (size_t)L_max + 4 * 64 + kBlockCand + 32 + ((n + 127) / 128) * 4;
 }
 
-// Brings the line of *p into L1; nothing waits for it.
-__device__ __forceinline__ void touch(const void* p) {
-    asm volatile("{\n\t.reg .u32 t;\n\tld.global.ca.u32 t, [%0];\n\t}\n" ::"l"(p));
-}
-// Quarter gt of a node's links and degree.
-__device__ __forceinline__ void touch_links(const SearchParams& p, uint32_t node, uint32_t gt) {
-    const uint32_t* lk = p.links + (size_t)node * p.degree;
-    if (gt == 3) touch(p.deg + node);
-    else touch(lk + (gt == 0 ? 0u : (gt == 1 ? p.degree / 2 : p.degree - 1)));
-}
-
 template <uint32_t kDim>
-__global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(SearchParams p) {
+__global__ void __launch_bounds__(kBlockThreads, 4) rknn_search_block_kernel(SearchParams p) {
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, gt = t & 3u, grp = t >> 2;
     const uint32_t ls = search_lstride<kDim>(p);
     float* qhat = reinterpret_cast<float*>(g_smem);
@@ -715,23 +701,9 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
                     if (!flood) bi[cur] = node | kExpanded;
                 }
             }
-            // the next node in line, for the rows its expansion will fetch
-            uint32_t nl0 = kEmpty, nl1 = kEmpty, ndg = 0;
-            if (warp == 6) {
-                if (!flood && nxt < size) load_links(p, bi[nxt] & kIdMask, lane, nl0, nl1, ndg);
-                else if (flood && head < ncand) load_links(p, cand_at(head), lane, nl0, nl1, ndg);
-            }
             __syncthreads();
             const uint32_t m = s_u[kM];
             nvis += m;
-            if (warp == 6) {
-                const bool t0 = lane < ndg && nl0 < p.n && !((bits[nl0 >> 5] >> (nl0 & 31u)) & 1u);
-                const bool t1 = lane + 32 < ndg && nl1 < p.n && !((bits[nl1 >> 5] >> (nl1 & 31u)) & 1u);
-                for (uint32_t o = 0; o < ls; o += 32) {
-                    if (t0) touch(p.lifted + (size_t)nl0 * ls + o);
-                    if (t1) touch(p.lifted + (size_t)nl1 * ls + o);
-                }
-            }
             if (m == 0) {
                 // nothing new; the barrier keeps the next expansion's kM apart from this one's
                 __syncthreads();
@@ -751,12 +723,6 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
                 const uint32_t p0 = ncand + __popc(b0 & lt), p1 = ncand + __popc(b0) + __popc(b1 & lt);
                 if (in0 && p0 < p.cand_cap) cand_at(p0) = ni[lane];
                 if (in1 && p1 < p.cand_cap) cand_at(p1) = ni[lane + 32];
-                if (flood) {
-                    for (uint32_t g = 0; g < 4; g++) {
-                        if (in0) touch_links(p, ni[lane], g);
-                        if (in1) touch_links(p, ni[lane + 32], g);
-                    }
-                }
                 const uint32_t tot = ncand + __popc(b0) + __popc(b1);
                 if (lane == 0) {
                     s_u[kNcand] = min(tot, p.cand_cap);
@@ -779,9 +745,8 @@ __global__ void __launch_bounds__(kBlockThreads) rknn_search_block_kernel(Search
                     sd[rank] = dv;
                     si[rank] = iv;
                 }
-                const bool keep = mine && (!full || ord(dv, iv, bd[L - 1], bi[L - 1]));
-                if (keep) touch_links(p, iv, gt);
-                mk = __syncthreads_count(keep && gt == 0);
+                const bool keep = mine && gt == 0 && (!full || ord(dv, iv, bd[L - 1], bi[L - 1]));
+                mk = __syncthreads_count(keep);
             } else {
                 __syncthreads();
             }
