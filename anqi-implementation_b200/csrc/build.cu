@@ -1883,9 +1883,12 @@ static int run_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_t
 }
 
 // The AKNN gather of rows without a component: a block per row where at least
-// three blocks share an SM (up to about 480,000 rows; above, the bitmap leaves
-// one block and the warp-per-row kernel keeps more searches in flight), else
-// gather_kernel.  ANQI_B200_GATHER_BLOCK=0 turns it off.
+// three blocks share an SM (up to about 480,000 rows under l2; above, the bitmap
+// leaves fewer and the warp-per-row kernel keeps more searches in flight), else
+// gather_kernel.  Block and warp form over unit rows, 16 trees: three blocks an SM,
+// 450,000 x 32 l2, 593 and 791 ms; two, 600,000 x 32 l2, 1,218 and 1,085, x 128
+// 1,574 and 1,336, but 450,000 x 32 ip 548 and 704 and 600,000 x 32 ip 743 and 993;
+// one, 900,000 x 32 l2, 3,784 and 1,690, 1.3M x 32 ip 3,185 and 2,387.  ANQI_B200_GATHER_BLOCK=0 turns it off.
 static int run_aknn_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_total, double* kernel_ms) {
     const char* env = std::getenv("ANQI_B200_GATHER_BLOCK");
     const size_t smem = gather_block_words(p.n, p.ef, p.stride, p.ip != 0) * 4;

@@ -165,9 +165,11 @@ typedef struct {
     uint64_t seed;       /* 10 */
     uint32_t nn_iters;   /* ANQI_NNITERS, default 0 */
     uint32_t nn_sample;  /* ANQI_NNSAMPLE, default 20 */
-    uint32_t precision;  /* init_knn leaf distances: 0 = FP32 CUDA cores, 1 = BF16 tensor-core
-                            tiles with FP32 recheck (identical output; d <= 1024, rows
-                            above 256 dimensions in K chunks; larger d runs on the CUDA cores) */
+    uint32_t precision;  /* 0 = FP32; 1 = init_knn leaf distances on BF16 tensor-core tiles and
+                            the forest's sides from BF16 rows, both with an error bound and
+                            an FP32 recheck of what it leaves open (identical output; d <=
+                            1024, rows above 256 dimensions in K chunks; larger d runs in
+                            FP32 on the CUDA cores) */
     uint32_t metric;     /* ANQI_METRIC_L2 (0) or ANQI_METRIC_IP (key 1 - <a, b>, either
                             precision); the ip metric takes no LocalJoin (nn_iters = 0) */
 } anqi_aknn_params;
