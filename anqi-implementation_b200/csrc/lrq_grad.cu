@@ -254,6 +254,7 @@ struct GradParams {
     double* g_mu;
     double* g_G;
     double* g_B;
+    bool zero_others;  // lrq_codebook_grad_kernel: zero g_mu and g_G
 };
 
 // Gradients of mu and G.  A warp keeps its lanes' columns of both in registers
@@ -355,11 +356,17 @@ __global__ void __launch_bounds__(kThreads, 1) lrq_objective_backward_kernel(Gra
 // Gradient of B: the sums of r by code.  A block has the histograms of 32
 // columns in shared memory, lane l of every warp adding to column l's (bank
 // pair l: no conflicts inside a warp, hardly any collisions between warps), and
-// adds them to g_B once (43 us at 120,000 x 100 x 256).  Adding every r to g_B in
-// global memory took an atomic per matrix entry.
+// adds them to g_B once (43 us at 120,000 x 100 x 256); one that has a column's rows
+// to itself stores them.  Adding every r to g_B in global memory took an atomic per
+// matrix entry.  Launched before the other half (zero_others) it also zeroes that
+// one's outputs.
 constexpr uint32_t kHistThreads = 1024;
 __global__ void __launch_bounds__(kHistThreads, 1) lrq_codebook_grad_kernel(GradParams p) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, k0 = blockIdx.x * 32, k = k0 + lane;
+    if (p.zero_others && blockIdx.x == 0 && blockIdx.y == 0) {
+        for (uint32_t t = threadIdx.x; t < p.nk; t += kHistThreads) p.g_mu[t] = 0.0;
+        for (uint32_t t = threadIdx.x; t < p.m * p.nk; t += kHistThreads) p.g_G[t] = 0.0;
+    }
     for (uint32_t t = threadIdx.x; t < p.cs * 32; t += kHistThreads) s_lrq[t] = 0.0;
     __syncthreads();
     constexpr uint32_t kAhead = 4, kWarps = kHistThreads / 32;
@@ -383,21 +390,33 @@ __global__ void __launch_bounds__(kHistThreads, 1) lrq_codebook_grad_kernel(Grad
     for (uint32_t t = threadIdx.x; t < p.cs * 32; t += kHistThreads) {
         const uint32_t a = t >> 5, kk = ((t & 31u) + a) & 31u;
         const double v = s_lrq[a * 32 + kk];
-        if (v != 0.0) atomicAdd(p.g_B + (size_t)(k0 + kk) * p.cs + a, p.scale * v);
+        if (k0 + kk >= p.nk) continue;
+        double* out = p.g_B + (size_t)(k0 + kk) * p.cs + a;
+        if (gridDim.y == 1) *out = p.scale * v;
+        else if (v != 0.0) atomicAdd(out, p.scale * v);
     }
 }
 
-int sm_count() {
+uint32_t sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
+    return (uint32_t)sms;
 }
 
 constexpr size_t kSmemMax = 227 * 1024;
 
-// At least four rows a warp, so small inputs do not pay for filling every SM's
-// shared memory.
+// allow_smem where a launch needs it (the calls are a fifth of a small step's host
+// time).
+template <class Kernel>
+cudaError_t large_smem(Kernel kern, size_t smem) {
+    return smem > 48 * 1024 ? allow_smem(kern) : cudaSuccess;
+}
+
+// A block an SM, fewer only where a warp would have no row: rows one after the other
+// cost a warp more than filling another SM's shared memory (forward and backward of
+// 1,000 x 100, rank 8, 256 codes: 17.2 and 10.8 us with four rows a warp, 11.0 and
+// 7.5 with one; 300 x 100: 17.0 and 10.6, 10.3 and 6.8).
 template <uint32_t M, uint32_t kThreads>
 cudaError_t launch_forward(ObjParams p, cudaStream_t st) {
     const size_t fixed = (size_t)M * 32 * kMaxCols * 8;
@@ -408,30 +427,44 @@ cudaError_t launch_forward(ObjParams p, cudaStream_t st) {
     p.bcols = fit >= p.nk ? p.nk : (uint32_t)fit / 32 * 32;
     const size_t smem = fixed + (p.codes_in ? 0 : (size_t)p.bcols * p.bpitch * 8);
     auto kern = lrq_objective_forward_kernel<M, kThreads>;
-    cudaError_t e = allow_smem(kern);
+    cudaError_t e = large_smem(kern, smem);
     if (e != cudaSuccess) return e;
-    constexpr uint64_t rows = kThreads / 32 * 4;
+    constexpr uint64_t rows = kThreads / 32;
     kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
     return cudaGetLastError();
 }
 
 template <uint32_t M, uint32_t kThreads>
-cudaError_t launch_backward(const GradParams& p, cudaStream_t st) {
+cudaError_t launch_backward(GradParams p, cudaStream_t st) {
+    // the codebook's: one block an SM, at least 64 rows a block
+    const size_t hist = (size_t)p.cs * 32 * 8;
+    cudaError_t e = large_smem(lrq_codebook_grad_kernel, hist);
+    if (e != cudaSuccess) return e;
+    const uint32_t sms = sm_count(), groups = (p.nk + 31) / 32;
+    const uint64_t rowgroups = std::min<uint64_t>((p.n + 63) / 64, std::max(1u, sms / groups));
+    if (rowgroups > 1 && (e = cudaMemsetAsync(p.g_B, 0, (size_t)p.nk * p.cs * sizeof(double), st)) != cudaSuccess)
+        return e;
+    auto codebook = [&] {
+        lrq_codebook_grad_kernel<<<dim3(groups, (unsigned)rowgroups), kHistThreads, hist, st>>>(p);
+        return cudaGetLastError();
+    };
+    // before the other half while T and r stay in L2, which saves two memsets (a step of
+    // 1,000 x 100: 37.8 and 33.8 us); past that after it, which reads T and r itself
+    // and leaves the end of r behind (120,000 x 100: 352 us before, 338 after)
+    p.zero_others = 2 * p.n * p.nk * sizeof(double) <= 64ull << 20;
+    if (p.zero_others) {
+        if ((e = codebook()) != cudaSuccess) return e;
+    } else if ((e = cudaMemsetAsync(p.g_mu, 0, p.nk * sizeof(double), st)) != cudaSuccess ||
+               (e = cudaMemsetAsync(p.g_G, 0, (size_t)p.m * p.nk * sizeof(double), st)) != cudaSuccess) {
+        return e;
+    }
     const size_t smem = (size_t)(2 * M + 1) * 32 * kMaxCols * 8;
     auto kern = lrq_objective_backward_kernel<M, kThreads>;
-    cudaError_t e = allow_smem(kern);
-    if (e != cudaSuccess) return e;
-    constexpr uint64_t rows = kThreads / 32 * 4;
-    kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sm_count()), kThreads, smem, st>>>(p);
+    if ((e = large_smem(kern, smem)) != cudaSuccess) return e;
+    constexpr uint64_t rows = kThreads / 32;
+    kern<<<(unsigned)std::min<uint64_t>((p.n + rows - 1) / rows, sms), kThreads, smem, st>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // one block an SM, at least 64 rows a block
-    const size_t hist = (size_t)p.cs * 32 * 8;
-    e = allow_smem(lrq_codebook_grad_kernel);
-    if (e != cudaSuccess) return e;
-    const uint32_t groups = (p.nk + 31) / 32;
-    const uint64_t rowgroups = std::min<uint64_t>((p.n + 63) / 64, std::max(1u, sm_count() / groups));
-    lrq_codebook_grad_kernel<<<dim3(groups, (unsigned)rowgroups), kHistThreads, hist, st>>>(p);
-    return cudaGetLastError();
+    return p.zero_others ? cudaSuccess : codebook();
 }
 
 }  // namespace
@@ -459,11 +492,7 @@ int anqi_lrq_objective_backward(const double* T, uint64_t n, uint32_t nk, uint32
     if (!T || !mu || !G || !r || !c || !a || !g_mu || !g_G || !g_B || n == 0) return ANQI_ERR_ARGS;
     if (nk == 0 || nk > 32 * kMaxCols || m == 0 || m > 16 || cs == 0 || cs > 256) return ANQI_ERR_ARGS;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(g_mu, 0, nk * sizeof(double), st) != cudaSuccess ||
-        cudaMemsetAsync(g_G, 0, (size_t)m * nk * sizeof(double), st) != cudaSuccess ||
-        cudaMemsetAsync(g_B, 0, (size_t)nk * cs * sizeof(double), st) != cudaSuccess)
-        return ANQI_ERR_DEVICE;
-    GradParams p{T, n, nk, m, cs, mu, G, r, c, a, scale, g_mu, g_G, g_B};
+    GradParams p{T, n, nk, m, cs, mu, G, r, c, a, scale, g_mu, g_G, g_B, false};
     const cudaError_t e = m <= 8 ? launch_backward<8, 384>(p, st) : launch_backward<16, 256>(p, st);
     return e == cudaSuccess ? ANQI_OK : ANQI_ERR_DEVICE;
 }
