@@ -16,6 +16,7 @@
 // fit to rounding, not bit for bit.  Every entry point takes device pointers,
 // enqueues on the caller's stream and allocates nothing; scratch comes from
 // the caller with its size checked.
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -219,11 +220,41 @@ __global__ void fit_lohi_init_kernel(double* lohi, uint32_t nk) {
 // Bound by the lanes' digit matching and the moves' scattered 8-byte writes.
 constexpr uint32_t kSortTile = 4096, kSortPer = 16;  // keys a tile of 8 warps; a thread's share
 
-// The digit at `shift` of a key's rank among doubles (sign folded in).
-__device__ __forceinline__ uint32_t sort_digit(double v, uint32_t shift) {
+// A key's rank among doubles (sign folded in), back, and the rank's digit at `shift`.
+__device__ __forceinline__ uint64_t sort_rank(double v) {
     const uint64_t b = (uint64_t)__double_as_longlong(v);
-    const uint64_t r = b ^ ((b >> 63) ? ~0ull : 0x8000000000000000ull);
-    return (uint32_t)(r >> shift) & 255u;
+    return b ^ ((b >> 63) ? ~0ull : 0x8000000000000000ull);
+}
+__device__ __forceinline__ double sort_key(uint64_t r) {
+    return __longlong_as_double((long long)(r ^ ((r >> 63) ? 0x8000000000000000ull : ~0ull)));
+}
+__device__ __forceinline__ uint32_t sort_digit(double v, uint32_t shift) {
+    return (uint32_t)(sort_rank(v) >> shift) & 255u;
+}
+
+// A column of at most a tile, whole in shared memory: a bitonic network over its ranks
+// padded to n2, a power of two.  The passes above are 24 launches whatever m is: a
+// fit of 100 columns (256 codes) of 500 / 2,000 / 4,096 values, 197 / 211 / 246 us with
+// them and 33 / 60 / 90 this way; past a tile they win (10,000: 447 us, the network 1,052).
+__global__ void __launch_bounds__(1024) fit_sort_small_kernel(const double* __restrict__ src, uint32_t m, uint32_t n2,
+                                                              double* __restrict__ dst) {
+    __shared__ uint64_t s[kSortTile];
+    for (uint32_t t = threadIdx.x; t < n2; t += blockDim.x)
+        s[t] = t < m ? sort_rank(src[(uint64_t)blockIdx.x * m + t]) : ~0ull;
+    __syncthreads();
+    for (uint32_t kk = 2; kk <= n2; kk <<= 1)
+        for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
+            for (uint32_t t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
+                const uint32_t i = 2 * t - (t & (j - 1));  // the t-th index with bit j clear
+                const uint64_t x = s[i], y = s[i + j];
+                if ((x > y) == ((i & kk) == 0)) {
+                    s[i] = y;
+                    s[i + j] = x;
+                }
+            }
+            __syncthreads();
+        }
+    for (uint32_t t = threadIdx.x; t < m; t += blockDim.x) dst[(uint64_t)blockIdx.x * m + t] = sort_key(s[t]);
 }
 
 // The tile's keys of this warp (512 in a row, 32 at a time) and their digits,
@@ -539,7 +570,11 @@ int anqi_lrq_fit_codebooks(const double* res, uint64_t m, uint32_t nk, uint32_t 
     uint64_t* counts = reinterpret_cast<uint64_t*>(prefix + (uint64_t)nk * (m + 1));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)tiles, nk);
-    for (uint32_t pass = 0; pass < 8; pass++) {
+    uint32_t n2 = 2;
+    while (n2 < m && n2 < kSortTile) n2 <<= 1;
+    if (tiles == 1)
+        fit_sort_small_kernel<<<nk, std::max(32u, std::min(1024u, n2 / 2)), 0, st>>>(res, (uint32_t)m, n2, a);
+    for (uint32_t pass = 0; pass < 8 && tiles > 1; pass++) {
         // between the prefix sums' room and a, which the last pass fills
         const double* src = pass == 0 ? res : pass & 1u ? prefix : a;
         fit_sort_count_kernel<<<grid, 256, 0, st>>>(src, m, 8 * pass, counts);
