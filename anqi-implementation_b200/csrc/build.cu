@@ -1888,7 +1888,8 @@ static int run_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_t
 // gather_kernel.  Block and warp form over unit rows, 16 trees: three blocks an SM,
 // 450,000 x 32 l2, 593 and 791 ms; two, 600,000 x 32 l2, 1,218 and 1,085, x 128
 // 1,574 and 1,336, but 450,000 x 32 ip 548 and 704 and 600,000 x 32 ip 743 and 993;
-// one, 900,000 x 32 l2, 3,784 and 1,690, 1.3M x 32 ip 3,185 and 2,387.  ANQI_B200_GATHER_BLOCK=0 turns it off.
+// one, 900,000 x 32 l2, 3,784 and 1,690, 1.3M x 32 ip 3,185 and 2,387.
+// ANQI_B200_GATHER_BLOCK=0 turns it off.
 static int run_aknn_gather(Ctx* c, GatherParams p, uint64_t max_rev, uint64_t* pool_total, double* kernel_ms) {
     const char* env = std::getenv("ANQI_B200_GATHER_BLOCK");
     const size_t smem = gather_block_words(p.n, p.ef, p.stride, p.ip != 0) * 4;
@@ -2083,8 +2084,8 @@ static int run_select_commit(Ctx* c, const DevBuf& dx, const DevBuf& dn, uint64_
     int rc;
     if (links && row_order && !c->edge.active) {
         bool done = false;
-        rc = component_select_commit(c, dx, dn, n, stride, dim, hid, hval, K, M, ef, cap, alpha, *links, *deg, pool_total,
-                                     row_order, kernel_ms, &done);
+        rc = component_select_commit(c, dx, dn, n, stride, dim, hid, hval, K, M, ef, cap, alpha, *links, *deg,
+                                     pool_total, row_order, kernel_ms, &done);
         if (done) return ANQI_OK;
         if (rc && !fall_back(c, rc)) return rc;
     }

@@ -1179,7 +1179,8 @@ static int block_cfg(Ctx* c, SearchCfg& cfg, bool* fits) {
     *fits = false;
     const char* env = std::getenv("ANQI_B200_BLOCK");
     const size_t smem = block_search_words(b.L_max, c->ix.lstride, c->ix.n) * 4;
-    if ((env && env[0] == '0') || (c->inject & ANQI_FAULT_DROP_ROW_COPIES) || smem > 227 * 1024 || stage_rows_for(c->ix.lstride, c->ix.bstride) != 8)
+    if ((env && env[0] == '0') || (c->inject & ANQI_FAULT_DROP_ROW_COPIES) || smem > 227 * 1024 ||
+        stage_rows_for(c->ix.lstride, c->ix.bstride) != 8)
         return ANQI_OK;
     auto kern = block_kernel_for(c->ix.dim);
     ANQI_CUDA(c, allow_smem(kern));

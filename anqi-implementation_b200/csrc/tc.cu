@@ -760,9 +760,10 @@ __global__ void __launch_bounds__(kLeafThreads, 1) tc_leaf_kernel(FilterParams p
 // column constants C (the norm, or norm minus threshold, less a margin for its
 // own rounding) come with the tile, a row constant R holds the rest of the
 // inequality less eps over all columns and a margin for its terms, and the sign of
-// C + R + f acc is shifted into a mask.  Each column carries its own margin: one
-// of the largest |C| in every row let a single threshold of FLT_MAX keep all pairs.  Survivors go to a queue per warp; 32 of them at a time take the exact
-// test and the output slot's atomic, so its latency is paid once per 32.
+// C + R + f acc is shifted into a mask.  Each column carries its own margin: one of
+// the largest |C| in every row let a single threshold of FLT_MAX keep all pairs.
+// Survivors go to a queue per warp; 32 of them at a time take the exact test and the
+// output slot's atomic, so its latency is paid once per 32.
 // At 100,000 x 300 (unit rows, top-100, then three CSRs of 2,000 queries) the
 // scans take 10.1 ms; tiles that were copied 16 bytes a thread and waited for
 // chunk by chunk took 60.7 ms.
